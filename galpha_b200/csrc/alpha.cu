@@ -959,36 +959,6 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
 // its ro / nu_min entry until its nu_max entry, a triangle from its ro entry).
 namespace {
 
-struct QueryRank {
-    const double *spectrum;
-    int nSpec;
-    double alpha, q;
-    int by_quantile;
-    Counters *ct;
-    __device__ void operator()(long long) const
-    {
-        double a = alpha;
-        if (by_quantile) {
-            double qq = q < 0.0 ? 0.0 : (q > 1.0 ? 1.0 : q);
-            int k = (int)llrint(qq * (double)(nSpec - 1));
-            a = spectrum[k];
-        }
-        int R = -1;
-        if (a >= 0.0) {
-            int lo = 0, hi = nSpec - 1;  // spectrum[0] = 0 <= a
-            while (lo < hi) {
-                int mid = lo + (hi - lo + 1) / 2;
-                if (spectrum[mid] <= a) lo = mid;
-                else hi = mid - 1;
-            }
-            R = lo;
-        }
-        ct->qrank = R;
-        ct->qalpha = a;
-        for (int k = 0; k < 12; k++) ct->qcount[k] = 0;
-    }
-};
-
 __device__ __forceinline__ int interval_class(int ro, int nu_min, int nu_max, int R)
 {
     if (nu_max > 0 && nu_max <= R) return 3;
@@ -997,138 +967,291 @@ __device__ __forceinline__ int interval_class(int ro, int nu_min, int nu_max, in
     return 0;
 }
 
-struct QueryClassify {
-    const int2 *pt;
-    const int *edge_ro;
-    const int2 *edge_nu;
-    const int *tri_ro;
-    uint8_t *cls;
+// Largest index r in [lo, n) with sp[r] <= a, given sp[lo] <= a (one whole
+// warp; every lane gets r).  The 32 entries after lo are tried first: a
+// quantile's value is its own answer unless neighbours round to the same
+// double, and then each step splits the rest in 33.
+template <class T>
+__device__ __forceinline__ int warp_last_leq(const T *__restrict__ sp, int lo, int n, T a)
+{
+    const int lane = threadIdx.x & 31;
+    int hi = n - 1;  // the answer lies in [lo, hi]
+    for (bool near = true; lo < hi; near = false) {
+        const int step = near ? 1 : (hi - lo + 32) / 33;
+        const int i = (int)min((long long)hi, (long long)lo + (long long)(lane + 1) * step);
+        const unsigned m = __ballot_sync(0xffffffffu, sp[i] <= a);  // a prefix of the lanes
+        const int k = __popc(m);
+        const int base = lo;
+        lo = (int)min((long long)hi, (long long)base + (long long)k * step);
+        if (k < 32) hi = (int)min((long long)hi, max((long long)lo, (long long)base + (long long)(k + 1) * step - 1));
+    }
+    return lo;
+}
+
+// Rank of a query: the value (given, or the spectrum's at a quantile) and the
+// largest rank whose spectrum value is at most it, -1 for a negative value.
+__device__ __forceinline__ int warp_query_rank(const double *__restrict__ sp, int n, double q, int by_quantile,
+                                               double *alpha)
+{
+    double a = q;
+    int lo = 0;  // spectrum[0] = 0
+    if (by_quantile) {
+        const double qq = q < 0.0 ? 0.0 : (q > 1.0 ? 1.0 : q);
+        lo = (int)llrint(qq * (double)(n - 1));
+        a = sp[lo];
+    }
+    *alpha = a;
+    return a >= 0.0 ? warp_last_leq(sp, lo, n, a) : -1;
+}
+
+// The classified arrays: points, then edges, then triangles.  A block takes
+// chunks of kQChunk consecutive entries of one kind.  The kernel reads 8, 12
+// and 4 bytes and writes one byte per entry, so it is bound by memory as long
+// as its counts stay in registers: with one atomic per warp on the twelve
+// shared counters a query took 860 us at 4.2 M points, 23 times the 37 us that
+// its 243 MB take at the copy rate; with register counts it takes 58 us.
+struct QueryArrays {
+    const int2 *__restrict__ pt;
+    const int *__restrict__ edge_ro;
+    const int2 *__restrict__ edge_nu;
+    const int *__restrict__ tri_ro;
+    uint8_t *__restrict__ cls;
     int N, nE, nT;
-    Counters *ct;
-    __device__ void operator()(long long ii) const
+};
+
+constexpr int kQThreads = 256, kQItems = 8, kQChunk = kQThreads * kQItems;
+
+__host__ __device__ inline int q_chunks(int n) { return n / kQChunk + (n % kQChunk != 0); }
+
+// This thread's entries e0 + u * kQThreads < n of one kind (0 points, 1 edges,
+// 2 triangles): load() puts all loads in flight; classify() stores their
+// classes at the ranks rank(u) and hands them to count(u, class).
+struct QChunk {
+    int ro[kQItems];
+    int2 nu[kQItems];
+    __device__ __forceinline__ void load(const QueryArrays &A, int kind, int e0, int n)
     {
-        int i = (int)ii;
-        const int R = ct->qrank;
-        int type, k;
-        if (i < N) {
-            type = 0;
-            int2 v = pt[i];
-            k = (v.x < 0 || R < 0) ? 0 : interval_class(0, v.x, v.y, R);
-        } else if (i < N + nE) {
-            type = 1;
-            int e = i - N;
-            int ro = edge_ro[e];
-            int2 nu = edge_nu[e];
-            k = R < 0 ? 0 : interval_class(ro != 0 ? ro : -1, nu.x, nu.y, R);
-        } else {
-            type = 2;
-            k = (R >= 0 && tri_ro[i - N - nE] <= R) ? 3 : 0;
+#pragma unroll
+        for (int u = 0; u < kQItems; u++) {
+            const int e = e0 + u * kQThreads;
+            if (e >= n) continue;
+            if (kind == 0) nu[u] = A.pt[e];
+            else if (kind == 1) {
+                ro[u] = A.edge_ro[e];
+                nu[u] = A.edge_nu[e];
+            } else ro[u] = A.tri_ro[e];
         }
-        cls[i] = (uint8_t)k;
-        int bin = type * 4 + k;
-        unsigned peers = __match_any_sync(__activemask(), bin);
-        if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(&ct->qcount[bin], __popc(peers));
+    }
+    template <class Rank, class Count>
+    __device__ __forceinline__ void classify(const QueryArrays &A, int kind, int e0, int n, Rank rank, Count count) const
+    {
+        uint8_t *out = A.cls + (kind == 0 ? 0ll : kind == 1 ? (long long)A.N : (long long)A.N + A.nE);
+#pragma unroll
+        for (int u = 0; u < kQItems; u++) {
+            const int e = e0 + u * kQThreads;
+            if (e >= n) continue;
+            const int R = rank(u);
+            int k;
+            if (kind == 0) k = (nu[u].x < 0 || R < 0) ? 0 : interval_class(0, nu[u].x, nu[u].y, R);
+            else if (kind == 1) k = R < 0 ? 0 : interval_class(ro[u] != 0 ? ro[u] : -1, nu[u].x, nu[u].y, R);
+            else k = (R >= 0 && ro[u] <= R) ? 3 : 0;
+            out[e] = (uint8_t)k;
+            count(u, k);
+        }
     }
 };
 
-// Per set of a batch: the set's spectrum is spectrum[spec_off[s] + s ..] of
-// length nd[s] + 1 (its own rank-0 sentinel first).
-struct QueryRankSets {
-    const double *spectrum;
-    const int *spec_off, *nd;
-    const double *param;
-    int by_quantile;
-    int *R;
-    double *alpha;
-    __device__ void operator()(long long ss) const
-    {
-        int s = (int)ss;
-        const double *sp = spectrum + spec_off[s] + s;
-        int ns = nd[s] + 1;
-        double a = param[s];
-        if (by_quantile) {
-            double qq = a < 0.0 ? 0.0 : (a > 1.0 ? 1.0 : a);
-            a = sp[(int)llrint(qq * (double)(ns - 1))];
-        }
-        int r = -1;
-        if (a >= 0.0) {
-            int lo = 0, hi = ns - 1;
-            while (lo < hi) {
-                int mid = lo + (hi - lo + 1) / 2;
-                if (sp[mid] <= a) lo = mid;
-                else hi = mid - 1;
+// Four class counts of up to 65,535 each in one word.
+__device__ __forceinline__ unsigned long long warp_sum64(unsigned long long v)
+{
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// One query of a single set: every block finds the rank itself (two loads in
+// a row for a quantile), so the query is one launch; the last block to finish
+// hands the counts to the host's mirror and clears them for the next query.
+__global__ void __launch_bounds__(kQThreads) k_query(QueryArrays A, const double *__restrict__ spectrum, int nSpec,
+                                                     double q, int by_quantile, Counters *ct, Counters *host)
+{
+    __shared__ int s_R, s_cnt[12], s_last;
+    if (threadIdx.x < 12) s_cnt[threadIdx.x] = 0;
+    if (threadIdx.x < 32) {
+        double a;
+        const int R = warp_query_rank(spectrum, nSpec, q, by_quantile, &a);
+        if (threadIdx.x == 0) {
+            s_R = R;
+            if (blockIdx.x == 0) {
+                ct->qrank = R;
+                ct->qalpha = a;
             }
-            r = lo;
         }
+    }
+    __syncthreads();
+    const int R = s_R;
+    const int cp = q_chunks(A.N), ce = q_chunks(A.nE), chunks = cp + ce + q_chunks(A.nT);
+    // class counts, 16 bits each: at most 6 * 2^28 entries in chunks of 8 per
+    // thread over 8 blocks per SM are under 6,000 per thread
+    unsigned long long acc[3] = {0ull, 0ull, 0ull};
+    for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+        const int kind = ch < cp ? 0 : (ch < cp + ce ? 1 : 2);
+        const int c0 = ch - (kind == 0 ? 0 : kind == 1 ? cp : cp + ce);
+        unsigned long long n = 0ull;
+        // c0 * kQChunk < 2^31 - kQChunk (entry counts stay below 1.7e9), so e0 + 7 * 256 does not wrap
+        const int e0 = c0 * kQChunk + (int)threadIdx.x, ne = kind == 0 ? A.N : kind == 1 ? A.nE : A.nT;
+        QChunk Q;
+        Q.load(A, kind, e0, ne);
+        Q.classify(A, kind, e0, ne, [&](int) { return R; }, [&](int, int k) { n += 1ull << (16 * k); });
+        if (kind == 0) acc[0] += n;
+        else if (kind == 1) acc[1] += n;
+        else acc[2] += n;
+    }
+#pragma unroll
+    for (int kind = 0; kind < 3; kind++) {
+        unsigned v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = __reduce_add_sync(0xffffffffu, (unsigned)(acc[kind] >> (16 * k)) & 0xffffu);
+        const int k = threadIdx.x & 31;
+        const unsigned x = k == 0 ? v[0] : k == 1 ? v[1] : k == 2 ? v[2] : v[3];
+        if (k < 4 && x) atomicAdd(&s_cnt[kind * 4 + k], (int)x);
+    }
+    __syncthreads();
+    if (threadIdx.x < 12 && s_cnt[threadIdx.x]) atomicAdd(&ct->qcount[threadIdx.x], s_cnt[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ct->qdone, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 12) {
+        host->qcount[threadIdx.x] = *(volatile int *)&ct->qcount[threadIdx.x];
+        ct->qcount[threadIdx.x] = 0;
+    } else if (threadIdx.x == 12) {
+        host->qrank = *(volatile int *)&ct->qrank;
+        host->qalpha = *(volatile double *)&ct->qalpha;
+        host->err = ct->err;
+        ct->qdone = 0;
+    }
+    __threadfence_system();
+}
+
+// Per set of a batch (one warp each): the set's spectrum is
+// spectrum[spec_off[s] + s ..] of length nd[s] + 1 (its own rank-0 sentinel
+// first).
+__global__ void __launch_bounds__(kQThreads) k_query_ranks(const double *__restrict__ spectrum,
+                                                           const int *__restrict__ spec_off,
+                                                           const int *__restrict__ nd,
+                                                           const double *__restrict__ param, int by_quantile, int K,
+                                                           int *R, double *alpha, int *counts)
+{
+    const int s = blockIdx.x * (kQThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (s >= K) return;
+    double a;
+    const int r = warp_query_rank(spectrum + spec_off[s] + s, nd[s] + 1, param[s], by_quantile, &a);
+    if (lane == 0) {
         R[s] = r;
         alpha[s] = a;
     }
-};
+    if (lane < 12) counts[12 * (long long)s + lane] = 0;
+}
 
-struct QueryClassifySets {
-    const int2 *pt;
-    const int *edge_ro;
-    const int2 *edge_nu;
-    const int4 *edges;
-    const int *tri_ro;
-    const int *vset, *tset, *R;
-    uint8_t *cls;
-    int *counts;  // [K][12]
-    int N, nE, nT;
-    __device__ void operator()(long long ii) const
-    {
-        int i = (int)ii;
-        int type, k, s;
-        if (i < N) {
-            type = 0;
-            s = vset[i];
-            int r = R[s];
-            int2 v = pt[i];
-            k = (v.x < 0 || r < 0) ? 0 : interval_class(0, v.x, v.y, r);
-        } else if (i < N + nE) {
-            type = 1;
-            int e = i - N;
-            s = tset[edges[e].z];
-            int r = R[s];
-            int ro = edge_ro[e];
-            int2 nu = edge_nu[e];
-            k = r < 0 ? 0 : interval_class(ro != 0 ? ro : -1, nu.x, nu.y, r);
-        } else {
-            type = 2;
-            int t = i - N - nE;
-            s = tset[t];
-            int r = R[s];
-            k = (r >= 0 && tri_ro[t] <= r) ? 3 : 0;
-        }
-        cls[i] = (uint8_t)k;
-        int bin = s * 12 + type * 4 + k;
-        unsigned peers = __match_any_sync(__activemask(), bin);
-        if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(&counts[bin], __popc(peers));
+// Last set in [lo, hi] whose base is at most x, base[lo] <= x.
+__device__ __forceinline__ int q_set(const int *__restrict__ base, int lo, int hi, int x)
+{
+    while (lo < hi) {
+        const int m = (lo + hi + 1) >> 1;
+        if (base[m] <= x) lo = m;
+        else hi = m - 1;
     }
-};
+    return lo;
+}
+
+// A batch's queries.  Points, edges and triangles are grouped by set, so a
+// chunk knows its sets from its first and last entry (found by whole warps,
+// two rounds of loads for 1,024 sets, behind the chunk's own loads: a binary
+// search of ten dependent loads ahead of them kept the kernel at 290 us, it
+// now takes 188): a chunk inside one set (most of them)
+// counts in registers, one that spans several finds each entry's set between
+// those two.  No per-entry set array is read (the edges' sets used to take a
+// 16-byte record and a gather each: 296 us per query of 9.7 M points in 1,024
+// sets).
+__global__ void __launch_bounds__(kQThreads) k_query_sets(QueryArrays A, const int *__restrict__ vbase,
+                                                          const int *__restrict__ ebase,
+                                                          const int *__restrict__ tbase, int K,
+                                                          const int *__restrict__ R, int *counts)
+{
+    const int cp = q_chunks(A.N), ce = q_chunks(A.nE), chunks = cp + ce + q_chunks(A.nT);
+    for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+        const int kind = ch < cp ? 0 : (ch < cp + ce ? 1 : 2);
+        const int c0 = (ch - (kind == 0 ? 0 : kind == 1 ? cp : cp + ce)) * kQChunk;
+        const int n = kind == 0 ? A.N : kind == 1 ? A.nE : A.nT;
+        const int *base = kind == 0 ? vbase : kind == 1 ? ebase : tbase;
+        const int e0 = c0 + (int)threadIdx.x;
+        QChunk Q;
+        Q.load(A, kind, e0, n);
+        const int s0 = warp_last_leq(base, 0, K, c0), s1 = warp_last_leq(base, s0, K, min(n - 1, c0 + kQChunk - 1));
+        if (s0 == s1) {
+            const int r = R[s0];
+            unsigned long long acc = 0ull;
+            Q.classify(A, kind, e0, n, [&](int) { return r; }, [&](int, int k) { acc += 1ull << (16 * k); });
+            acc = warp_sum64(acc);  // at most 256 per class
+            const int k = threadIdx.x & 31;
+            if (k < 4) {
+                const int x = (int)(acc >> (16 * k)) & 0xffff;
+                if (x) atomicAdd(&counts[12 * (long long)s0 + kind * 4 + k], x);
+            }
+        } else {
+            int st[kQItems];
+#pragma unroll
+            for (int u = 0; u < kQItems; u++) {
+                const int e = e0 + u * kQThreads;
+                st[u] = e < n ? q_set(base, s0, s1, e) : s1;
+            }
+            Q.classify(A, kind, e0, n, [&](int u) { return R[st[u]]; },
+                       [&](int u, int k) {
+                           const int bin = st[u] * 12 + kind * 4 + k;
+                           const unsigned peers = __match_any_sync(__activemask(), bin);
+                           if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(&counts[bin], __popc(peers));
+                       });
+        }
+    }
+}
+
+QueryArrays query_arrays(const Ctx &c)
+{
+    return QueryArrays{c.pt_nu, c.edge_ro, c.edge_nu, c.tri_ro, c.qclass, c.N, c.nE, c.nT_out};
+}
+
+unsigned query_blocks(const Ctx &c)
+{
+    const long long chunks = (long long)q_chunks(c.N) + q_chunks(c.nE) + q_chunks(c.nT_out);
+    return (unsigned)std::max(1ll, std::min(chunks, (long long)c.sm_count * 8));
+}
 
 }  // namespace
 
-int alpha_query_sets(Ctx &c, int K, const int *vset, const int *tset, const int *spec_off, const int *nd,
-                     const double *param, int by_quantile, int *R, double *alpha, int *counts)
+int alpha_query_sets(Ctx &c, int K, const int *vbase, const int *ebase, const int *tbase, const int *spec_off,
+                     const int *nd, const double *param, int by_quantile, int *R, double *alpha, int *counts)
 {
-    GALPHA_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * 12 * (size_t)K, c.stream));
-    launch_n(c, QueryRankSets{c.spectrum, spec_off, nd, param, by_quantile, R, alpha}, K);
-    long long n = (long long)c.N + c.nE + c.nT_out;
-    launch_n(c, QueryClassifySets{c.pt_nu, c.edge_ro, c.edge_nu, c.edges, c.tri_ro, vset, tset, R, c.qclass, counts,
-                                  c.N, c.nE, c.nT_out},
-             n);
+    k_query_ranks<<<(unsigned)((K + kQThreads / 32 - 1) / (kQThreads / 32)), kQThreads, 0, c.stream>>>(
+        c.spectrum, spec_off, nd, param, by_quantile, K, R, alpha, counts);
+    k_query_sets<<<query_blocks(c), kQThreads, 0, c.stream>>>(query_arrays(c), vbase, ebase, tbase, K, R, counts);
+    count_launch(2);
     GALPHA_CUDA(cudaGetLastError());
     return GPUDT_OK;
 }
 
+// The query's answer is left in the host mirror's q* fields and err.
 int alpha_query(Ctx &c, double alpha, double q, bool by_quantile)
 {
-    launch_n(c, QueryRank{c.spectrum, c.nSpec, alpha, q, by_quantile ? 1 : 0, c.ctr}, 1);
-    long long n = (long long)c.N + c.nE + c.nT_out;
-    launch_n(c, QueryClassify{c.pt_nu, c.edge_ro, c.edge_nu, c.tri_ro, c.qclass, c.N, c.nE, c.nT_out, c.ctr}, n);
+    k_query<<<query_blocks(c), kQThreads, 0, c.stream>>>(query_arrays(c), c.spectrum, c.nSpec,
+                                                         by_quantile ? q : alpha, by_quantile ? 1 : 0, c.ctr,
+                                                         c.hctr_dev);
+    count_launch();
+    c.host_reads++;
     GALPHA_CUDA(cudaGetLastError());
-    return read_counters(c);
+    GALPHA_CUDA(cudaStreamSynchronize(c.stream));
+    return GPUDT_OK;
 }
 
 }  // namespace galpha

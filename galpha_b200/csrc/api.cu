@@ -1129,8 +1129,8 @@ int galphaBatchQuery(galphaHandle h, const double *values, int byQuantile, galph
     cudaGetLastError();  // clear an error left by unrelated runtime calls
     const int K = bh.K;
     GALPHA_CUDA(cudaMemcpyAsync(B.qparam, values, sizeof(double) * (size_t)K, cudaMemcpyHostToDevice, c.stream));
-    int r = alpha_query_sets(c, K, B.vsetall, B.tset, B.spec_off, B.nd, B.qparam, byQuantile ? 1 : 0, B.qR, B.qalpha,
-                             B.qcounts);
+    int r = alpha_query_sets(c, K, B.vbases, B.ebase, B.tbase, B.spec_off, B.nd, B.qparam, byQuantile ? 1 : 0, B.qR,
+                             B.qalpha, B.qcounts);
     if (r) return r;
     std::vector<int> R(K), cnt(12 * (size_t)K);
     std::vector<double> a(K);

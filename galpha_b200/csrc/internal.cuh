@@ -78,6 +78,7 @@ struct Counters {
     int sh_total;    // shift: all dropped sites listed so far
     int grp[8];      // per-round counts of a group of rounds run between two counter reads
     int ndup;        // missing sites found to be exact duplicates
+    int qdone;       // alpha query: blocks that have added their counts
 };
 
 // Relink record: an edge of a triangle created this round (loc = (t<<2)|i, or -1
@@ -493,8 +494,8 @@ struct AlphaSegs {
 };
 int stage_alpha(Ctx &c, AlphaSegs *segs = nullptr);
 int alpha_query(Ctx &c, double alpha, double q, bool by_quantile);
-int alpha_query_sets(Ctx &c, int K, const int *vset, const int *tset, const int *spec_off, const int *nd,
-                     const double *param, int by_quantile, int *R, double *alpha, int *counts);
+int alpha_query_sets(Ctx &c, int K, const int *vbase, const int *ebase, const int *tbase, const int *spec_off,
+                     const int *nd, const double *param, int by_quantile, int *R, double *alpha, int *counts);
 int master_list(Ctx &c);
 int alpha_from_host_mesh(Ctx &c, const double *h_xy, int n, const gpudtTriangle *tris, int nt);
 
