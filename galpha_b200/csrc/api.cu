@@ -37,10 +37,10 @@ __global__ void k_read_words(const unsigned *__restrict__ src, unsigned *dst, in
     __threadfence_system();
 }
 
-int read_counters(Ctx &c)
+int read_counters(Ctx &c, bool all)
 {
     static_assert(sizeof(Counters) % 4 == 0, "counter block is read as 32-bit words");
-    const int nw = (int)(sizeof(Counters) / 4);
+    const int nw = (int)((all ? sizeof(Counters) : offsetof(Counters, filt_spread)) / 4);
     k_read_words<<<1, 256, 0, c.stream>>>((const unsigned *)c.ctr, (unsigned *)c.hctr_dev, nw);
     count_launch();
     c.host_reads++;
@@ -221,6 +221,7 @@ static int ensure_sizes(HandleState &H, const Sizes &z)
     // round ids restart well before the int range ends; every stage that
     // compares stamps with round ids initialises its stamps first
     if (c.round_counter > (1 << 30)) c.round_counter = 1;
+    c.rec_round = 0;
     GALPHA_CUDA(cudaMemsetAsync(c.epoch, 0, sizeof(int) * z.cap, c.stream));
     GALPHA_CUDA(cudaMemsetAsync(c.vote, 0x7f, sizeof(int) * z.cap, c.stream));
     GALPHA_CUDA(cudaMemsetAsync(c.ctr, 0, sizeof(Counters), c.stream));
@@ -299,9 +300,7 @@ static int run_dt(HandleState &H, const double *d_xy, int n, double minX, double
     STAGE("compact", stage_compact(c));
 #undef STAGE
     ev_record(c, 8);
-    r = read_counters(c);
-    if (r) return r;
-    if (c.hctr->err) return stage_fail(c, c.hctr->err, "final");
+    if (c.hctr->err) return stage_fail(c, c.hctr->err, "final");  // as of the compaction's read
     c.st.nVerts = c.V;
     c.st.nFake = c.F;
     fill_predicate_stats(c);
@@ -394,7 +393,7 @@ static int run_batch(HandleState &H, int K, const int *sizes, const double *d_xy
     }
     ev_record(c, 9);
 #undef STAGE
-    r = read_counters(c);
+    r = read_counters(c, true);
     if (r) return r;
     if (c.hctr->err) return stage_fail(c, c.hctr->err, "final");
     c.st.nVerts = c.V;

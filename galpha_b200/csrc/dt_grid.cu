@@ -610,6 +610,7 @@ int emit_global(Ctx &c, int base, int cells, const int *cellmap)
     r = launch_emit_cells(c, ntiles, nwin, true, c.tv + base, cells, cellmap);
     if (r) return r;
     launch_n(c, SetInt{&c.ctr->ntris, base + total}, 1);
+    c.hctr->ntris = base + total;
     GALPHA_CUDA(cudaGetLastError());
     return GPUDT_OK;
 }

@@ -97,9 +97,9 @@ __device__ __forceinline__ int get_link(const int4 *tn, int loc)
     return p[dori(loc)];
 }
 
-__device__ __forceinline__ void push_rec(Relink *rec, Counters *ct, int loc, int old)
+__device__ __forceinline__ void push_rec(Relink *rec, int *nrec, int loc, int old)
 {
-    int k = atomicAdd(&ct->nrec, 1);
+    int k = atomicAdd(nrec, 1);
     rec[k] = Relink{loc, old};
 }
 
@@ -123,17 +123,6 @@ __device__ __forceinline__ int alloc_slot(int *freelist, Counters *ct, int cap)
     return s;
 }
 
-// After a round of allocations: a free-list count driven below zero by pops
-// that fell through to the tail is reset, so that a later free_slot appends
-// at index 0.
-struct ClampFree {
-    Counters *ct;
-    __device__ void operator()(long long) const
-    {
-        if (ct->nfree < 0) ct->nfree = 0;
-    }
-};
-
 __device__ __forceinline__ void free_slot(int4 *tv, int *freelist, Counters *ct, int t)
 {
     tv[t] = make_int4(-1, -1, -1, 0);
@@ -156,11 +145,12 @@ struct CountDeg {
 };
 
 // Incidence entry of vertex v in triangle t (v = vtx[k]): the oriented slot
-// and the next vertex counterclockwise, so matching reads only the list.
+// and the next vertex counterclockwise, so matching reads only the list.  The
+// degrees count down as the lists fill, so no cursors have to be cleared.
 struct FillInc {
     const int4 *tv;
     const int *start;
-    int *cursor;
+    int *deg;
     int2 *inc;
     __device__ void operator()(long long i) const
     {
@@ -169,7 +159,7 @@ struct FillInc {
         if (v.x < 0) return;
         int a[3] = {v.x, v.y, v.z};
         for (int k = 0; k < 3; k++) {
-            int s = start[a[k]] + atomicAdd(&cursor[a[k]], 1);
+            int s = start[a[k]] + atomicSub(&deg[a[k]], 1) - 1;
             inc[s] = make_int2(enc(t, k), a[p1(k)]);
         }
     }
@@ -205,21 +195,10 @@ struct MatchLinks {
                 }
             }
             if (cnt > 1) set_err(ct, GPUDT_ERR_TOPOLOGY, 20);
-            if (found < 0) atomicAdd(&ct->changed, 1);  // hull edge
+            if (found < 0) atomicAdd(&ct->nhull, 1);  // hull edge
             n[k] = found;
         }
         tn[t] = make_int4(n[0], n[1], n[2], 0);
-    }
-};
-
-struct SetVtri {
-    const int4 *tv;
-    int *vtri;
-    __device__ void operator()(long long i) const
-    {
-        int t = (int)i;
-        int4 v = tv[t];
-        if (v.x < 0) return;
         vtri[v.x] = enc(t, 0);
         vtri[v.y] = enc(t, 1);
         vtri[v.z] = enc(t, 2);
@@ -228,28 +207,24 @@ struct SetVtri {
 
 int stage_links(Ctx &c)
 {
-    int r = read_counters(c);
-    if (r) return r;
-    int nt = c.hctr->ntris;
+    int r;
+    int nt = c.hctr->ntris;  // as the emission left it
     int *deg = c.deg;       // [V+1]
     int *start = c.aux2;    // [V+1]
     GALPHA_CUDA(cudaMemsetAsync(deg, 0, sizeof(int) * (size_t)(c.V + 1), c.stream));
     launch_n(c, CountDeg{c.tv, deg}, nt);
     r = exclusive_scan_int(c, deg, start, c.V + 1, nullptr);
     if (r) return r;
-    GALPHA_CUDA(cudaMemsetAsync(deg, 0, sizeof(int) * (size_t)(c.V + 1), c.stream));
     int2 *inc = (int2 *)c.rec;  // relink records are not in use yet: 3*cap int2
     launch_n(c, FillInc{c.tv, start, deg, inc}, nt);
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
     launch_n(c, MatchLinks{c.tv, c.tn, start, inc, c.vtri, c.ctr}, nt);
-    launch_n(c, SetVtri{c.tv, c.vtri}, nt);
     GALPHA_CUDA(cudaGetLastError());
     r = read_counters(c);
     if (r) return r;
     if (c.hctr->err) return c.hctr->err;
     // the only hull edges are the F edges of the fake ring
-    if (c.hctr->changed != c.F) {
-        c.hctr->errinfo = c.hctr->changed;
+    if (c.hctr->nhull != c.F) {
+        c.hctr->errinfo = c.hctr->nhull;
         return GPUDT_ERR_TOPOLOGY;
     }
     return GPUDT_OK;
@@ -298,6 +273,16 @@ static int next_round(Ctx &c)
 {
     return ++c.round_counter;
 }
+// The relink-record count of a round, and the word the round's last launch
+// clears.
+static int *rec_word(const Ctx &c, int ahead = 0)
+{
+    return &c.ctr->r_rec[(c.rec_round + ahead) % kRing];
+}
+static int ring(int k)
+{
+    return k % kRing;
+}
 // Marks the k ids after `first` (first + 1 .. first + k) as used by rounds
 // that device code numbered itself.
 static void skip_rounds(Ctx &c, int first, int k)
@@ -332,6 +317,7 @@ struct ShiftRound {
     int *vround;
     const int *vtri;
     int round;
+    int *waiting;  // sites of the round that wait for another one
     Counters *ct;
     __device__ void operator()(long long ii) const
     {
@@ -356,7 +342,7 @@ struct ShiftRound {
             return;
         }
         if (wait) {
-            atomicAdd(&ct->nlist, 1);
+            atomicAdd(waiting, 1);
             return;
         }
         vround[v] = round;
@@ -365,7 +351,7 @@ struct ShiftRound {
             vstate[v] = VS_SHIFTED;
         } else {
             vstate[v] = VS_BAD;
-            atomicAdd(&ct->changed, 1);
+            atomicAdd(&ct->nbad, 1);
         }
     }
 };
@@ -379,7 +365,12 @@ struct ShiftRound {
 struct ShiftCandidates {
     const int8_t *vstate;
     int8_t *cand;
-    __device__ void operator()(long long i) const { cand[i] = vstate[i] == VS_UNDECIDED ? 1 : 0; }
+    int *drop;
+    __device__ void operator()(long long i) const
+    {
+        cand[i] = vstate[i] == VS_UNDECIDED ? 1 : 0;
+        drop[i] = 0;
+    }
 };
 
 // Drops candidate v (once per iteration) and lists it.
@@ -488,7 +479,7 @@ struct BadSelect {
     const int8_t *vstate;
     const int *vtri;
     int *list;
-    Counters *ct;
+    int *count;
     __device__ void operator()(long long ii) const
     {
         int v = (int)ii;
@@ -503,7 +494,7 @@ struct BadSelect {
             return true;
         });
         if (wait) return;
-        int k = atomicAdd(&ct->nlist, 1);
+        int k = atomicAdd(count, 1);
         list[k] = v;
     }
 };
@@ -525,6 +516,7 @@ struct BadRemove {
     double2 *pos;
     int8_t *vstate;
     Relink *rec;
+    int *nrec;
     int round, nreal;
     Counters *ct;
     __device__ void operator()(long long ii) const
@@ -562,7 +554,7 @@ struct BadRemove {
             if (ownv <= -2) {
                 int k = -2 - ownv;
                 set_fwd(fwd, Fs[k], Fi[k], loc);
-                push_rec(rec, ct, loc, O[k]);
+                push_rec(rec, nrec, loc, O[k]);
             } else {
                 set_link(tn, loc, ownv);
                 set_link(tn, ownv, loc);
@@ -652,20 +644,21 @@ struct CountState {
     __device__ void operator()(long long i) const
     {
         const bool hit = vstate[i] == s;
-        const int k = warp_reserve(&ct->nlist, hit ? 1 : 0);  // one atomic per warp
+        const int k = warp_reserve(&ct->nmiss, hit ? 1 : 0);  // one atomic per warp
         if (hit && list) list[k] = (int)i;
     }
 };
 
 // Rounds of the shifting loops run in groups of c.shift_group between counter
 // reads: list lengths stay on the device (launch_dev), each round's count is
-// kept in ct->grp[], and a round after the loop's last one does nothing (an
+// kept in its ring word, and a round after the loop's last one does nothing (an
 // empty list, or no site left in the state it acts on), so running past the
 // end of a loop changes no result.
 
 int stage_shift(Ctx &c)
 {
     const int kShiftGroup = c.shift_group;
+    Counters *ct = c.ctr;
     int r;
     int shiftRounds = 0, badCount = 0;
     int *dropped = c.aux2;  // every site the optimistic phase dropped: the only undecided ones after it
@@ -674,31 +667,28 @@ int stage_shift(Ctx &c)
         int8_t *cand = (int8_t *)c.list2;
         int *drop = c.list2 + ((c.V + 1023) >> 2) + 256;
         int *lists[2] = {c.list, c.aux};  // vertices dropped in an iteration (ping-pong)
-        launch_n(c, ShiftCandidates{c.vstate, cand}, c.V);
-        GALPHA_CUDA(cudaMemsetAsync(drop, 0, sizeof(int) * (size_t)c.V, c.stream));
-        GALPHA_CUDA(cudaMemsetAsync(c.ctr->sh_n, 0, 3 * sizeof(int), c.stream));  // sh_n[2], sh_total
+        launch_n(c, ShiftCandidates{c.vstate, cand, drop}, c.V);
         bool settled = false;
         for (int it = 0; !settled;) {
+            const int it0 = it;
             for (int j = 0; j < kShiftGroup; j++, it++) {
                 int *cur = lists[it & 1], *prev = lists[(it + 1) & 1];
-                int *curn = &c.ctr->sh_n[it & 1], *prevn = &c.ctr->sh_n[(it + 1) & 1];
-                GALPHA_CUDA(cudaMemsetAsync(curn, 0, sizeof(int), c.stream));
+                int *curn = &ct->r_drop[ring(it)], *prevn = &ct->r_drop[ring(it + kRing - 1)];
                 if (it == 0)
-                    launch_dev(c, ShiftCheckTris{c.tv, c.pos, c.opos, cand, drop, cur, curn, c.ctr}, &c.ctr->ntris,
+                    launch_dev(c, ShiftCheckTris{c.tv, c.pos, c.opos, cand, drop, cur, curn, ct}, &ct->ntris,
                                c.cap_tris);
                 else
-                    launch_dev(c, ShiftCheckFans{c.tv, c.tn, c.vtri, c.pos, c.opos, cand, prev, drop, cur, curn,
-                                                 c.ctr},
+                    launch_dev(c, ShiftCheckFans{c.tv, c.tn, c.vtri, c.pos, c.opos, cand, prev, drop, cur, curn, ct},
                                prevn, c.V);
-                launch_dev(c, ShiftDropList{cur, cand, drop, dropped, &c.ctr->sh_total, c.N, c.ctr}, curn, c.V);
-                launch_n(c, CopyElems<int>{&c.ctr->grp[j], curn}, 1);
+                launch_dev(c, ShiftDropList{cur, cand, drop, dropped, &ct->sh_total, c.N, ct}, curn, c.V,
+                           Clears{{&ct->r_drop[ring(it + kRing / 2)]}});
             }
             r = read_counters(c);
             if (r) return r;
             if (c.hctr->err) return c.hctr->err;
             for (int j = 0; j < kShiftGroup && !settled; j++) {
                 shiftRounds++;
-                settled = c.hctr->grp[j] == 0;
+                settled = c.hctr->r_drop[ring(it0 + j)] == 0;
             }
             if (!settled && shiftRounds >= c.max_rounds) return GPUDT_ERR_NOCONVERGE;
         }
@@ -707,45 +697,44 @@ int stage_shift(Ctx &c)
     // vertices fixed from the start (fake ring) and the optimistic set count
     // as decided in the first shifting round (id 1); the rest go through
     // priority rounds
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
     for (int round = 2, done = 0; !done;) {
-        for (int j = 0; j < kShiftGroup; j++, round++) {
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist, 0, sizeof(int), c.stream));
+        const int round0 = round;
+        for (int j = 0; j < kShiftGroup; j++, round++)
             launch_dev(c,
-                       ShiftRoundList{ShiftRound{c.tv, c.tn, c.pos, c.opos, c.vstate, c.vround, c.vtri, round, c.ctr},
+                       ShiftRoundList{ShiftRound{c.tv, c.tn, c.pos, c.opos, c.vstate, c.vround, c.vtri, round,
+                                                 &ct->r_wait[ring(round)], ct},
                                       dropped},
-                       &c.ctr->sh_total, c.N);
-            launch_n(c, CopyElems<int>{&c.ctr->grp[j], &c.ctr->nlist}, 1);
-        }
+                       &ct->sh_total, c.N, Clears{{&ct->r_wait[ring(round + kRing / 2)]}});
         r = read_counters(c);
         if (r) return r;
         if (c.hctr->err) return c.hctr->err;
         for (int j = 0; j < kShiftGroup && !done; j++) {
             shiftRounds++;
-            done = c.hctr->grp[j] == 0;
+            done = c.hctr->r_wait[ring(round0 + j)] == 0;
         }
         if (!done && shiftRounds > c.max_rounds) return GPUDT_ERR_NOCONVERGE;
     }
-    badCount = c.hctr->changed;
+    badCount = c.hctr->nbad;
     c.st.shiftRounds = shiftRounds;
     c.st.nBadShift = badCount;
     // remove the unshiftable sites in independent rounds
     int guard = 0;
     const long long recn = 4LL * c.cap_tris;
     while (badCount > 0) {
+        const int it0 = guard;
         for (int j = 0; j < kShiftGroup; j++) {
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist, 0, sizeof(int), c.stream));
-            launch_dev(c, BadSelectList{BadSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, c.ctr}, dropped},
-                       &c.ctr->sh_total, c.N);
-            launch_n(c, CopyElems<int>{&c.ctr->grp[j], &c.ctr->nlist}, 1);
+            const int it = it0 + j;
+            int *nsel = &ct->r_bad[ring(it)], *nrec = rec_word(c);
+            launch_dev(c, BadSelectList{BadSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, nsel}, dropped},
+                       &ct->sh_total, c.N, Clears{{&ct->r_bad[ring(it + kRing / 2)], rec_word(c, kRing / 2)}});
             const int round = next_round(c);
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nrec, 0, sizeof(int), c.stream));
             // a round selects at most the bad sites left (the grid is sized by them:
             // an empty round of this local-memory-heavy kernel then stays cheap)
             launch_dev(c, BadRemove{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.anchor, c.list, c.pos,
-                                    c.vstate, c.rec, round, c.N, c.ctr},
-                       &c.ctr->nlist, badCount);
-            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, c.ctr}, &c.ctr->nrec, recn);
+                                    c.vstate, c.rec, nrec, round, c.N, ct},
+                       nsel, badCount);
+            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, nrec, recn);
+            c.rec_round++;
         }
         GALPHA_CUDA(cudaGetLastError());
         r = read_counters(c);
@@ -753,8 +742,9 @@ int stage_shift(Ctx &c)
         if (c.hctr->err) return c.hctr->err;
         bool stuck = false;
         for (int j = 0; j < kShiftGroup && !stuck; j++) {
-            stuck = c.hctr->grp[j] == 0;
-            badCount -= c.hctr->grp[j];
+            const int done = c.hctr->r_bad[ring(it0 + j)];
+            stuck = done == 0;
+            badCount -= done;
         }
         if (stuck) break;
         guard += kShiftGroup;
@@ -871,12 +861,14 @@ struct MissingLocate {
     const int *list;
     int *loc;  // [nlist] encoded (t<<2)|edge, kind in bit 30..31 via separate array
     int *kind;
+    int *tag;  // neighbour slot an on-edge insertion voted for, or -1
     int *vote;
     int fallback;
     Counters *ct;
     __device__ void operator()(long long ii) const
     {
         int m = list[ii];
+        tag[ii] = -1;
         if (vstate[m] != VS_MISSING) {
             kind[ii] = -1;
             return;
@@ -900,8 +892,10 @@ struct MissingLocate {
             int nb = geti(tn[t], e);
             if (nb < 0) {
                 set_err(ct, GPUDT_ERR_TOPOLOGY, 61);
+                kind[ii] = -1;
                 return;
             }
+            tag[ii] = dtri(nb);
             atomicMin(&vote[dtri(nb)], m);
         }
     }
@@ -915,6 +909,7 @@ struct MissingInsert {
     int8_t *vstate;
     const int *list, *loc, *kind;
     Relink *rec;
+    int *nrec, *done;  // relink records, sites inserted or dropped
     int round, cap;
     Counters *ct;
     __device__ void operator()(long long ii) const
@@ -925,7 +920,7 @@ struct MissingInsert {
         int t = dtri(loc[ii]), i = dori(loc[ii]);
         if (k == 2) {
             vstate[p] = VS_DUP;
-            atomicAdd(&ct->changed, 1);
+            atomicAdd(done, 1);
             atomicAdd(&ct->ndup, 1);
             return;
         }
@@ -943,9 +938,9 @@ struct MissingInsert {
             tn[s1] = make_int4(-1, enc(s2, 2), enc(t, 1), 0);
             tn[s2] = make_int4(-1, enc(t, 2), enc(s1, 1), 0);
             fwd[t] = make_int4(enc(t, 0), enc(s1, 0), enc(s2, 0), 0);
-            push_rec(rec, ct, enc(t, 0), n.x);
-            push_rec(rec, ct, enc(s1, 0), n.y);
-            push_rec(rec, ct, enc(s2, 0), n.z);
+            push_rec(rec, nrec, enc(t, 0), n.x);
+            push_rec(rec, nrec, enc(s1, 0), n.y);
+            push_rec(rec, nrec, enc(s2, 0), n.z);
             vtri[p] = enc(t, 0);
             vtri[v1] = enc(t, 1);
             vtri[v2] = enc(t, 2);
@@ -981,10 +976,10 @@ struct MissingInsert {
             seti(fu, m1(j), enc(s2, 0));
             fwd[t] = ft;
             fwd[u] = fu;
-            push_rec(rec, ct, enc(t, 0), o1);
-            push_rec(rec, ct, enc(s1, 0), o2);
-            push_rec(rec, ct, enc(u, 0), ou1);
-            push_rec(rec, ct, enc(s2, 0), ou2);
+            push_rec(rec, nrec, enc(t, 0), o1);
+            push_rec(rec, nrec, enc(s1, 0), o2);
+            push_rec(rec, nrec, enc(u, 0), ou1);
+            push_rec(rec, nrec, enc(s2, 0), ou2);
             vtri[p] = enc(t, 0);
             vtri[v2] = enc(t, 1);
             vtri[v0] = enc(t, 2);
@@ -993,98 +988,91 @@ struct MissingInsert {
         }
         pos[p] = opos[p];
         vstate[p] = VS_SHIFTED;
-        atomicAdd(&ct->changed, 1);
+        atomicAdd(done, 1);
     }
 };
 
-struct ResetVotes {
+// The last launch of an insertion round: the relinks, and, independent of
+// them, the votes of the round taken back (a located site's triangle, and the
+// neighbour an on-edge insertion voted for) and the free list's count, which
+// pops that fell through to the tail may have driven below zero, reset so that
+// a later free_slot appends at index 0.  As launches of their own (two vote
+// resets, the tags, the clamp) these cost a round four launches more.
+struct VotesBack {
     int *vote;
-    const int4 *tn;
-    const int *loc, *kind;
+    const int *loc, *kind, *tag;
     __device__ void operator()(long long ii) const
     {
-        int k = kind[ii];
+        const int k = kind[ii];
         if (k < 0 || k == 2) return;
-        int t = dtri(loc[ii]);
-        vote[t] = 0x7fffffff;
+        vote[dtri(loc[ii])] = 0x7fffffff;
+        if (tag[ii] >= 0) vote[tag[ii]] = 0x7fffffff;
     }
 };
 
-struct ResetVotesEdge {
-    int *vote;
-    const int *list2;  // neighbour slots tagged for edge insertions
-    __device__ void operator()(long long ii) const { vote[list2[ii]] = 0x7fffffff; }
-};
-
-// Record the neighbour slot of every on-edge insertion (before the mesh changes).
-struct EdgeTags {
-    const int4 *tn;
-    const int *loc, *kind;
-    int *list2;
-    Counters *ct;
-    __device__ void operator()(long long ii) const
-    {
-        if (kind[ii] != 1) return;
-        int t = dtri(loc[ii]), e = dori(loc[ii]);
-        int nb = geti(tn[t], e);
-        if (nb < 0) return;
-        int k = atomicAdd(&ct->nlist2, 1);
-        list2[k] = dtri(nb);
+__global__ void __launch_bounds__(256) k_missing_finish(Relinker rl, const int *nrec, VotesBack vb, const int *nmiss,
+                                                        Counters *ct, Clears z)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (z.p[k]) *z.p[k] = 0;
+        if (ct->nfree < 0) ct->nfree = 0;
     }
-};
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const int nr = *nrec, nm = *nmiss;
+    for (int i = t; i < nr; i += stride) rl(i);
+    for (int i = t; i < nm; i += stride) vb(i);
+}
 
 int stage_missing(Ctx &c)
 {
     int r;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist, 0, sizeof(int), c.stream));
-    launch_n(c, CountState{c.vstate, VS_MISSING, c.list, c.ctr}, c.N);
-    r = read_counters(c);
-    if (r) return r;
-    int nmiss = c.hctr->nlist;
-    c.st.nMissing = nmiss;
-    if (nmiss == 0) return GPUDT_OK;
-    int *loc = c.aux, *kind = c.aux2 + 0;
-    // aux2 holds kind at [0, nmiss) ; edge tags in list2.  Rounds run in
-    // groups of c.missing_group between counter reads (a round after the last
-    // insertion finds no missing site and does nothing); each round's
-    // insertions are kept in ct->grp[].
+    Counters *ct = c.ctr;
+    // The list's length stays on the device until the first group of rounds
+    // has run.
+    launch_n(c, CountState{c.vstate, VS_MISSING, c.list, ct}, c.N);
+    int *loc = c.aux, *kind = c.aux2, *tag = c.list2;  // per list entry
+    // Rounds run in groups of c.missing_group between counter reads (a round
+    // after the last insertion finds no missing site and does nothing); each
+    // round's insertions are kept in its ring word.
     const int kMissingGroup = c.missing_group;
-    const long long recn = 4LL * c.cap_tris;
-    int rounds = 0, remaining = nmiss, dups = 0;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->ndup, 0, sizeof(int), c.stream));
-    while (remaining > 0) {
+    int rounds = 0, remaining = 1;
+    long long bound = c.N;  // of the list's length, for the grids
+    for (int it0 = 0; remaining > 0; it0 += kMissingGroup) {
         for (int j = 0; j < kMissingGroup; j++) {
-            int round = next_round(c);
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nrec, 0, sizeof(int), c.stream));
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist2, 0, sizeof(int), c.stream));
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
-            launch_n(c, MissingLocate{c.tv, c.tn, c.pos, c.opos, c.vtri, c.anchor, c.vstate, c.list, loc, kind,
-                                      c.vote, c.N, c.ctr},
-                     nmiss);
-            launch_n(c, EdgeTags{c.tn, loc, kind, c.list2, c.ctr}, nmiss);
-            launch_n(c, MissingInsert{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.vote, c.pos, c.opos,
-                                      c.vstate, c.list, loc, kind, c.rec, round, c.cap_tris, c.ctr},
-                     nmiss);
-            launch_n(c, ClampFree{c.ctr}, 1);  // a pop past the free list took tail slots
-            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, c.ctr}, &c.ctr->nrec, recn);
-            launch_n(c, ResetVotes{c.vote, c.tn, loc, kind}, nmiss);
-            launch_dev(c, ResetVotesEdge{c.vote, c.list2}, &c.ctr->nlist2, c.cap_tris);
-            launch_n(c, CopyElems<int>{&c.ctr->grp[j], &c.ctr->changed}, 1);
+            const int it = it0 + j, round = next_round(c);
+            int *nrec = rec_word(c), *done = &ct->r_mis[ring(it)];
+            launch_dev(c, MissingLocate{c.tv, c.tn, c.pos, c.opos, c.vtri, c.anchor, c.vstate, c.list, loc, kind, tag,
+                                        c.vote, c.N, ct},
+                       &ct->nmiss, bound);
+            launch_dev(c, MissingInsert{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.vote, c.pos, c.opos,
+                                        c.vstate, c.list, loc, kind, c.rec, nrec, done, round, c.cap_tris, ct},
+                       &ct->nmiss, bound);
+            const long long blocks = std::max(1ll, std::min((4 * bound + 255) / 256, (long long)c.sm_count * 8));
+            k_missing_finish<<<(unsigned)blocks, 256, 0, c.stream>>>(
+                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, nrec, VotesBack{c.vote, loc, kind, tag},
+                &ct->nmiss, ct, Clears{{&ct->r_mis[ring(it + kRing / 2)], rec_word(c, kRing / 2)}});
+            count_launch();
+            c.rec_round++;
         }
         GALPHA_CUDA(cudaGetLastError());
         r = read_counters(c);
         if (r) return r;
         if (c.hctr->err) return c.hctr->err;
         if (c.hctr->ntris > c.cap_tris) return GPUDT_ERR_NOMEM;
+        if (it0 == 0) {
+            bound = remaining = c.hctr->nmiss;
+            c.st.nMissing = remaining;
+        }
         for (int j = 0; j < kMissingGroup && remaining > 0; j++) {
-            const int done = c.hctr->grp[j];
+            const int done = c.hctr->r_mis[ring(it0 + j)];
             remaining -= done;
             rounds++;
             if (done == 0 || rounds > c.max_rounds) return GPUDT_ERR_NOCONVERGE;
         }
     }
-    dups = c.hctr->ndup;
-    c.st.nDuplicates = dups;
+    c.st.nDuplicates = c.hctr->ndup;
     c.st.missingRounds = rounds;
     return GPUDT_OK;
 }
@@ -1194,7 +1182,7 @@ struct FakeSelect {
                 }
             }
         }
-        warp_reserve(&ct->changed, pick ? 1 : 0);
+        warp_reserve(&ct->fk_removed, pick ? 1 : 0);
     }
 };
 
@@ -1364,16 +1352,7 @@ struct FakeRunJoin {
                 }
             }
         }
-        warp_reserve(&ct->changed, pick ? nmem : 0);
-    }
-};
-
-struct ZeroInts {
-    int *a, *b;
-    __device__ void operator()(long long) const
-    {
-        *a = 0;
-        if (b) *b = 0;
+        warp_reserve(&ct->fk_removed, pick ? nmem : 0);
     }
 };
 
@@ -1399,6 +1378,7 @@ struct FakeRemoveArgs {
     const double2 *pos;
     int8_t *vstate;
     Relink *rec;
+    int *nrec;
     int *cand;  // boundary-candidate vertices
     int round;
     Counters *ct;
@@ -1502,7 +1482,7 @@ __global__ void __launch_bounds__(32) k_fake_remove(FakeRemoveArgs a, const int 
         // every one of the d chain edges ends with exactly one relink record,
         // at rbase + its index (linked to a new triangle, or left as a hull edge)
         int rbase = 0;
-        if (lane == 0 && d > 0) rbase = atomicAdd(&a.ct->nrec, d);
+        if (lane == 0 && d > 0) rbase = atomicAdd(a.nrec, d);
         rbase = __shfl_sync(0xffffffffu, rbase, 0);
         __syncwarp();
         const int G = max(1, min(kFrPieces, d / kFrMinPiece));
@@ -1581,7 +1561,7 @@ __global__ void __launch_bounds__(32) k_fake_remove(FakeRemoveArgs a, const int 
             const int nrel = __shfl_sync(0xffffffffu, incl, 31);
             int cb = 0, fb = 0;
             if (lane == 0) {
-                cb = atomicAdd(&a.ct->nlist2, top);
+                cb = atomicAdd(&a.ct->ncand, top);
                 fb = nrel || nsh ? atomicAdd(&a.ct->nfree, nrel + nsh) : 0;
             }
             cb = __shfl_sync(0xffffffffu, cb, 0);
@@ -1774,8 +1754,7 @@ struct ConvexReset {
 int stage_boundary(Ctx &c)
 {
     int r;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist2, 0, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
+    Counters *ct = c.ctr;
     int *cand = c.aux;  // boundary candidates
     const int order[4] = {0, 2, 1, 3};
     const long long recn = 4LL * c.cap_tris;
@@ -1788,48 +1767,47 @@ int stage_boundary(Ctx &c)
     while (run_levels < 6 && (1LL << (4 * run_levels)) < (c.F + 3) / 4) run_levels++;
     // first pass: the four ring classes in turn (independent by construction);
     // then rounds of priority-minimal fakes among all that remain
-    for (int pass = 0; removed < c.F; pass++) {
+    for (int pass = 0, it = 0; removed < c.F; pass++) {
         if (pass > c.max_rounds / 4) return GPUDT_ERR_NOCONVERGE;
         // pass 0: three ring classes one fake at a time, then the last class
         // (a chain by then) as runs, one separator level after another; later
         // passes: priority rounds among the fakes left
         const int nsub = pass == 0 ? 3 + run_levels : 1;
-        for (int q = 0; q < nsub; q++) {
+        for (int q = 0; q < nsub; q++, it++) {
             int round = next_round(c);
-            launch_n(c, ZeroInts{&c.ctr->nlist, &c.ctr->nrec}, 1);
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->cand, 0, sizeof(int), c.stream));  // fan entries
+            int *nsel = &ct->r_fk[ring(it)], *nfan = &ct->r_fan[ring(it)], *nrec = rec_word(c);
             if (pass == 0 && q >= 3) {
                 // staging in alpha-stage buffers, idle until the mesh is final
                 int2 *stage = (int2 *)c.keys2;
                 int *rec5 = (int *)c.spectrum;
-                GALPHA_CUDA(cudaMemsetAsync(&c.ctr->runstage, 0, sizeof(int), c.stream));
-                launch_n(c, FakeRunStage{c.tv, c.tn, c.vstate, c.vtri, c.N, order[3], q - 3, stage, &c.ctr->runstage,
-                                         rec5, c.ctr},
+                launch_n(c, FakeRunStage{c.tv, c.tn, c.vstate, c.vtri, c.N, order[3], q - 3, stage,
+                                         &ct->r_stage[ring(it)], rec5, ct},
                          c.F);
                 launch_n(c, FakeRunJoin{c.vstate, c.N, order[3], q - 3, stage, rec5, c.list, fanoff, fanlen, fan,
-                                        &c.ctr->nlist, &c.ctr->cand, c.ctr},
+                                        nsel, nfan, ct},
                          c.F);
             } else
-                launch_n(c, FakeSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, fanoff, fanlen, fan, &c.ctr->nlist,
-                                       &c.ctr->cand, c.N, pass == 0 ? order[q] : -1, c.ctr},
+                launch_n(c, FakeSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, fanoff, fanlen, fan, nsel, nfan, c.N,
+                                       pass == 0 ? order[q] : -1, ct},
                          c.F);
             r = launch_fake_remove(c,
                                FakeRemoveArgs{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.list, fanoff, fanlen, fan,
-                                              c.pos, c.vstate, c.rec, cand, round, c.ctr},
-                               &c.ctr->nlist, c.F);
+                                              c.pos, c.vstate, c.rec, nrec, cand, round, ct},
+                               nsel, c.F);
             if (r) return r;
-            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, c.ctr}, &c.ctr->nrec, recn);
+            const int ahead = ring(it + kRing / 2);
+            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, nrec, recn,
+                       Clears{{&ct->r_fk[ahead], &ct->r_fan[ahead], &ct->r_stage[ahead], rec_word(c, kRing / 2)}});
+            c.rec_round++;
         }
         GALPHA_CUDA(cudaGetLastError());
         r = read_counters(c);
         if (r) return r;
         if (c.hctr->err) return c.hctr->err;
-        if (c.hctr->changed == removed) return GPUDT_ERR_NOCONVERGE;  // a full pass removed nothing
-        removed = c.hctr->changed;
+        if (c.hctr->fk_removed == removed) return GPUDT_ERR_NOCONVERGE;  // a full pass removed nothing
+        removed = c.hctr->fk_removed;
     }
-    r = read_counters(c);
-    if (r) return r;
-    int ncand = c.hctr->nlist2;
+    int ncand = c.hctr->ncand;
     GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist, 0, sizeof(int), c.stream));
     // per-vertex stamps of the convexify rounds: this arena region may hold
     // another stage's data (or a differently planned call's)
@@ -1997,6 +1975,7 @@ struct FlipApply {
     int8_t *eflag;
     bool first;  // first round: a losing candidate was tested one-sided, so all its edges stay marked
     const int *cand_n;  // candidates of the round (the launch count)
+    int *rec_n;         // relink records of the round
     long long rec_cap;  // relink records the array holds
     __device__ bool fresh(int x) const { return x >= 0 && atomicExch(&stamp[x], round) != round; }
     __device__ void operator()(long long ii) const
@@ -2054,7 +2033,7 @@ struct FlipApply {
         const int nc = *cand_n;  // the same for every thread of the launch
         if (4ll * nc <= rec_cap) {
             if (ii == 0) {
-                ct->nrec = 4 * nc;
+                *rec_n = 4 * nc;
                 *next_n = 2 * nc;
             }
             Relink *rr = rec + 4 * ii;
@@ -2063,14 +2042,14 @@ struct FlipApply {
             next[2 * ii + 1] = nn > 1 ? nx[1] : -1;
             const unsigned m = __activemask();
             const int wins = __popc(__ballot_sync(m, win));
-            if ((int)(threadIdx.x & 31) == __ffs(m) - 1 && wins) atomicAdd(&ct->nflips, wins);
+            if ((int)(threadIdx.x & 31) == __ffs(m) - 1 && wins) atomicAdd(&ct->flips_total, wins);
             return;
         }
         // one atomic per warp for each of the records, the flip count and the next list
-        const int rb = warp_reserve(&ct->nrec, win ? 4 : 0);
+        const int rb = warp_reserve(rec_n, win ? 4 : 0);
         if (win)
             for (int k = 0; k < 4; k++) rec[rb + k] = r4[k];
-        warp_reserve(&ct->nflips, win ? 1 : 0);
+        warp_reserve(&ct->flips_total, win ? 1 : 0);
         const int nb = warp_reserve(next_n, nn);
         for (int k = 0; k < nn; k++) next[nb + k] = nx[k];
     }
@@ -2087,109 +2066,140 @@ struct FlipReset {
     }
 };
 
-// Start of a flip round: the next list becomes current (counts stay in the
-// counter block; the host alternates the list buffers).
-struct FlipRoundStart {
-    int p;  // parity of the round: act[p] is current
-    Counters *ct;
-    __device__ void operator()(long long) const
-    {
-        ct->act[1 - p] = 0;
-        ct->flips_total += ct->nflips;
-        ct->nflips = 0;
-        ct->cand = 0;
-        ct->nrec = 0;
+// The last launch of a flip round: the relinks and, independent of them, the
+// votes of the round's candidates taken back; it clears the words of the round
+// kRing / 2 ahead.
+__global__ void __launch_bounds__(256) k_flip_finish(Relinker rl, const int *nrec, FlipReset rs, const int *ncand,
+                                                     Clears z)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (z.p[k]) *z.p[k] = 0;
     }
-};
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const int nr = *nrec, nc = *ncand;
+    for (int i = t; i < nr; i += stride) rl(i);
+    for (int i = t; i < nc; i += stride) rs(i);
+}
 
 // The tail of the stage: once the active list is short, whole rounds run
 // inside ONE block, with __syncthreads between their phases instead of a launch
 // per phase (long flip chains -- a retriangulated hull pocket, a dense cluster
-// -- otherwise cost five launches per round for a handful of flips).  The same
+// -- otherwise cost three launches per round for a handful of flips).  The same
 // functors run in the same phase order with consecutive round ids, so the mesh
 // is the one the launched rounds produce.  The block stops when the list
 // empties, when a round's list exceeds `leave` (the host goes back to launched
-// rounds) or after max_rounds; no thread ever waits on another block.
+// rounds) or after max_rounds; no thread ever waits on another block.  It
+// clears a round's ring words before using them, and leaves all of them zero
+// but the current list length.
 constexpr int kTailThreads = 1024;
 // c.tail_enter: the host hands over at or below this many active triangles;
 // c.tail_leave: the block hands back above this many.
 
 __global__ void __launch_bounds__(kTailThreads) k_flip_tail(FlipCheck ck, FlipApply ap, Relinker rl, FlipReset rs,
-                                                             int *l0, int *l1, int p0, int round0,
+                                                             int *l0, int *l1, int k0, int round0,
                                                              int max_rounds, int leave)
 {
     Counters *ct = ck.ct;
     int k = 0;
     for (; k < max_rounds; k++) {
-        const int p = (p0 + k) & 1;
-        const int n = *(volatile int *)&ct->act[p];
+        const int w = (k0 + k) % kRing, w1 = (k0 + k + 1) % kRing;
+        const int n = *(volatile int *)&ct->r_act[w];
         if (n == 0 || n > leave) break;
-        if (threadIdx.x == 0) FlipRoundStart{p, ct}(0);
+        if (threadIdx.x == 0) {
+            ct->r_cand[w] = 0;
+            ct->r_frec[w] = 0;
+            ct->r_act[w1] = 0;
+        }
         __syncthreads();
         const int round = round0 + k;
-        ck.act = p ? l1 : l0;
+        const bool odd = (k0 + k) & 1;
+        ck.act = odd ? l1 : l0;
+        ck.cand_n = &ct->r_cand[w];
         for (int i = threadIdx.x; i < n; i += kTailThreads) ck(i);
         __syncthreads();
-        const int nc = *(volatile int *)&ct->cand;
-        ap.next = p ? l0 : l1;
-        ap.next_n = &ct->act[1 - p];
+        const int nc = *(volatile int *)&ct->r_cand[w];
+        ap.next = odd ? l0 : l1;
+        ap.next_n = &ct->r_act[w1];
+        ap.cand_n = &ct->r_cand[w];
+        ap.rec_n = &ct->r_frec[w];
         ap.round = round;
         for (int i = threadIdx.x; i < nc; i += kTailThreads) ap(i);
         __syncthreads();
-        const int nr = *(volatile int *)&ct->nrec;
+        const int nr = *(volatile int *)&ct->r_frec[w];
         rl.round = round;
         for (int i = threadIdx.x; i < nr; i += kTailThreads) rl(i);
         for (int i = threadIdx.x; i < nc; i += kTailThreads) rs(i);  // independent of the relinks
         __syncthreads();
     }
+    const int w = (k0 + k) % kRing;
+    if (threadIdx.x < kRing) {
+        ct->r_cand[threadIdx.x] = 0;
+        ct->r_frec[threadIdx.x] = 0;
+        if ((int)threadIdx.x != w) ct->r_act[threadIdx.x] = 0;
+    }
     if (threadIdx.x == 0) ct->tail_rounds = k;
 }
 
-struct AllAlive {
+// Start of the stage, four slots per thread: no vote (unsigned words start at
+// the maximum), no stamp, and the edges still to be tested: none marked before
+// a first launched round (it tests all), all when the in-block rounds start
+// from the list of live slots, made here (the arrays are 256-byte aligned).
+struct FlipInit {
     const int4 *tv;
-    int *list;
-    int *count;
-    __device__ void operator()(long long i) const
+    int *vote, *stamp;
+    int8_t *eflag;
+    int *list, *count;  // live slots (null: not wanted)
+    int nt, cap;
+    __device__ void operator()(long long q) const
     {
-        if (tv[i].x >= 0) {
-            int k = atomicAdd(count, 1);
-            list[k] = (int)i;
+        const int s = 4 * (int)q;
+        const unsigned char e = list ? 7 : 0;
+        if (s + 3 < cap) {
+            *(int4 *)(stamp + s) = make_int4(-1, -1, -1, -1);
+            *(uchar4 *)(eflag + s) = make_uchar4(e, e, e, e);
+        } else {
+            for (int k = s; k < cap; k++) {
+                stamp[k] = -1;
+                eflag[k] = (int8_t)e;
+            }
+        }
+        if (s + 3 < nt) *(int4 *)(vote + s) = make_int4(-1, -1, -1, -1);
+        for (int k = s; k < min(s + 4, nt); k++) {
+            if (s + 3 >= nt) vote[k] = -1;
+            if (list && tv[k].x >= 0) list[atomicAdd(count, 1)] = k;
         }
     }
 };
 
+// The counters on the host are those of the boundary or constraint stage's
+// last read: nothing in between changes ntris.
 int stage_flip(Ctx &c)
 {
-    int r = read_counters(c);
-    if (r) return r;
+    int r;
+    Counters *ct = c.ctr;
     int nt = c.hctr->ntris;
     int *lists[2] = {c.list, c.list2};
     int *prop = c.aux, *target = c.aux2, *cands = c.inc, *stamp = c.stamp;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->act[0], 0, 2 * sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->flips_total, 0, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nflips, 0, sizeof(int), c.stream));
     // the first launched round tests every slot directly; the in-block tail
     // (small meshes) starts from a list of the live slots
-    if (nt <= c.tail_enter) launch_n(c, AllAlive{c.tv, lists[0], &c.ctr->act[0]}, nt);
-    // marked edges: none before the first launched round (it tests all), all
-    // when the in-block rounds start from the list of live slots
-    GALPHA_CUDA(cudaMemsetAsync(c.eflag, nt <= c.tail_enter ? 7 : 0, (size_t)c.cap_tris, c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.vote, 0xff, sizeof(int) * (size_t)nt, c.stream));  // unsigned votes start at max
-    GALPHA_CUDA(cudaMemsetAsync(stamp, 0xff, sizeof(int) * (size_t)c.cap_tris, c.stream));
+    launch_n(c, FlipInit{c.tv, c.vote, stamp, c.eflag, nt <= c.tail_enter ? lists[0] : nullptr, &ct->r_act[0], nt,
+                         c.cap_tris},
+             ((long long)c.cap_tris + 3) / 4);
     const long long capn = c.cap_tris, recn = 4LL * c.cap_tris;
     int rounds = 0;
     long long known = nt;  // active-list length at `rounds`, as last read (nt bounds the first)
     while (known > 0) {
         if (known <= c.tail_enter) {
-            const int p = rounds & 1;
             const int round0 = next_round(c);
             k_flip_tail<<<1, kTailThreads, 0, c.stream>>>(
-                FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &c.ctr->cand, c.ctr, c.eflag,
-                          c.chash, c.cmask},
+                FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, nullptr, ct, c.eflag, c.chash,
+                          c.cmask},
                 FlipApply{c.tv, c.tn, c.fwd, c.epoch, c.vtri, c.vote, stamp, nullptr, nullptr, prop, target, cands,
-                          c.rec, 0, c.ctr, c.eflag, false, &c.ctr->cand, 3ll * c.cap_tris},
-                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, 0, c.ctr}, FlipReset{c.vote, target, cands},
-                lists[0], lists[1], p, round0, c.max_rounds + 1 - rounds, c.tail_leave);
+                          c.rec, 0, ct, c.eflag, false, nullptr, nullptr, 3ll * c.cap_tris},
+                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, 0, ct}, FlipReset{c.vote, target, cands},
+                lists[0], lists[1], rounds, round0, c.max_rounds + 1 - rounds, c.tail_leave);
             count_launch();
             GALPHA_CUDA(cudaGetLastError());
             r = read_counters(c);
@@ -2198,39 +2208,42 @@ int stage_flip(Ctx &c)
             const int k = c.hctr->tail_rounds;
             skip_rounds(c, round0, k - 1);
             rounds += k;
-            known = c.hctr->act[rounds & 1];
+            known = c.hctr->r_act[ring(rounds)];
             if (known == 0) break;
             if (rounds > c.max_rounds) return GPUDT_ERR_NOCONVERGE;
             if (known <= c.tail_leave) return set_last_error("flip: in-block rounds stopped early"), GPUDT_ERR_TOPOLOGY;
         }
         for (int k = 0; k < c.flip_sync; k++) {
-            int p = rounds & 1;
+            const int p = rounds & 1, w = ring(rounds), w1 = ring(rounds + 1), ahead = ring(rounds + kRing / 2);
             int round = next_round(c);
-            launch_n(c, FlipRoundStart{p, c.ctr}, 1);
             if (rounds == 0)
-                launch_n(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &c.ctr->cand, c.ctr,
+                launch_n(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &ct->r_cand[w], ct,
                                       c.eflag, c.chash, c.cmask},
                          nt);
             else
-                launch_dev(c, FlipCheck{c.tv, c.tn, c.pos, lists[p], c.vote, prop, target, cands, &c.ctr->cand,
-                                        c.ctr, c.eflag, c.chash, c.cmask},
-                           &c.ctr->act[p], capn);
-            launch_dev(c, FlipApply{c.tv, c.tn, c.fwd, c.epoch, c.vtri, c.vote, stamp, lists[1 - p],
-                                    &c.ctr->act[1 - p], prop, target, cands, c.rec, round, c.ctr, c.eflag,
-                                    rounds == 0, &c.ctr->cand, 3ll * c.cap_tris},
-                       &c.ctr->cand, capn);
-            launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, c.ctr}, &c.ctr->nrec, recn);
-            launch_dev(c, FlipReset{c.vote, target, cands}, &c.ctr->cand, capn);
+                launch_dev(c, FlipCheck{c.tv, c.tn, c.pos, lists[p], c.vote, prop, target, cands, &ct->r_cand[w], ct,
+                                        c.eflag, c.chash, c.cmask},
+                           &ct->r_act[w], capn);
+            launch_dev(c, FlipApply{c.tv, c.tn, c.fwd, c.epoch, c.vtri, c.vote, stamp, lists[1 - p], &ct->r_act[w1],
+                                    prop, target, cands, c.rec, round, ct, c.eflag, rounds == 0, &ct->r_cand[w],
+                                    &ct->r_frec[w], 3ll * c.cap_tris},
+                       &ct->r_cand[w], capn);
+            const long long blocks = std::max(1ll, std::min((recn + 255) / 256, (long long)c.sm_count * 8));
+            k_flip_finish<<<(unsigned)blocks, 256, 0, c.stream>>>(
+                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, &ct->r_frec[w],
+                FlipReset{c.vote, target, cands}, &ct->r_cand[w],
+                Clears{{&ct->r_act[ahead], &ct->r_cand[ahead], &ct->r_frec[ahead]}});
+            count_launch();
             rounds++;
         }
         GALPHA_CUDA(cudaGetLastError());
         r = read_counters(c);
         if (r) return r;
         if (c.hctr->err) return c.hctr->err;
-        known = c.hctr->act[rounds & 1];
+        known = c.hctr->r_act[ring(rounds)];
         if (rounds > c.max_rounds) return GPUDT_ERR_NOCONVERGE;
     }
-    c.st.nFlips = c.hctr->flips_total + c.hctr->nflips;
+    c.st.nFlips = c.hctr->flips_total;
     c.st.flipRounds = rounds;
     return GPUDT_OK;
 }
@@ -2929,9 +2942,8 @@ int ensure_outtri(Ctx &c)
 
 int stage_compact(Ctx &c)
 {
-    int r = read_counters(c);
-    if (r) return r;
-    int nt = c.hctr->ntris;
+    int r;
+    int nt = c.hctr->ntris;  // as of the flip stage's last read
     launch_n(c, MarkAlive{c.tv, c.aux}, nt);
     r = exclusive_scan_int(c, c.aux, c.aux2, nt, &c.ctr->nlist);
     if (r) return r;
@@ -2942,7 +2954,7 @@ int stage_compact(Ctx &c)
              nt);
     c.outtri_ready = c.want_outtri;
     GALPHA_CUDA(cudaGetLastError());
-    r = read_counters(c);
+    r = read_counters(c, true);
     if (r) return r;
     c.nT_out = c.hctr->nlist;
     return GPUDT_OK;

@@ -27,7 +27,12 @@ constexpr int kSpinLimit = 1 << 22;              // bound of every look-back wai
 constexpr int kBlockRun = 1 << 16;
 constexpr int kShiftGroupDefault = 4, kMissingGroupDefault = 2, kFlipSyncDefault = 4;
 constexpr int kTailEnterDefault = 4096, kTailLeaveDefault = 32768;
-constexpr int kMaxGroup = 8;  // Counters::grp holds one group's per-round counts               // longest exact-sort run for one block (default)
+constexpr int kMaxGroup = 8;   // rounds between two counter reads
+// Per-round counts live in rings of kRing words: round k counts in word
+// k mod kRing and clears the word of round k + kRing / 2, so that the words of
+// a group of rounds stay readable until the next group's are needed and no
+// launch is spent on clearing them (all are zero when a call starts).
+constexpr int kRing = 2 * kMaxGroup;
 
 // vertex states
 enum : int8_t {
@@ -46,38 +51,49 @@ struct Counters {
     int nfree;      // entries of the free-slot stack
     int nlist;      // generic work-list length
     int nlist2;     // second work list
-    int nrec;       // relink records this round
     int changed;    // generic progress flag / count
     int err;        // first error code (GPUDT_ERR_*), 0 if none
     int errinfo;    // stage-specific detail of the first error
     int nisland;    // island pixels
-    int nflips;     // flips this round
     int nties;      // exact spectrum ties merged
-    int act[2];     // flip: active-list lengths (ping-pong)
-    int cand;       // flip: candidates this round
     int flips_total;
     int escalate;   // island repair could not stay local: redo the Voronoi stage globally
     unsigned long long exact_compares;
     unsigned long long exact_orient;
     unsigned long long exact_incircle;
     unsigned long long exact_attached;
-    // predicate stage counts, each spread over 64 counters (one per warp id mod 64)
-    unsigned long long filt_spread[64];  // in-circle tests decided by the FP64 filter
-    unsigned long long icc_spread[64];   // in-circle tests, all stages
-    unsigned long long ori_spread[64];   // orientation tests of the mesh stages, all stages
-    unsigned long long ori64_spread[64]; // orientation tests decided by the FP64 filter
     int qcount[12];  // alpha query: [type*4 + class], type 0 points, 1 edges, 2 triangles
     int qrank;       // alpha query: largest spectrum rank <= alpha (-1 if alpha < 0)
     int qpad;
     double qalpha;   // alpha query: the alpha value classified
     int tail_rounds; // flip: rounds run by the last in-block tail launch
-    int runstage;    // fake runs: staged fan entries
     int nlong;       // key sort: out-of-order pairs recorded in groups too long for one thread
     int nhuge;       // alpha ranks: runs too long for one block, listed for the multi-block merge
-    int sh_n[2];     // shift: sites dropped by the current / previous optimistic iteration
     int sh_total;    // shift: all dropped sites listed so far
-    int grp[8];      // per-round counts of a group of rounds run between two counter reads
+    int nbad;        // shift: sites that cannot be shifted
+    int nhull;       // links: hull edges
+    int nmiss;       // missing sites listed
     int ndup;        // missing sites found to be exact duplicates
+    int fk_removed;  // fake removal: fakes removed so far
+    int ncand;       // fake removal: boundary candidates listed
+    // per-round rings (kRing)
+    int r_drop[kRing];   // shift: sites dropped by an optimistic iteration
+    int r_wait[kRing];   // shift: sites left waiting by a priority round
+    int r_bad[kRing];    // shift: bad sites removed in a round
+    int r_mis[kRing];    // missing sites inserted (or dropped) in a round
+    int r_rec[kRing];    // relink records of a round (bad sites, missing sites, fakes)
+    int r_fk[kRing];     // fake removal: units selected
+    int r_fan[kRing];    // fake removal: stored fan entries
+    int r_stage[kRing];  // fake removal: staged fan entries of runs
+    int r_act[kRing];    // flip: active-list length of a round
+    int r_cand[kRing];   // flip: candidates of a round
+    int r_frec[kRing];   // flip: relink records of a round
+    // predicate stage counts, each spread over 64 counters (one per warp id mod
+    // 64); last, because only a call's final read takes them along
+    unsigned long long filt_spread[64];  // in-circle tests decided by the FP64 filter
+    unsigned long long icc_spread[64];   // in-circle tests, all stages
+    unsigned long long ori_spread[64];   // orientation tests of the mesh stages, all stages
+    unsigned long long ori64_spread[64]; // orientation tests decided by the FP64 filter
     int qdone;       // alpha query: blocks that have added their counts
 };
 
@@ -188,6 +204,7 @@ struct Ctx {
     int sort_passes = 0;  // radix passes of the last radix_sort call
     bool fused_done = false;  // triangles came from the fused colour + dual kernel
     int round_counter = 1;    // ids of operation rounds (per handle: stamps live in its arena)
+    int rec_round = 0;        // rounds of this call that took a word of Counters::r_rec
     int host_reads = 0;       // device -> host reads (each a stream synchronisation) of the current call
 
     // constrained edges of the current call (GPUDTPARAMS.nConstraints > 0)
@@ -236,7 +253,8 @@ void set_last_error(const char *text);
 
 // Reserve device buffers for V vertices, T texture, cap triangles.
 int reserve(Ctx &c, int V, int T, int cap_tris, bool alpha);
-int read_counters(Ctx &c);
+// Counter block -> host mirror; `all`: the predicate stage counts too.
+int read_counters(Ctx &c, bool all = false);
 // Small device -> host read (bytes a multiple of 4, src 4-byte aligned): a
 // kernel writes into mapped pinned memory, so the read never queues behind
 // large copies on the copy engines; synchronises the handle's stream.
@@ -273,11 +291,22 @@ __global__ void __launch_bounds__(256, MINB) k_for_each_occ(F f, long long n)
     for (; i < n; i += stride) f(i);
 }
 
+// Counter words a launch sets to zero (null: none): words no thread of the
+// same launch uses.
+struct Clears {
+    int *p[4] = {nullptr, nullptr, nullptr, nullptr};
+};
+
 // Grid-stride launch over [0, *n) with the count read on the device, so a
 // round of kernels can run without the host learning its size.
 template <class F>
-__global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n)
+__global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n, Clears z)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (z.p[k]) *z.p[k] = 0;
+    }
     long long nn = *n;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -285,13 +314,13 @@ __global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n)
 }
 
 template <class F>
-inline void launch_dev(const Ctx &c, F f, const int *n_dev, long long max_n)
+inline void launch_dev(const Ctx &c, F f, const int *n_dev, long long max_n, const Clears &z = Clears())
 {
     if (max_n <= 0) return;
     long long blocks = (max_n + 255) / 256;
     long long maxb = (long long)c.sm_count * 8;
     if (blocks > maxb) blocks = maxb;
-    k_for_each_dev<<<(unsigned)blocks, 256, 0, c.stream>>>(f, n_dev);
+    k_for_each_dev<<<(unsigned)blocks, 256, 0, c.stream>>>(f, n_dev, z);
     count_launch();
 }
 

@@ -1,0 +1,31 @@
+"""GPU tests of the round loops' device-side counts (shifting, missing sites,
+fake removal, flips): clustered input that needs more rounds than a ring of
+per-round counts holds, under schedules that read the counters after every
+round, after groups of eight, and only at the end, with and without the
+in-block flip tail.  The triangulation must be the oracle's every time."""
+import numpy as np
+import pytest
+
+import galpha_b200 as G
+from galpha_b200 import datasets as D
+from dtcheck import canon_set
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [4, 1023, 20001])
+@pytest.mark.parametrize("sched", [(1, 1, 1, 0, 1), (8, 8, 64, 0, 1), (3, 5, 7, 2000, 2001), (0, 0, 0, -1, 0)])
+def test_rounds_under_schedules(n, sched):
+    pts = D.gaussian_blobs(n, 17, nblobs=3, sigma=0.02)
+    pts[::7] = D.uniform_points(len(pts[::7]), 18) * 2.0 - 1.0  # far points: long chains of flips
+    eng = G.Engine()
+    try:
+        eng.set_schedule(*sched)
+        for _ in range(2):  # the handle's second call starts from the first one's words
+            dt = eng.triangulate(G.GPUDTParams(pts, fboSize=256))
+            assert canon_set(dt.vtx) == canon_set(O.dt(pts)[0])
+    finally:
+        eng.close()
+    if n > 20000 and sched[2] == 1:
+        assert dt.status.flipRounds > 16 and dt.status.missingRounds > 2
