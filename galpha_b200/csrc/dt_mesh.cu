@@ -1620,25 +1620,33 @@ static int launch_fake_remove(Ctx &c, const FakeRemoveArgs &a, const int *n_dev,
 }
 
 // Convexity check of a boundary candidate: finds its hull edges (u->v, v->w)
-// and reports reflex vertices (orient(u,v,w) < 0).
+// and reports reflex vertices (orient(u,v,w) < 0).  A hull vertex's fan has no
+// bound (a far point over a collinear row of thousands sees every one of
+// them), so the walks are bounded only against a broken mesh; a walk that runs
+// out gives no answer.
+constexpr int kMaxHullWalk = 1 << 24;
+
 __device__ bool hull_neighbours(const int4 *tv, const int4 *tn, int v, int start, int *u, int *w, int *tin,
                                 int *tout)
 {
     // clockwise to the outgoing hull edge v->w (edge opposite b of (v,a,b) ... )
     int e = start;
-    for (int guard = 0; guard < 8 * kMaxFan; guard++) {
+    bool found = false;
+    for (int guard = 0; guard < kMaxHullWalk && !found; guard++) {
         int t = dtri(e), i = dori(e);
         int nx = geti(tn[t], m1(i));  // across (v, a)
         if (nx < 0) {
             *w = geti(tv[t], p1(i));
             *tout = enc(t, m1(i));
-            break;
+            found = true;
+        } else {
+            e = enc(dtri(nx), m1(dori(nx)));
+            if (e == start) return false;  // interior vertex
         }
-        e = enc(dtri(nx), m1(dori(nx)));
-        if (e == start) return false;  // interior vertex
     }
+    if (!found) return false;
     e = start;
-    for (int guard = 0; guard < 8 * kMaxFan; guard++) {
+    for (int guard = 0; guard < kMaxHullWalk; guard++) {
         int t = dtri(e), i = dori(e);
         int nx = geti(tn[t], p1(i));  // across (b, v)
         if (nx < 0) {

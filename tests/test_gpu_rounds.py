@@ -8,7 +8,7 @@ import pytest
 
 import galpha_b200 as G
 from galpha_b200 import datasets as D
-from dtcheck import canon_set
+from dtcheck import canon_set, compare_dt
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +29,18 @@ def test_rounds_under_schedules(n, sched):
         eng.close()
     if n > 20000 and sched[2] == 1:
         assert dt.status.flipRounds > 16 and dt.status.missingRounds > 2
+
+
+@pytest.mark.parametrize("row", [200, 511, 513, 1000])
+def test_hull_vertex_with_a_long_fan(engine, row):
+    """A far point over a collinear row sees every segment of it, so its fan on
+    the hull is as long as the row; the walks to its hull neighbours must reach
+    the ends (they once gave up after 512 triangles)."""
+    y = np.arange(row + 1) / 4096.0
+    line = np.stack([np.zeros(row + 1), y], axis=1)
+    rest = D.uniform_points(4000, row) * [1.0, y[-1]] + [1e-3, 0.0]
+    far = np.array([[-0.6 * y[-1], 0.47 * y[-1]], [-0.7 * y[-1], 0.53 * y[-1]]])
+    pts = np.concatenate([line, rest, far])
+    dt = engine.triangulate(G.GPUDTParams(pts, fboSize=4096))
+    ok, rep = compare_dt(pts, dt.vtx, dt.tri)
+    assert ok, rep
