@@ -1,14 +1,14 @@
 // alpha.cu -- alpha spectrum and per-simplex intervals on the device.
 //
 // Stage map (reference -> here):
-//   computeTriEdgeCount + exclusive_scan +          k_edge_count + scan: the reference's
-//   computeEdgeTriMap (kernel.cu:138-217)           ownership and numbering rule
-//   computeTriangleRo / computeEdgeRo /             k_tri_keys / k_edge_keys: birth times in
+//   computeTriEdgeCount + exclusive_scan +          k_alpha_keys: the reference's ownership
+//   computeEdgeTriMap (kernel.cu:138-217)           and numbering rule (offsets by look-back)
+//   computeTriangleRo / computeEdgeRo /             k_alpha_keys: birth times in
 //   processAttached (kernel.cu:219-358,             double-double (<= 1 ulp, certified),
 //   predicates.h:1297-1444)                         slivers recomputed exactly; attached test
 //                                                   filtered then exact (closed disc)
-//   thrust::remove_if x2 (Alpha_Shapes_2D.cu:       unattached edges compacted by a scan
-//   276-281)
+//   thrust::remove_if x2 (Alpha_Shapes_2D.cu:       k_alpha_keys: unattached edges compacted
+//   276-281)                                        by the same look-back
 //   thrust::sort_by_key (Alpha_Shapes_2D.cu:317)    radix_sort: LSD radix sort of the FP64
 //                                                   bit patterns with an int payload
 //   markSpectrum + sorT odd-even rounds +           k_mark_runs / k_resolve_runs: every run
@@ -108,20 +108,6 @@ __device__ __forceinline__ double rho_tri(double2 A, double2 B, double2 C, bool 
 }
 
 // ------------------------------------------------------------------ kernels
-struct EdgeCount {
-    const int4 *cv, *cn;
-    int *cnt;
-    __device__ void operator()(long long ii) const
-    {
-        int t = (int)ii;
-        int4 v = cv[t], n = cn[t];
-        int k = 0;
-        for (int i = 0; i < 3; i++)
-            if (geti(v, p1(i)) < geti(v, m1(i)) || geti(n, i) == -1) k++;
-        cnt[t] = k;
-    }
-};
-
 // The exact attached test, called with coordinates by value: the caller then
 // keeps its operands in registers (an array argument would have to live in
 // local memory on the hot path, for a call that almost never happens).
@@ -131,64 +117,204 @@ __device__ __noinline__ int attached_exact_v(double ix, double iy, double jx, do
     return attached_exact(i, j, k);
 }
 
-// Triangle keys + owned edges + attached test.
-struct TriKeys {
+// Triangle keys, edge numbering, attached tests and edge keys in one pass over
+// the triangles.  A block takes the next tile of kAkTile triangles by ticket,
+// computes their birth times, which edges they own and which of those are
+// unattached (their birth times stay in shared memory), and finds the edges
+// and the unattached edges of all earlier tiles by decoupled look-back; then
+// it writes the tile's edges and edge keys at their places.  The loads are a
+// triangle's three records, its corners and, for an owned edge its own corner
+// leaves unattached, the corner across it; bound by the latency of those
+// gathers (issue slots 38 % busy at 32 warps per SM, which the registers of the
+// double-double arithmetic allow), so a round's records are loaded one round
+// ahead, and by the wait for earlier tiles: 4 triangles per thread take 0.57
+// ms at 8.4 M triangles, 2 take 0.64, 1 takes 0.75, 8 by blocks of 128 take
+// 0.80 (longer chains ahead of the tiles that wait).  As five launches (edge
+// counts, a scan, keys, a scan over the edges, edge keys from a second gather)
+// it took 0.77 ms, and a counter read between the first and the third.
+// A status word holds kind (bits 63-62), the edges (61-31) and the unattached
+// edges (30-0) of its tile or of all tiles up to it; fewer than 2^31 edges.
+constexpr int kAkSpinLimit = 1 << 22;
+constexpr int kAkThreads = 256, kAkItems = 4, kAkTile = kAkThreads * kAkItems;
+constexpr unsigned long long kAkAgg = 1ull << 62, kAkInc = 2ull << 62, kAkVal = (1ull << 62) - 1;
+
+struct AlphaKeysArgs {
     const int4 *cv, *cn;
     const int4 *gv;  // the triangles with the ids that index P
     const double2 *P;
-    const int *e_off;
+    int nT;
+    int *e_off;
     unsigned long long *keys;
     int *vals;
-    int4 *edges;    // p1, p2, tIndex, vOpp
-    int *unatt;     // 1 if the edge enters the spectrum
-    int *edge_ro;
+    int *edges;     // enc(tIndex, vOpp)
+    int *edge_ro;   // 0 for attached edges
     int *slivers;
+    unsigned long long *status;  // [tiles], zero; then the ticket
+    int tiles;
     Counters *ct;
-    __device__ void operator()(long long ii) const
-    {
-        int t = (int)ii;
-        int4 v = cv[t], n = cn[t];
-        const int4 g = gv[t];
-        const double2 Q[3] = {P[g.x], P[g.y], P[g.z]};
-        const double2 A = Q[0], B = Q[1], C = Q[2];
-        bool sl;
-        double r = rho_tri(A, B, C, &sl);
-        keys[1 + t] = (unsigned long long)__double_as_longlong(r);
-        vals[1 + t] = t;
-        if (sl) {
-            int k = atomicAdd(&ct->nlist2, 1);
-            slivers[k] = t;
-        }
-        int e = e_off[t];
+};
+
+__global__ void __launch_bounds__(kAkThreads, 4) k_alpha_keys(AlphaKeysArgs A)
+{
+    __shared__ double s_rho[3 * kAkTile];  // birth time of edge i of the tile's triangle j at [i][j]
+    __shared__ int s_part[kAkItems * (kAkThreads / 32)];
+    __shared__ int s_tile;
+    __shared__ unsigned long long s_excl;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = atomicAdd((int *)(A.status + A.tiles), 1);
+    __syncthreads();
+    const int tile = s_tile;
+    unsigned flags[kAkItems];  // bits 0-2 owned edges, 3-5 unattached ones
+    int incl[kAkItems], cnt[kAkItems];  // owned | unattached << 16
+    const long long t0 = (long long)tile * kAkTile + threadIdx.x;
+    int4 v, n, g;  // the next triangle's records, loaded one round ahead
+    if (t0 < A.nT) {
+        v = A.cv[t0];
+        n = A.cn[t0];
+        g = A.gv[t0];
+    }
+#pragma unroll 1
+    for (int u = 0; u < kAkItems; u++) {
+        const int j = u * kAkThreads + threadIdx.x;
+        const long long t = t0 + u * kAkThreads;
+        unsigned f = 0;
+        if (t < A.nT) {
+            const double2 Q[3] = {A.P[g.x], A.P[g.y], A.P[g.z]};
+            // the corner across each owned edge: one word of its triangle, in
+            // flight with the corners
+            int nb[3], opp[3];
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            int a = geti(v, p1(i)), b = geti(v, m1(i));
-            int nb = geti(n, i);
-            if (!(a < b || nb == -1)) continue;
-            edges[e] = make_int4(a, b, t, i);
-            const double2 pa = Q[p1(i)], pb = Q[m1(i)], pk = Q[i];
-            double qa[2] = {pa.x, pa.y}, qb[2] = {pb.x, pb.y}, qk[2] = {pk.x, pk.y};
-            int att = attached_filter(qa, qb, qk);
-            if (att == 2) {
-                atomicAdd(&ct->exact_attached, 1ull);
-                att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, pk.x, pk.y);
+            for (int i = 0; i < 3; i++) {
+                nb[i] = geti(n, i);
+                const bool own = geti(v, p1(i)) < geti(v, m1(i)) || nb[i] == -1;
+                f |= own ? 1u << i : 0u;
+                opp[i] = own && nb[i] >= 0 ? ((const int *)A.gv)[4ll * dtri(nb[i]) + dori(nb[i])] : -1;
             }
-            if (att == 0 && nb >= 0) {
-                double2 po = P[geti(gv[dtri(nb)], dori(nb))];
-                double qo[2] = {po.x, po.y};
-                att = attached_filter(qa, qb, qo);
+            if (u + 1 < kAkItems && t + kAkThreads < A.nT) {
+                v = A.cv[t + kAkThreads];
+                n = A.cn[t + kAkThreads];
+                g = A.gv[t + kAkThreads];
+            }
+            double2 O[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) O[i] = opp[i] >= 0 ? A.P[opp[i]] : make_double2(0.0, 0.0);
+            bool sl;
+            const double r = rho_tri(Q[0], Q[1], Q[2], &sl);
+            A.keys[1 + t] = (unsigned long long)__double_as_longlong(r);
+            A.vals[1 + t] = (int)t;
+            if (sl) A.slivers[atomicAdd(&A.ct->al_sliver, 1)] = (int)t;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                if (!((f >> i) & 1u)) continue;
+                const double2 pa = Q[p1(i)], pb = Q[m1(i)], pk = Q[i], po = O[i];
+                double qa[2] = {pa.x, pa.y}, qb[2] = {pb.x, pb.y}, qk[2] = {pk.x, pk.y};
+                int att = attached_filter(qa, qb, qk);
                 if (att == 2) {
-                    atomicAdd(&ct->exact_attached, 1ull);
-                    att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, po.x, po.y);
+                    atomicAdd(&A.ct->exact_attached, 1ull);
+                    att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, pk.x, pk.y);
+                }
+                if (att == 0 && opp[i] >= 0) {
+                    double qo[2] = {po.x, po.y};
+                    att = attached_filter(qa, qb, qo);
+                    if (att == 2) {
+                        atomicAdd(&A.ct->exact_attached, 1ull);
+                        att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, po.x, po.y);
+                    }
+                }
+                if (att == EXACT_OVERFLOW) set_err(A.ct, GPUDT_ERR_EXACT, 100);
+                if (!att) {
+                    f |= 8u << i;
+                    s_rho[i * kAkTile + j] = rho_edge(pa, pb);
                 }
             }
-            if (att == EXACT_OVERFLOW) set_err(ct, GPUDT_ERR_EXACT, 100);
-            unatt[e] = att ? 0 : 1;
-            if (att) edge_ro[e] = 0;
+        }
+        const int own = __popc(f & 7u) | (__popc(f & 56u) << 16);
+        int x = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_part[u * (kAkThreads / 32) + w] = x;
+#pragma unroll
+        for (int q = 0; q < kAkItems; q++)
+            if (q == u) {
+                flags[q] = f;
+                cnt[q] = own;
+                incl[q] = x;
+            }
+    }
+    __syncthreads();
+    if (w == 0) {
+        constexpr int kParts = kAkItems * (kAkThreads / 32);
+        static_assert(kParts <= 32, "one warp scans the partial sums of a tile");
+        const int v = lane < kParts ? s_part[lane] : 0;
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane < kParts) s_part[lane] = x - v;
+        const int tot = __shfl_sync(0xffffffffu, x, 31);
+        const unsigned long long mine = ((unsigned long long)(tot & 0xffff) << 31) | (unsigned)(tot >> 16);
+        unsigned long long acc = 0;
+        if (tile > 0) {
+            volatile unsigned long long *st = A.status;
+            if (lane == 0) st[tile] = kAkAgg | mine;
+            bool bad = false;
+            for (int j = tile - 1;; j -= 32) {
+                const int idx = j - lane;
+                unsigned long long wd = kAkInc;  // before tile 0: nothing to add
+                for (int spins = 0; idx >= 0 && ((wd = st[idx]) >> 62) == 0; spins++) {
+                    if (spins > kAkSpinLimit) {
+                        bad = true;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+                bad = __any_sync(0xffffffffu, bad);
+                if (bad) break;
+                const unsigned inc = __ballot_sync(0xffffffffu, (wd >> 62) == 2);
+                const int first = inc ? __ffs(inc) - 1 : 31;  // lanes up to the nearest inclusive count
+                unsigned long long add = lane <= first && idx >= 0 ? wd & kAkVal : 0ull;
+                for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+                acc += add;
+                if (inc) break;
+            }
+            if (bad && lane == 0) set_err(A.ct, GPUDT_ERR_NOCONVERGE, 96);
+        }
+        if (lane == 0) {
+            ((volatile unsigned long long *)A.status)[tile] = kAkInc | (acc + mine);
+            s_excl = acc;
+            if (tile == A.tiles - 1) {
+                A.ct->al_edges = (int)((acc + mine) >> 31);
+                A.ct->al_unatt = (int)((acc + mine) & 0x7fffffffu);
+            }
+        }
+    }
+    __syncthreads();
+    const int e0 = (int)(s_excl >> 31), k0 = 1 + A.nT + (int)(s_excl & 0x7fffffffu);
+#pragma unroll
+    for (int u = 0; u < kAkItems; u++) {
+        const int j = u * kAkThreads + threadIdx.x;
+        const long long t = (long long)tile * kAkTile + j;
+        if (t >= A.nT) continue;
+        const int at = s_part[u * (kAkThreads / 32) + w] + incl[u] - cnt[u];
+        int e = e0 + (at & 0xffff), k = k0 + (at >> 16);
+        A.e_off[t] = e;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            if (!((flags[u] >> i) & 1u)) continue;
+            A.edges[e] = enc((int)t, i);
+            if ((flags[u] >> i) & 8u) {
+                A.keys[k] = (unsigned long long)__double_as_longlong(s_rho[i * kAkTile + j]);
+                A.vals[k++] = A.nT + e;
+            } else {
+                A.edge_ro[e] = 0;
+            }
             e++;
         }
     }
-};
+}
 
 struct SliverKeys {
     const int4 *cv;  // the triangles with the ids that index P
@@ -204,26 +330,6 @@ struct SliverKeys {
         double r = rho_rounded_exact(3, p);
         if (r != r) set_err(ct, GPUDT_ERR_EXACT, 101);
         keys[1 + t] = (unsigned long long)__double_as_longlong(r);
-    }
-};
-
-struct EdgeKeys {
-    const int4 *edges;
-    const int4 *gv;  // the triangles with the ids that index P
-    const double2 *P;
-    const int *unatt, *spos;
-    unsigned long long *keys;
-    int *vals;
-    int base, nT;
-    __device__ void operator()(long long ii) const
-    {
-        int e = (int)ii;
-        if (!unatt[e]) return;
-        int4 E = edges[e];
-        int k = base + spos[e];
-        const int4 g = gv[E.z];
-        keys[k] = (unsigned long long)__double_as_longlong(rho_edge(P[geti(g, p1(E.w))], P[geti(g, m1(E.w))]));
-        vals[k] = nT + e;
     }
 };
 
@@ -254,7 +360,7 @@ struct MarkRuns {
         }
         if (i >= 2 && (!seg || seg[i] == seg[i - 1]) && near_equal(keys[i - 1], keys[i])) {
             nr[i] = 0;
-            int k = atomicAdd(&ct->nlist, 1);
+            int k = atomicAdd(&ct->al_unc, 1);
             unc[k] = i;
         } else {
             nr[i] = 1;
@@ -262,7 +368,7 @@ struct MarkRuns {
     }
 };
 
-__device__ __forceinline__ void entry_points(int val, int nT, const int4 *cv, const int4 *edges,
+__device__ __forceinline__ void entry_points(int val, int nT, const int4 *cv, const int *edges,
                                              const double2 *P, int *kind, double *p)
 {
     if (val < nT) {
@@ -271,15 +377,15 @@ __device__ __forceinline__ void entry_points(int val, int nT, const int4 *cv, co
         p[0] = a.x; p[1] = a.y; p[2] = b.x; p[3] = b.y; p[4] = c.x; p[5] = c.y;
         *kind = 3;
     } else {
-        int4 E = edges[val - nT];
-        const int4 g = cv[E.z];  // cv: the triangles with the ids that index P
-        double2 a = P[geti(g, p1(E.w))], b = P[geti(g, m1(E.w))];
+        const int E = edges[val - nT];
+        const int4 g = cv[dtri(E)];  // cv: the triangles with the ids that index P
+        double2 a = P[geti(g, p1(dori(E)))], b = P[geti(g, m1(dori(E)))];
         p[0] = a.x; p[1] = a.y; p[2] = b.x; p[3] = b.y;
         *kind = 2;
     }
 }
 
-__device__ __forceinline__ int exact_cmp_vals(int va, int vb, int nT, const int4 *cv, const int4 *edges,
+__device__ __forceinline__ int exact_cmp_vals(int va, int vb, int nT, const int4 *cv, const int *edges,
                                               const double2 *P)
 {
     int ka, kb;
@@ -292,19 +398,22 @@ __device__ __forceinline__ int exact_cmp_vals(int va, int vb, int nT, const int4
 // One exact comparison per uncertain adjacent pair (parallel over pairs): a
 // smaller left value starts a new rank, an exact tie shares the rank, and an
 // order violation sends the whole run to k_resolve (rare: it needs two distinct
-// values within one ulp whose keys rounded the wrong way).
+// values within one ulp whose keys rounded the wrong way).  Without slowflag
+// the runs are only counted: the caller starts over when there is one.
 struct ExactAdjacent {
     const unsigned long long *keys;
     const int *vals;
     int *nr, *slow, *slowflag;
     const int *unc;
-    const int4 *cv, *edges;
+    const int4 *cv;
+    const int *edges;
     const double2 *P;
     int nT;
     Counters *ct;
     const int *seg;
     __device__ void operator()(long long ii) const
     {
+        if (ct->err) return;  // a sort that gave up leaves entries that name no simplex
         int i = unc[ii];
         int cmp = exact_cmp_vals(vals[i - 1], vals[i], nT, cv, edges, P);
         atomicAdd(&ct->exact_compares, 1ull);
@@ -319,9 +428,13 @@ struct ExactAdjacent {
             atomicAdd(&ct->nties, 1);
         } else {
             int s = i - 1;
+            if (!slowflag) {
+                atomicAdd(&ct->al_slow, 1);
+                return;
+            }
             while (s >= 2 && (!seg || seg[s - 1] == seg[s]) && near_equal(keys[s - 1], keys[s])) s--;
             if (atomicCAS(&slowflag[s], 0, 1) == 0) {
-                int k = atomicAdd(&ct->nlist2, 1);
+                int k = atomicAdd(&ct->al_slow, 1);
                 slow[k] = s;
             }
         }
@@ -339,7 +452,8 @@ struct ResolveRuns {
     unsigned long long *keys;
     int *vals, *nr;
     const int *runs;
-    const int4 *cv, *edges;
+    const int4 *cv;
+    const int *edges;
     const double2 *P;
     int n, nT;
     Counters *ct;
@@ -387,7 +501,7 @@ struct ResolveRuns {
 // Order of two spectrum entries: by key where the keys are more than 2 ulp
 // apart (each carries at most 1 ulp of error), else exactly.
 __device__ __forceinline__ int cmp_entries(unsigned long long ka, int va, unsigned long long kb, int vb, int nT,
-                                           const int4 *cv, const int4 *edges, const double2 *P)
+                                           const int4 *cv, const int *edges, const double2 *P)
 {
     if (ka < kb && !near_equal(ka, kb)) return -1;
     if (kb < ka && !near_equal(kb, ka)) return 1;
@@ -402,7 +516,7 @@ __device__ __forceinline__ int cmp_entries(unsigned long long ka, int va, unsign
 constexpr int kLongThreads = 256;
 __global__ void __launch_bounds__(kLongThreads) k_resolve_long(unsigned long long *keys, int *vals, int *nr,
                                                                unsigned long long *tk, int *tv, const int *runs,
-                                                               const int4 *cv, const int4 *edges, const double2 *P,
+                                                               const int4 *cv, const int *edges, const double2 *P,
                                                                int n, int nT, Counters *ct, const int *seg,
                                                                int block_run, int2 *huge)
 {
@@ -506,7 +620,7 @@ constexpr int kMergeChunk = 16;
 __global__ void __launch_bounds__(256) k_merge_level(const unsigned long long *__restrict__ sk,
                                                      const int *__restrict__ sv, unsigned long long *__restrict__ dk,
                                                      int *__restrict__ dv, int L, int w, const int4 *cv,
-                                                     const int4 *edges, const double2 *P, int nT, Counters *ct)
+                                                     const int *edges, const double2 *P, int nT, Counters *ct)
 {
     const long long o0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kMergeChunk;
     if (o0 >= L) return;
@@ -556,7 +670,8 @@ __global__ void __launch_bounds__(256) k_merge_level(const unsigned long long *_
 struct RunFlags {
     const int *vals;
     int *nr;
-    const int4 *cv, *edges;
+    const int4 *cv;
+    const int *edges;
     const double2 *P;
     int s, nT;
     Counters *ct;
@@ -603,8 +718,10 @@ struct ScatterRanks {
     int *tri_ro, *edge_ro;
     double *spectrum;
     int nT;
+    const Counters *ct;
     __device__ void operator()(long long ii) const
     {
+        if (ct->err) return;  // as in ExactAdjacent
         int i = (int)ii;
         int r = excl[i] + nr[i];
         if (i == 0) {
@@ -618,44 +735,55 @@ struct ScatterRanks {
     }
 };
 
+// Intervals of the edges a triangle owns and, from them, of its vertices: the
+// triangle's contributions to a vertex are combined before the atomics (1.5
+// owned edges on average reach 2.5 vertices, not 3), and the triangles are
+// read in order, where one thread per edge gathered a 16-byte record and a
+// link each.  The atomics bound it either way (348 us at 8.4 M triangles).
+// The intervals start as all ones: -1 for the signed maximum, the largest
+// value for the unsigned minimum, and (-1, -1) for a vertex without edges, so
+// no launch sets them up or converts them.
 struct EdgeIntervals {
-    const int4 *edges, *cn;
-    const int *tri_ro, *edge_ro;
+    const int4 *cv, *cn;
+    const int *e_off, *tri_ro, *edge_ro;
     int2 *edge_nu;
-    int2 *pt;  // (min, max) accumulators
-    __device__ void operator()(long long ii) const
+    int2 *pt;
+    __device__ void operator()(long long t) const
     {
-        int e = (int)ii;
-        int4 E = edges[e];
-        int nb = geti(cn[E.z], E.w);
-        int tr = tri_ro[E.z];
-        int2 nu;
-        if (nb == -1) {
-            nu = make_int2(tr, 0);
-        } else {
-            int o = tri_ro[dtri(nb)];
-            nu = tr <= o ? make_int2(tr, o) : make_int2(o, tr);
+        const int4 v = cv[t], n = cn[t];
+        const int tr = tri_ro[t];
+        int e = e_off[t];
+        int o[3], lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
+        bool own[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int nb = geti(n, i);
+            own[i] = geti(v, p1(i)) < geti(v, m1(i)) || nb == -1;
+            o[i] = own[i] && nb != -1 ? tri_ro[dtri(nb)] : 0;
         }
-        edge_nu[e] = nu;
-        int ro = edge_ro[e];
-        int vmin = ro != 0 ? ro : nu.x;
-        atomicMin(&pt[E.x].x, vmin);
-        atomicMax(&pt[E.x].y, nu.y);
-        atomicMin(&pt[E.y].x, vmin);
-        atomicMax(&pt[E.y].y, nu.y);
-    }
-};
-
-struct InitPt {
-    int2 *pt;
-    __device__ void operator()(long long i) const { pt[i] = make_int2(0x7fffffff, -1); }
-};
-
-struct FixPt {
-    int2 *pt;
-    __device__ void operator()(long long i) const
-    {
-        if (pt[i].x == 0x7fffffff) pt[i] = make_int2(-1, -1);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            if (!own[i]) continue;
+            int2 nu;
+            if (geti(n, i) == -1) nu = make_int2(tr, 0);
+            else nu = tr <= o[i] ? make_int2(tr, o[i]) : make_int2(o[i], tr);
+            edge_nu[e] = nu;
+            const int ro = edge_ro[e];
+            const int vmin = ro != 0 ? ro : nu.x;
+            e++;
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                if (q == i) continue;
+                lo[q] = min(lo[q], vmin);
+                hi[q] = max(hi[q], nu.y);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            if (hi[q] < 0) continue;
+            atomicMin((unsigned *)&pt[geti(v, q)].x, (unsigned)lo[q]);
+            atomicMax(&pt[geti(v, q)].y, hi[q]);
+        }
     }
 };
 
@@ -789,36 +917,131 @@ struct SetSentinels {
 };
 
 // ------------------------------------------------------------------ stage
+// Up to this many entries the host looks at nothing between the sort and the
+// intervals: what it would have looked for (a long group of equal key tops, a
+// run out of exact order) then costs a second pass over the ranks, about 40 us
+// at this size, where the two reads cost 30 us on every call.
+constexpr int kDeferEntries = 1 << 19;
+
+// Ranks of the sorted entries (keys, vals): near-equal neighbours compared
+// exactly, runs out of exact order re-sorted.  With `defer` such runs are only
+// counted (al_slow) and the host reads nothing.
+static int alpha_ranks(Ctx &c, AlphaSegs *segs, int nIn, bool defer)
+{
+    int r;
+    const int nT = c.nT_out;
+    const int *seg = segs ? segs->seg : nullptr;
+    int *nr = c.aux, *unc = c.list, *slow = c.list2, *slowflag = c.stamp;
+    launch_n(c, MarkRuns{c.keys, nr, unc, nIn, c.ctr, seg}, nIn);
+    const ExactAdjacent adj{c.keys, c.vals, nr, slow, defer ? nullptr : slowflag, unc, alpha_geom_tris(c), c.edges,
+                            c.opos, nT, c.ctr, seg};
+    if (defer) {
+        launch_dev(c, adj, &c.ctr->al_unc, nIn);
+        return GPUDT_OK;
+    }
+    r = read_counters(c);
+    if (r) return r;
+    if (c.hctr->al_unc == 0) return GPUDT_OK;
+    GALPHA_CUDA(cudaMemsetAsync(slowflag, 0, sizeof(int) * (size_t)nIn, c.stream));
+    launch_n(c, adj, c.hctr->al_unc);
+    r = read_counters(c);
+    if (r) return r;
+    if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+    if (c.hctr->al_slow == 0) return GPUDT_OK;
+    // runs longer than kThreadRun are listed after the slow runs
+    const int nslow = c.hctr->al_slow;
+    int *longs = slow + nslow;
+    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlong, 0, sizeof(int), c.stream));
+    launch_n(c, ResolveRuns{c.keys, c.vals, nr, slow, alpha_geom_tris(c), c.edges, c.opos, nIn, nT, c.ctr, seg, longs},
+             nslow);
+    r = read_counters(c);
+    if (r) return r;
+    if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+    if (c.hctr->nlong == 0) return GPUDT_OK;
+    // (keys2, vals2) are free now: the second buffer of each run's merge sort
+    const int nlong = c.hctr->nlong;
+    // runs for the multi-block merge: (start, length) pairs after the long runs, 8-byte aligned
+    uintptr_t hp = reinterpret_cast<uintptr_t>(longs + nlong);
+    int2 *huge = reinterpret_cast<int2 *>((hp + 7) & ~(uintptr_t)7);
+    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nhuge, 0, sizeof(int), c.stream));
+    k_resolve_long<<<(unsigned)nlong, kLongThreads, 0, c.stream>>>(c.keys, c.vals, nr, c.keys2, c.vals2, longs,
+                                                                   alpha_geom_tris(c), c.edges, c.opos, nIn, nT, c.ctr,
+                                                                   seg, c.block_run, huge);
+    count_launch();
+    GALPHA_CUDA(cudaGetLastError());
+    r = read_counters(c);
+    if (r) return r;
+    if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+    const int nhuge = c.hctr->nhuge;
+    if (nhuge > 0) {
+        std::vector<int2> hs(nhuge);
+        r = read_small(c, hs.data(), huge, sizeof(int2) * (size_t)nhuge);
+        if (r) return r;
+        for (const int2 &h : hs) {
+            r = merge_sort_run(c, c.keys, c.vals, c.keys2, c.vals2, nr, h.x, h.y, nT);
+            if (r) return r;
+        }
+        r = read_counters(c);
+        if (r) return r;
+        if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+    }
+    return GPUDT_OK;
+}
+
+// Spectrum, simplex ranks and intervals from the rank-start flags (c.aux).
+static int alpha_scatter(Ctx &c, AlphaSegs *segs, int nIn)
+{
+    const int nT = c.nT_out;
+    const int *nr = c.aux;
+    int r = exclusive_scan_int(c, nr, c.rank, nIn, &c.ctr->al_ranks);
+    if (r) return r;
+    if (!segs) {
+        launch_n(c, ScatterRanks{c.keys, c.vals, nr, c.rank, c.tri_ro, c.edge_ro, c.spectrum, nT, c.ctr}, nIn);
+    } else {
+        GALPHA_CUDA(cudaMemsetAsync(segs->nd, 0, sizeof(int) * (size_t)segs->K, c.stream));
+        GALPHA_CUDA(cudaMemsetAsync(segs->firstexcl, 0, sizeof(int) * (size_t)segs->K, c.stream));
+        launch_n(c, SetRankBounds{segs->seg, nr, c.rank, nIn, segs->firstexcl, segs->nd}, nIn);
+        launch_n(c, SetDistinct{segs->firstexcl, segs->nd}, segs->K);
+        r = exclusive_scan_int(c, segs->nd, segs->spec_off, segs->K, nullptr);
+        if (r) return r;
+        launch_n(c, ScatterRanksSeg{c.keys, c.vals, nr, c.rank, segs->seg, segs->firstexcl, segs->spec_off,
+                                    c.tri_ro, c.edge_ro, c.spectrum, nT},
+                 nIn);
+        launch_n(c, SetSentinels{segs->spec_off, c.spectrum}, segs->K);
+    }
+    GALPHA_CUDA(cudaMemsetAsync(c.pt_nu, 0xff, sizeof(int2) * (size_t)c.N, c.stream));
+    launch_n(c, EdgeIntervals{c.cv, c.cn, c.e_off, c.tri_ro, c.edge_ro, c.edge_nu, c.pt_nu}, nT);
+    GALPHA_CUDA(cudaGetLastError());
+    return read_counters(c);
+}
+
 int stage_alpha(Ctx &c, AlphaSegs *segs)
 {
     int r;
     const int nT = c.nT_out;
-    int *cnt = c.aux, *e_off = c.e_off;
     // an alpha call on a resident mesh starts without the error of an earlier
-    // failed alpha call (err and errinfo are adjacent words)
+    // failed alpha call (err and errinfo are adjacent words) and with its own
+    // counts
     GALPHA_CUDA(cudaMemsetAsync(&c.ctr->err, 0, 2 * sizeof(int), c.stream));
-    launch_n(c, EdgeCount{c.cv, c.cn, cnt}, nT);
-    r = exclusive_scan_int(c, cnt, e_off, nT, &c.ctr->nlist);
-    if (r) return r;
-    r = read_counters(c);
-    if (r) return r;
-    const int nE = c.hctr->nlist;
-    c.nE = nE;
-    int *unatt = c.aux2, *spos = c.rank;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist2, 0, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.keys, 0, sizeof(unsigned long long), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.vals, 0, sizeof(int), c.stream));
-    launch_occ<4>(c, TriKeys{c.cv, c.cn, alpha_geom_tris(c), c.opos, e_off, c.keys, c.vals, c.edges, unatt, c.edge_ro, c.list, c.ctr}, nT);
-    // the sliver list's length stays on the device; TriKeys' errors are read
-    // with the spectrum length below
-    launch_dev(c, SliverKeys{alpha_geom_tris(c), c.opos, c.list, c.keys, c.ctr}, &c.ctr->nlist2, nT);
-    r = exclusive_scan_int(c, unatt, spos, nE, &c.ctr->nlist);
-    if (r) return r;
-    launch_n(c, EdgeKeys{c.edges, alpha_geom_tris(c), c.opos, unatt, spos, c.keys, c.vals, 1 + nT, nT}, nE);
+    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->al_edges, 0, kAlphaBytes, c.stream));
+    const int tiles = (nT + kAkTile - 1) / kAkTile;
+    if (nT > 0) {
+        // status words in the sort's scratch, which no sort uses yet
+        unsigned long long *status = (unsigned long long *)c.rhist;
+        GALPHA_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (size_t)(tiles + 1), c.stream));
+        k_alpha_keys<<<(unsigned)tiles, kAkThreads, 0, c.stream>>>(
+            AlphaKeysArgs{c.cv, c.cn, alpha_geom_tris(c), c.opos, nT, c.e_off, c.keys, c.vals, c.edges, c.edge_ro,
+                          c.list, status, tiles, c.ctr});
+        count_launch();
+    }
+    // the sliver list's length stays on the device
+    launch_dev(c, SliverKeys{alpha_geom_tris(c), c.opos, c.list, c.keys, c.ctr}, &c.ctr->al_sliver, nT);
     r = read_counters(c);
     if (r) return r;
     if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-    const int nIn = 1 + nT + c.hctr->nlist;
+    const int nE = c.hctr->al_edges;
+    c.nE = nE;
+    const int nIn = 1 + nT + c.hctr->al_unatt;
     c.nSpecIn = nIn;
     c.sort_passes = 0;
     if (c.events) {
@@ -826,16 +1049,22 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
         c.kev_rec[8] = true;
     }
     bool second = false;
-    r = radix_sort(c, c.keys + 1, c.vals + 1, c.keys2 + 1, c.vals2 + 1, nIn - 1, &second);
+    // entry 0 is the sentinel (no key of its own); a batch's entries are
+    // regrouped after the sort, so a late look at its long groups is no option
+    const bool defer = !segs && nIn <= kDeferEntries;
+    unsigned long long *k1 = c.keys, *k2 = c.keys2;
+    int *v1 = c.vals, *v2 = c.vals2;
+    r = radix_sort(c, k1 + 1, v1 + 1, k2 + 1, v2 + 1, nIn - 1, &second, defer);
     if (r) return r;
-    if (second) {
-        // the sorted entries are in the second buffers: they become keys / vals
-        // (sentinel entry 0 included) for the rest of this result's life
-        GALPHA_CUDA(cudaMemsetAsync(c.keys2, 0, sizeof(unsigned long long), c.stream));
-        GALPHA_CUDA(cudaMemsetAsync(c.vals2, 0, sizeof(int), c.stream));
-        std::swap(c.keys, c.keys2);
-        std::swap(c.vals, c.vals2);
-    }
+    // the sorted entries may be in the second buffers: they become keys / vals
+    // for the rest of this result's life
+    auto take_sorted = [&]() {
+        c.keys = second ? k2 : k1;
+        c.keys2 = second ? k1 : k2;
+        c.vals = second ? v2 : v1;
+        c.vals2 = second ? v1 : v2;
+    };
+    take_sorted();
     if (c.events) {
         cudaEventRecord(c.kev[9], c.stream);
         c.kev_rec[9] = true;
@@ -859,87 +1088,25 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
         if (r) return r;
         launch_n(c, SetOfSorted{ka, segs->seg}, m);
     }
-    // ranks
-    int *nr = c.aux, *unc = c.list, *slow = c.list2, *slowflag = c.stamp;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist, 0, 2 * sizeof(int), c.stream));
-    launch_n(c, MarkRuns{c.keys, nr, unc, nIn, c.ctr, segs ? segs->seg : nullptr}, nIn);
-    r = read_counters(c);
-    if (r) return r;
-    int nunc = c.hctr->nlist;
-    if (nunc > 0) {
-        GALPHA_CUDA(cudaMemsetAsync(slowflag, 0, sizeof(int) * (size_t)nIn, c.stream));
-        launch_n(c, ExactAdjacent{c.keys, c.vals, nr, slow, slowflag, unc, alpha_geom_tris(c), c.edges, c.opos, nT, c.ctr,
-                                  segs ? segs->seg : nullptr},
-                 nunc);
-        r = read_counters(c);
-        if (r) return r;
-        if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-        if (c.hctr->nlist2 > 0) {
-            // runs longer than kThreadRun are listed after the slow runs
-            const int nslow = c.hctr->nlist2;
-            int *longs = slow + nslow;
-            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlong, 0, sizeof(int), c.stream));
-            launch_n(c, ResolveRuns{c.keys, c.vals, nr, slow, alpha_geom_tris(c), c.edges, c.opos, nIn, nT, c.ctr,
-                                    segs ? segs->seg : nullptr, longs},
-                     nslow);
-            r = read_counters(c);
-            if (r) return r;
-            if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-            if (c.hctr->nlong > 0) {
-                // (keys2, vals2) are free now: the second buffer of each run's merge sort
-                const int nlong = c.hctr->nlong;
-                // runs for the multi-block merge: (start, length) pairs after the long runs, 8-byte aligned
-                uintptr_t hp = reinterpret_cast<uintptr_t>(longs + nlong);
-                int2 *huge = reinterpret_cast<int2 *>((hp + 7) & ~(uintptr_t)7);
-                GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nhuge, 0, sizeof(int), c.stream));
-                k_resolve_long<<<(unsigned)nlong, kLongThreads, 0, c.stream>>>(
-                    c.keys, c.vals, nr, c.keys2, c.vals2, longs, alpha_geom_tris(c), c.edges, c.opos, nIn, nT, c.ctr,
-                    segs ? segs->seg : nullptr, c.block_run, huge);
-                count_launch();
-                GALPHA_CUDA(cudaGetLastError());
-                r = read_counters(c);
-                if (r) return r;
-                if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-                const int nhuge = c.hctr->nhuge;
-                if (nhuge > 0) {
-                    std::vector<int2> hs(nhuge);
-                    r = read_small(c, hs.data(), huge, sizeof(int2) * (size_t)nhuge);
-                    if (r) return r;
-                    for (const int2 &h : hs) {
-                        r = merge_sort_run(c, c.keys, c.vals, c.keys2, c.vals2, nr, h.x, h.y, nT);
-                        if (r) return r;
-                    }
-                    r = read_counters(c);
-                    if (r) return r;
-                    if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-                }
-            }
-        }
-    }
-    r = exclusive_scan_int(c, nr, c.rank, nIn, &c.ctr->nlist);
-    if (r) return r;
-    if (!segs) {
-        launch_n(c, ScatterRanks{c.keys, c.vals, nr, c.rank, c.tri_ro, c.edge_ro, c.spectrum, nT}, nIn);
-    } else {
-        GALPHA_CUDA(cudaMemsetAsync(segs->nd, 0, sizeof(int) * (size_t)segs->K, c.stream));
-        GALPHA_CUDA(cudaMemsetAsync(segs->firstexcl, 0, sizeof(int) * (size_t)segs->K, c.stream));
-        launch_n(c, SetRankBounds{segs->seg, nr, c.rank, nIn, segs->firstexcl, segs->nd}, nIn);
-        launch_n(c, SetDistinct{segs->firstexcl, segs->nd}, segs->K);
-        r = exclusive_scan_int(c, segs->nd, segs->spec_off, segs->K, nullptr);
-        if (r) return r;
-        launch_n(c, ScatterRanksSeg{c.keys, c.vals, nr, c.rank, segs->seg, segs->firstexcl, segs->spec_off,
-                                    c.tri_ro, c.edge_ro, c.spectrum, nT},
-                 nIn);
-        launch_n(c, SetSentinels{segs->spec_off, c.spectrum}, segs->K);
-    }
-    launch_n(c, InitPt{c.pt_nu}, c.N);
-    launch_n(c, EdgeIntervals{c.edges, c.cn, c.tri_ro, c.edge_ro, c.edge_nu, c.pt_nu}, nE);
-    launch_n(c, FixPt{c.pt_nu}, c.N);
-    GALPHA_CUDA(cudaGetLastError());
-    r = read_counters(c);
+    r = alpha_ranks(c, segs, nIn, defer);
+    if (!r) r = alpha_scatter(c, segs, nIn);
     if (r) return r;
     if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
-    c.nSpec = c.hctr->nlist + (segs ? segs->K : 1);  // distinct ranks incl. the sentinel(s)
+    if (defer && (c.hctr->fx_long || c.hctr->fx_many || c.hctr->al_slow)) {
+        // a long group or a run out of order after all: that, and the ranks again
+        if (c.hctr->fx_long || c.hctr->fx_many) {
+            r = radix_sort_finish(c, k1 + 1, v1 + 1, k2 + 1, v2 + 1, nIn - 1, &second, false);
+            if (r) return r;
+            take_sorted();
+            c.st.sortPasses = c.sort_passes;
+        }
+        GALPHA_CUDA(cudaMemsetAsync(&c.ctr->fx_groups, 0, kRankBytes, c.stream));
+        r = alpha_ranks(c, segs, nIn, false);
+        if (!r) r = alpha_scatter(c, segs, nIn);
+        if (r) return r;
+        if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+    }
+    c.nSpec = c.hctr->al_ranks + (segs ? segs->K : 1);  // distinct ranks incl. the sentinel(s)
     return GPUDT_OK;
 }
 

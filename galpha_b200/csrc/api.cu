@@ -152,7 +152,7 @@ static size_t plan(const Sizes &z, Ctx *c, Arena *A)
     TAKE(rhist, int, radix_sort_scratch_ints((long long)(3 * cap)) + 16);
     if (c) c->rhist_ints = radix_sort_scratch_ints((long long)(3 * cap)) + 16;
     TAKE(e_off, int, cap + 1);
-    TAKE(edges, int4, 2 * cap);
+    TAKE(edges, int, 2 * cap);
     TAKE(edge_ro, int, 2 * cap);
     TAKE(edge_nu, int2, 2 * cap);
     TAKE(tri_ro, int, cap);
@@ -506,6 +506,8 @@ static int handle_init(galpha_ctx *h, int device, long long budget)
         c.hmail = (char *)hp + ctr_bytes;
         c.hmail_dev = (char *)dp + ctr_bytes;
     }
+    GALPHA_CUDA(cudaMalloc(&c.scan_buf, kScanBufBytes));
+    GALPHA_CUDA(cudaMemsetAsync(c.scan_buf, 0, kScanBufBytes, c.stream));
     for (int k = 0; k < GALPHA_STAGE_TOTAL + 2; k++) GALPHA_CUDA(cudaEventCreate(&c.ev[k]));
     for (int k = 0; k < 10; k++) GALPHA_CUDA(cudaEventCreate(&c.kev[k]));
     c.events = true;
@@ -546,6 +548,7 @@ int galphaDestroy(galphaHandle h)
     if (h->H.arena.base) cudaFree(h->H.arena.base);
     if (h->H.d_xy) cudaFree(h->H.d_xy);
     if (c.ml_buf) cudaFree(c.ml_buf);
+    if (c.scan_buf) cudaFree(c.scan_buf);
     if (c.cons_buf) cudaFree(c.cons_buf);
     if (c.cons_pool) cudaFree(c.cons_pool);
     if (h->H.bd.buf) cudaFree(h->H.bd.buf);
@@ -806,20 +809,20 @@ int galphaCopyTriangles(galphaHandle h, gpudtTriangle *dst, int cap)
 
 // Edge records in the reference's edge_interval layout, built on the device.
 struct EdgeAos {
-    const int4 *edges;
+    const int *edges;
     const int *ero;
     const int2 *enu;
     galphaEdgeInterval *out;
     __device__ void operator()(long long e) const
     {
         galphaEdgeInterval E;
-        int4 q = edges[e];
+        const int q = edges[e];
         E.ro_rank = ero[e];
         E.nu_min_rank = enu[e].x;
         E.nu_max_rank = enu[e].y;
         E.sc = E.ro_rank == 0 ? 0 : 1;
-        E.tIndex = q.z;
-        E.vOpp = q.w;
+        E.tIndex = dtri(q);
+        E.vOpp = dori(q);
         out[e] = E;
     }
 };

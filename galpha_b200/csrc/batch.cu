@@ -355,21 +355,21 @@ struct LocalTriangles {
 };
 
 struct LocalEdges {
-    const int4 *edges;
+    const int *edges;
     const int *ero;
     const int2 *enu;
     const int *tset, *tbase;
     galphaEdgeInterval *out;
     __device__ void operator()(long long e) const
     {
-        int4 q = edges[e];
+        const int q = edges[e], t = dtri(q);
         galphaEdgeInterval E;
         E.ro_rank = ero[e];
         E.nu_min_rank = enu[e].x;
         E.nu_max_rank = enu[e].y;
         E.sc = E.ro_rank == 0 ? 0 : 1;
-        E.tIndex = q.z - tbase[tset[q.z]];
-        E.vOpp = q.w;
+        E.tIndex = t - tbase[tset[t]];
+        E.vOpp = dori(q);
         out[e] = E;
     }
 };

@@ -55,9 +55,20 @@ struct Counters {
     int err;        // first error code (GPUDT_ERR_*), 0 if none
     int errinfo;    // stage-specific detail of the first error
     int nisland;    // island pixels
-    int nties;      // exact spectrum ties merged
     int flips_total;
     int escalate;   // island repair could not stay local: redo the Voronoi stage globally
+    // alpha stage, cleared together when it starts (kAlphaWords from al_edges on)
+    int al_edges;    // edges numbered
+    int al_unatt;    // of them, unattached: in the spectrum
+    int al_sliver;   // triangles whose radius needs exact arithmetic
+    int al_ranks;    // distinct values
+    // the rest again when the ranks are redone (kRankWords from fx_groups on)
+    int fx_groups;   // key sort: short groups out of order
+    int fx_long;     // key sort: out-of-order pairs recorded in groups too long for one thread
+    int fx_many;     // key sort: more of those than can be recorded
+    int al_unc;      // adjacent keys within 2 ulp
+    int al_slow;     // runs out of exact order
+    int nties;       // exact spectrum ties merged
     unsigned long long exact_compares;
     unsigned long long exact_orient;
     unsigned long long exact_incircle;
@@ -67,7 +78,7 @@ struct Counters {
     int qpad;
     double qalpha;   // alpha query: the alpha value classified
     int tail_rounds; // flip: rounds run by the last in-block tail launch
-    int nlong;       // key sort: out-of-order pairs recorded in groups too long for one thread
+    int nlong;       // alpha ranks: runs too long for one thread; master list: long runs
     int nhuge;       // alpha ranks: runs too long for one block, listed for the multi-block merge
     int sh_total;    // shift: all dropped sites listed so far
     int nbad;        // shift: sites that cannot be shifted
@@ -104,6 +115,9 @@ struct Relink {
     int loc;
     int old;
 };
+
+constexpr size_t kAlphaBytes = offsetof(Counters, exact_orient) - offsetof(Counters, al_edges);
+constexpr size_t kRankBytes = offsetof(Counters, exact_orient) - offsetof(Counters, fx_groups);
 
 // A grown-on-demand device buffer.
 struct DevBuf {
@@ -165,7 +179,7 @@ struct Ctx {
     // alpha arrays
     int nT_out = 0, nE = 0, nSpecIn = 0, nSpec = 0;
     int *e_off = nullptr;      // [nT+1] first edge of each triangle
-    int4 *edges = nullptr;     // [nE] p1, p2, tIndex | vOpp<<30? (see alpha.cu)
+    int *edges = nullptr;      // [nE] owner triangle and the corner opposite: enc(tIndex, vOpp)
     int *edge_ro = nullptr;    // [nE]
     int2 *edge_nu = nullptr;   // [nE]
     int *tri_ro = nullptr;     // [nT]
@@ -182,7 +196,11 @@ struct Ctx {
     int *ml_sp = nullptr;           // [nSpecPtr]
     int nMaster = 0, nSpecPtr = 0;
     bool have_master = false;
-    int *hist = nullptr;       // scan scratch
+    int *hist = nullptr;       // scratch of scans over more than kScanMaxTiles tiles
+    // single-launch scans: status words, then the tile ticket (own allocation,
+    // made with the handle); scans started so far
+    unsigned long long *scan_buf = nullptr;
+    unsigned scan_no = 0;
     int *rhist = nullptr;      // radix sort histograms
     long long rhist_ints = 0;  // its size
     gpudtTriangle *outtri = nullptr;  // [cap] AoS output staging
@@ -262,6 +280,8 @@ int read_small(Ctx &c, void *host_dst, const void *dev_src, size_t bytes);
 // Records the failing stage and the device-side detail code (galphaLastError).
 int stage_fail(Ctx &c, int r, const char *stage);
 constexpr size_t kMailBytes = 65536;
+constexpr long long kScanMaxTiles = 32768;  // of 4,096 elements, scanned by one launch
+constexpr size_t kScanBufBytes = sizeof(unsigned long long) * (kScanMaxTiles + 1);
 
 // Limits of galphaEdgeListNoAlloc (noalloc.cu), set by galphaSetLimits(NULL, ...).
 void noalloc_set_limits(int spin_limit, int hold_first);
@@ -550,7 +570,9 @@ int launch_column_pass_cells(Ctx &c, int T, int W2, int cells, const uint32_t *o
                              int16_t *ycol);
 // LSD radix sort of (keys, vals) ascending (sort.cu)
 int radix_sort(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *keys2, int *vals2, int n,
-               bool *in_second);
+               bool *in_second, bool defer = false);
+int radix_sort_finish(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *keys2, int *vals2, int n,
+                      bool *in_second, bool fresh);
 int radix_sort32(Ctx &c, unsigned int *keys, int *vals, unsigned int *keys2, int *vals2, int n, int *scratch,
                  int key_bits = 0);
 // Stable sort by the low nbits of 32-bit set ids, moving (keys, vals) along;

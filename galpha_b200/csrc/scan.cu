@@ -3,11 +3,14 @@
 // Replaces the reference's recursive Blelloch scan (cudaScanLargeArray.cu:
 // 222-477, prescanArray) and its host-side row prefix sum
 // (cudaReconstruction.cu:470-478).  Each block scans a 4096-element tile held
-// in registers (16 per thread) with warp shuffles.  Up to 32736 tiles, one
+// in registers (16 per thread) with warp shuffles.  Up to 32768 tiles, one
 // launch scans the whole array (tile offsets by decoupled look-back, int4
 // accesses); above that, tile sums are scanned recursively and a final pass
-// adds the tile offsets.  Scratch comes from a per-handle buffer, so a scan
-// allocates nothing.
+// adds the tile offsets.  Scratch comes from per-handle buffers, so a scan
+// allocates nothing, and its status words carry the scan's number, so it
+// clears nothing either: a scan is one launch (two memsets and, for a single
+// tile, two copies around it made it three to five before; 50 us of a call of
+// 1,000 points).
 #include "internal.cuh"
 
 namespace galpha {
@@ -124,20 +127,22 @@ static int scan_rec(Ctx &c, const int *in, int *out, long long n, int *scratch)
 // broken invariant and reports it in the counter block.
 constexpr unsigned long long kScAgg = 1ull << 62;  // status: the tile's own sum
 constexpr unsigned long long kScPre = 2ull << 62;  // status: the sum of this and all earlier tiles
-constexpr unsigned long long kScVal = (1ull << 62) - 1;
+// Status words: bits 63-62 kind, 61-32 the scan's number on this handle (a word
+// of another scan counts as not published), 31-0 the sum.  The scratch
+// belongs to the handle and to scans alone, so an old word is always an older
+// scan's.  A word carries its own payload, so relaxed accesses suffice.
+constexpr unsigned long long kScTag = ((1ull << 30) - 1) << 32;
 constexpr int kScanSpinLimit = 1 << 22;
-constexpr int kScanStatusOff = 64;  // ints before the status words in the scratch (ticket at [2])
-constexpr long long kScanMaxTiles = (65536 - kScanStatusOff) / 2;
 
-__device__ __forceinline__ void sc_st_release(unsigned long long *p, unsigned long long v)
+__device__ __forceinline__ void sc_st(unsigned long long *p, unsigned long long v)
 {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ unsigned long long sc_ld_acquire(const unsigned long long *p)
+__device__ __forceinline__ unsigned long long sc_ld(const unsigned long long *p)
 {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -151,12 +156,16 @@ static_assert(kScanSlices * (kScanThreads / 32) == 32, "one warp scans the parti
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_1p(const int *__restrict__ in, int *__restrict__ out,
                                                           long long n, unsigned long long *status, int *ticket,
-                                                          int *total, Counters *ct, bool vec)
+                                                          unsigned long long tag, int *total, Counters *ct, bool vec)
 {
     __shared__ int s_tile;
     __shared__ long long s_excl;
     __shared__ int s_part[32];
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
+    if (threadIdx.x == 0) {
+        const int t = gridDim.x > 1 ? atomicAdd(ticket, 1) : 0;
+        if (gridDim.x > 1 && t == (int)gridDim.x - 1) *ticket = 0;  // every tile is taken: ready for the next scan
+        s_tile = t;
+    }
     __syncthreads();
     const int tile = s_tile;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -190,14 +199,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_1p(const int *__restrict_
     if (threadIdx.x < 32) {
         long long acc = 0;
         if (tile > 0) {
-            if (lane == 0) sc_st_release(&status[tile], kScAgg | (unsigned long long)(unsigned)tot);
+            if (lane == 0) sc_st(&status[tile], kScAgg | tag | (unsigned long long)(unsigned)tot);
             bool bad = false;
             for (int j = tile - 1;; j -= 32) {
                 const int idx = j - lane;
-                unsigned long long wd = kScPre;  // before tile 0: nothing to add
+                unsigned long long wd = kScPre | tag;  // before tile 0: nothing to add
                 if (idx >= 0) {
                     int spins = 0;
-                    while (((wd = sc_ld_acquire(&status[idx])) >> 62) == 0) {
+                    while (((wd = sc_ld(&status[idx])) >> 62) == 0 || (wd & kScTag) != tag) {
                         if (++spins > kScanSpinLimit) {
                             bad = true;
                             break;
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_1p(const int *__restrict_
                 }
                 const unsigned pre = __ballot_sync(0xffffffffu, (wd >> 62) == 2);
                 const int first = pre ? __ffs(pre) - 1 : 31;  // lanes up to the nearest prefix count
-                long long mine = (lane <= first && idx >= 0) ? (long long)(wd & kScVal) : 0;
+                long long mine = (lane <= first && idx >= 0) ? (long long)(unsigned)wd : 0;
                 for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
                 acc += mine;
                 if (pre) break;
@@ -219,7 +228,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_1p(const int *__restrict_
             if (bad && lane == 0) set_err(ct, GPUDT_ERR_NOCONVERGE, 97);
         }
         if (lane == 0) {
-            sc_st_release(&status[tile], kScPre | (unsigned long long)(acc + tot));
+            if (gridDim.x > 1) sc_st(&status[tile], kScPre | tag | (unsigned)(acc + tot));
             s_excl = acc;
         }
     }
@@ -252,13 +261,16 @@ int exclusive_scan_int(Ctx &c, const int *in, int *out, int n, int *total_dev)
         return GPUDT_OK;
     }
     const long long tiles = ((long long)n + kScanTile - 1) / kScanTile;
-    if (tiles > 1 && tiles <= kScanMaxTiles) {
-        int *ticket = c.hist + 2;
-        unsigned long long *status = reinterpret_cast<unsigned long long *>(c.hist + kScanStatusOff);
-        GALPHA_CUDA(cudaMemsetAsync(ticket, 0, sizeof(int), c.stream));
-        GALPHA_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (size_t)tiles, c.stream));
+    if (tiles <= kScanMaxTiles) {
+        if (++c.scan_no >= (1u << 30)) {  // the numbers start over: no word of the first run may be left
+            GALPHA_CUDA(cudaMemsetAsync(c.scan_buf, 0, kScanBufBytes, c.stream));
+            c.scan_no = 1;
+        }
+        int *ticket = reinterpret_cast<int *>(c.scan_buf + kScanMaxTiles);
         const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-        k_scan_1p<<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(in, out, n, status, ticket, total_dev, c.ctr, vec);
+        k_scan_1p<<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(in, out, n, c.scan_buf, ticket,
+                                                                  (unsigned long long)c.scan_no << 32, total_dev, c.ctr,
+                                                                  vec);
         count_launch();
         GALPHA_CUDA(cudaGetLastError());
         return GPUDT_OK;

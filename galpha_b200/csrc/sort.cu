@@ -260,9 +260,9 @@ struct FixFind {
     Counters *ct;
     __device__ void long_pair(int i) const
     {
-        const int k = atomicAdd(&ct->nlong, 1);
+        const int k = atomicAdd(&ct->fx_long, 1);
         if (k < lcap) longs[k] = i;
-        else ct->changed = 1;  // too many: full sort
+        else ct->fx_many = 1;  // too many: full sort
     }
     __device__ void operator()(long long ii) const
     {
@@ -291,7 +291,7 @@ struct FixFind {
         const unsigned m = __activemask();
         const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
         int base = 0;
-        if (lane == leader) base = atomicAdd(&ct->nlist2, __popc(m));
+        if (lane == leader) base = atomicAdd(&ct->fx_groups, __popc(m));
         base = __shfl_sync(m, base, leader);
         starts[base + __popc(m & ((1u << lane) - 1u))] = s;
     }
@@ -651,8 +651,9 @@ static int onesweep_top(Ctx &c, unsigned long long *keys, int *vals, unsigned lo
     const long long tiles = ((long long)n + kRsTile - 1) / kRsTile;
     int *ghist = c.rhist, *tickets = c.rhist + kOsTicketOff;
     unsigned long long *status = reinterpret_cast<unsigned long long *>(c.rhist + kOsHeadInts);
-    GALPHA_CUDA(cudaMemsetAsync(ghist, 0, sizeof(int) * (kOsTicketOff + 8), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * 256 * (size_t)tiles, c.stream));
+    // digit counts, tickets and status words, one after the other
+    GALPHA_CUDA(cudaMemsetAsync(ghist, 0, sizeof(int) * kOsHeadInts + sizeof(unsigned long long) * 256 * (size_t)tiles,
+                                c.stream));
     {
         const long long blocks = std::max(1ll, std::min<long long>((n + 1023) / 1024, (long long)c.sm_count * 8));
         k_rs_hist_top<<<(unsigned)blocks, 256, 0, c.stream>>>(keys, n, ghist);
@@ -676,9 +677,26 @@ static int onesweep_top(Ctx &c, unsigned long long *keys, int *vals, unsigned lo
 
 // The result is left in (keys, vals) or, when *in_second comes back true, in
 // (keys2, vals2): where the last digit pass left it, since a copy back would
-// cost a full read and write of both arrays.
+// cost a full read and write of both arrays.  The fx_* counters must be zero.
+// With `defer` the short groups are fixed from the count on the device and the
+// host looks at nothing: the caller must call radix_sort_finish after its next
+// counter read when fx_long or fx_many is set.
+struct FixScratch {
+    int *starts, *longs;
+    int lcap;
+    FixScratch(unsigned long long *fk, int n)
+    {
+        // in the other key buffer (2n ints, free now): group starts (at most
+        // n / 2), then the long pairs and their extents (3 ints each)
+        starts = (int *)fk;
+        const long long soff = ((long long)n / 2 + 2) & ~1ll;
+        lcap = std::max(0, (int)(std::min<long long>(kMaxLongPairs, (2ll * n - soff) / 3) & ~1ll));
+        longs = starts + soff;
+    }
+};
+
 int radix_sort(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *keys2, int *vals2, int n,
-               bool *in_second)
+               bool *in_second, bool defer)
 {
     bool sec = false;
     int r;
@@ -691,30 +709,50 @@ int radix_sort(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *
     *in_second = sec;
     if (r || n <= 1) return r;
     unsigned long long *rk = sec ? keys2 : keys, *fk = sec ? keys : keys2;
-    int *rv = sec ? vals2 : vals, *fv = sec ? vals : vals2;
-    // group fix-up in the other key buffer (2n ints, free now): group starts
-    // (at most n / 2), then the long pairs and their extents (3 ints each)
-    int *starts = (int *)fk;
-    const long long soff = ((long long)n / 2 + 2) & ~1ll;
-    const int lcap = (int)(std::min<long long>(kMaxLongPairs, (2ll * n - soff) / 3) & ~1ll);
-    int *longs = starts + soff;
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlist2, 0, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nlong, 0, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
+    int *rv = sec ? vals2 : vals;
+    const FixScratch f(fk, n);
     {
         const long long blocks = std::max(1ll, std::min<long long>(((long long)n / 8 + 255) / 256, (long long)c.sm_count * 8));
-        k_fix_find<<<(unsigned)blocks, 256, 0, c.stream>>>(rk, starts, longs, n, std::max(lcap, 0), c.ctr);
+        k_fix_find<<<(unsigned)blocks, 256, 0, c.stream>>>(rk, f.starts, f.longs, n, f.lcap, c.ctr);
         count_launch();
+    }
+    if (defer) {
+        launch_dev(c, FixGroups{rk, rv, f.starts, n}, &c.ctr->fx_groups, n / 2);
+        GALPHA_CUDA(cudaGetLastError());
+        return GPUDT_OK;
     }
     r = read_counters(c);
     if (r) return r;
     if (c.hctr->err) return stage_fail(c, c.hctr->err, "spectrum sort");
-    const int nlong = std::min(c.hctr->nlong, std::max(lcap, 0));
+    return radix_sort_finish(c, keys, vals, keys2, vals2, n, in_second, true);
+}
+
+// The groups k_fix_find reported (counters already read): the short ones
+// unless they have been fixed, and the long ones.  Called after a deferred
+// sort, the list of long pairs in the other key buffer is stale, and is made
+// again first.
+int radix_sort_finish(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *keys2, int *vals2, int n,
+                      bool *in_second, bool fresh)
+{
+    const bool sec = *in_second;
+    unsigned long long *rk = sec ? keys2 : keys, *fk = sec ? keys : keys2;
+    int *rv = sec ? vals2 : vals, *fv = sec ? vals : vals2;
+    const FixScratch f(fk, n);
+    int r;
+    if (!fresh) {
+        GALPHA_CUDA(cudaMemsetAsync(&c.ctr->fx_groups, 0, 3 * sizeof(int), c.stream));  // fx_groups, fx_long, fx_many
+        const long long blocks = std::max(1ll, std::min<long long>(((long long)n / 8 + 255) / 256, (long long)c.sm_count * 8));
+        k_fix_find<<<(unsigned)blocks, 256, 0, c.stream>>>(rk, f.starts, f.longs, n, f.lcap, c.ctr);
+        count_launch();
+        r = read_counters(c);
+        if (r) return r;
+    }
+    const int nlong = std::min(c.hctr->fx_long, f.lcap);
     std::vector<int2> groups;
-    if (!c.hctr->changed && nlong > 0) {
+    if (!c.hctr->fx_many && nlong > 0) {
         // extents of the long groups, merged on the host
-        int2 *ext = reinterpret_cast<int2 *>(longs + lcap);
-        k_group_extent<<<(unsigned)nlong, 256, 0, c.stream>>>(rk, n, longs, ext);
+        int2 *ext = reinterpret_cast<int2 *>(f.longs + f.lcap);
+        k_group_extent<<<(unsigned)nlong, 256, 0, c.stream>>>(rk, n, f.longs, ext);
         count_launch();
         GALPHA_CUDA(cudaGetLastError());
         std::vector<int2> h(nlong);
@@ -724,13 +762,13 @@ int radix_sort(Ctx &c, unsigned long long *keys, int *vals, unsigned long long *
         for (const int2 &g : h)
             if (groups.empty() || g.x != groups.back().x) groups.push_back(g);
     }
-    if (c.hctr->changed || groups.size() > (size_t)kMaxLongGroups) {
+    if (c.hctr->fx_many || groups.size() > (size_t)kMaxLongGroups) {
         bool sec2 = false;
         r = radix_sort_keys<unsigned long long>(c, rk, rv, fk, fv, n, c.rhist, 0, &sec2);
         if (sec2) *in_second = !sec;
         return r;
     }
-    if (c.hctr->nlist2 > 0) launch_n(c, FixGroups{rk, rv, starts, n}, c.hctr->nlist2);
+    if (c.hctr->fx_groups > 0) launch_n(c, FixGroups{rk, rv, f.starts, n}, c.hctr->fx_groups);
     GALPHA_CUDA(cudaGetLastError());
     // each long group as a sub-array (the other buffers are free now)
     for (const int2 &g : groups) {
