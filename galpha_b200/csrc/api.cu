@@ -166,6 +166,7 @@ static size_t plan(const Sizes &z, Ctx *c, Arena *A)
     TAKE(outtri, gpudtTriangle, cap);
     TAKE(edge_aos, galphaEdgeInterval, 2 * cap);
     TAKE(qclass, uint8_t, V + 3 * cap);
+    TAKE(longfan, unsigned char, small_mesh_scratch_bytes());
     TAKE(ctr, Counters, 1);
 #undef TAKE
     return total + 4096;
@@ -250,6 +251,41 @@ int stage_fail(Ctx &c, int r, const char *stage)
     return r;
 }
 
+// Shifting to flipping: each stage as launches of its own, or, while the mesh
+// is small for that stage, in one launch with its neighbours.
+static int mesh_stages(Ctx &c)
+{
+    static const char *const names[] = {"shift", "missing", "boundary", "flip"};
+    const bool few = c.V <= kSmShiftV;
+    bool one[] = {few, few, c.F <= (few ? kSmBoundaryFSmall : kSmBoundaryF), c.V <= kSmFlipV};
+    c.small_mesh = 0;
+    int r;
+    for (int s = kSmShift; s <= kSmFlip;) {
+        int next = s + 1;
+        const char *stage = names[s];
+        if (one[s]) {
+            int to = s;
+            while (to < kSmFlip && one[to + 1] && !(to == kSmBoundary && c.n_cons > 0)) to++;
+            r = stage_small(c, s, to, &next);
+            if (r) return stage_fail(c, r, to > s ? "mesh" : stage);
+            for (int k = s; k < next; k++) c.small_mesh |= 1u << k;
+            if (next <= to) one[next] = false;  // too many missing sites for it
+            for (int k = s; k < next; k++) c.reads_at[4 + k] = c.host_reads;
+        } else {
+            r = s == kSmShift ? stage_shift(c) : s == kSmMissing ? stage_missing(c) : s == kSmBoundary ? stage_boundary(c)
+                                                                                                  : stage_flip(c);
+            if (r) return stage_fail(c, r, stage);
+        }
+        if (next == kSmFlip) {
+            r = stage_constraints(c);
+            if (r) return stage_fail(c, r, "constraints");
+        }
+        s = next;
+        ev_record(c, 3 + s);
+    }
+    return GPUDT_OK;
+}
+
 // DT of n device points (interleaved xy).  Leaves the compacted mesh in c.cv/c.cn.
 static int run_dt(HandleState &H, const double *d_xy, int n, double minX, double minY, double maxX, double maxY,
                   int T)
@@ -274,6 +310,7 @@ static int run_dt(HandleState &H, const double *d_xy, int n, double minX, double
         c.N = n;
         c.nT_out = 0;
         c.have_mesh = true;
+        c.small_mesh = 0;
         for (int k = 2; k <= 8; k++) ev_record(c, k);
         return GPUDT_OK;
     }
@@ -288,15 +325,8 @@ static int run_dt(HandleState &H, const double *d_xy, int n, double minX, double
     STAGE("triangles", stage_triangles(c));
     STAGE("links", stage_links(c));
     ev_record(c, 3);
-    STAGE("shift", stage_shift(c));
-    ev_record(c, 4);
-    STAGE("missing", stage_missing(c));
-    ev_record(c, 5);
-    STAGE("boundary", stage_boundary(c));
-    STAGE("constraints", stage_constraints(c));
-    ev_record(c, 6);
-    STAGE("flip", stage_flip(c));
-    ev_record(c, 7);
+    r = mesh_stages(c);
+    if (r) return r;
     STAGE("compact", stage_compact(c));
 #undef STAGE
     ev_record(c, 8);
@@ -361,15 +391,8 @@ static int run_batch(HandleState &H, int K, const int *sizes, const double *d_xy
     ev_record(c, 2);
     STAGE("links", stage_links(c));
     ev_record(c, 3);
-    STAGE("shift", stage_shift(c));
-    ev_record(c, 4);
-    STAGE("missing", stage_missing(c));
-    ev_record(c, 5);
-    STAGE("boundary", stage_boundary(c));
-    STAGE("constraints", stage_constraints(c));
-    ev_record(c, 6);
-    STAGE("flip", stage_flip(c));
-    ev_record(c, 7);
+    r = mesh_stages(c);
+    if (r) return r;
     STAGE("compact", batch_compact(c, H.bd, bh));
     ev_record(c, 8);
     c.have_mesh = true;
@@ -409,6 +432,11 @@ static void fill_times(Ctx &c, int last)
     cudaEventSynchronize(c.ev[last]);
     for (int k = 1; k < last; k++) {
         float ms = 0.f;
+        if (k >= 3 && k < 7 && ((c.small_mesh >> (k - 3)) & 1u)) {  // inside a launch: the device's own clock
+            c.st.ms[k] = c.small_ms[k - 3];
+            c.st.hostReadsStage[k] = c.reads_at[k + 1] - c.reads_at[k];
+            continue;
+        }
         if (cudaEventElapsedTime(&ms, c.ev[k], c.ev[k + 1]) == cudaSuccess && k < 12) c.st.ms[k] = ms;
         if (k < 12) c.st.hostReadsStage[k] = c.reads_at[k + 1] - c.reads_at[k];
     }

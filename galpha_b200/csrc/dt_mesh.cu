@@ -1447,150 +1447,163 @@ struct FrRule {
     }
 };
 
+// What the lanes of a removal share besides the arrays.
+struct FrWarp {
+    int top[kFrPieces], used[kFrPieces];
+    int top2, cl, co;
+};
+
+// Removes one selected unit (one warp); mem: fake_remove_smem(M) bytes, 16-byte
+// aligned, M at least its fan's length.
+__device__ void fake_remove_item(const FakeRemoveArgs &a, int item, int M, unsigned char *mem, FrWarp &w)
+{
+    int *Fs = (int *)mem, *Fi = Fs + M, *O = Fi + M, *U = O + M, *S = U + M + 1, *SO = S + M + 1 + kFrPieces;
+    double2 *P = (double2 *)(mem + (fake_remove_ints(M) * sizeof(int) + 15) / 16 * 16);
+    const int lane = threadIdx.x & 31;
+    const int f = a.list[item], d = a.fanlen[item] & 0xffff, nsh = a.fanlen[item] >> 16,
+              base = a.fanoff[item];
+    for (int k = lane; k < d; k += 32) {
+        const int2 q = a.fan[base + k];
+        const int t = dtri(q.x), i = dori(q.x);
+        Fs[k] = t;
+        Fi[k] = i;
+        O[k] = q.y;
+        const int4 w = a.tv[t];
+        U[k] = geti(w, p1(i));
+        if (k == d - 1) U[d] = geti(w, m1(i));
+        a.epoch[t] = a.round;
+        const int fk = geti(w, i);  // the fake of this fan triangle (a run has several)
+        if (fk != f) {
+            a.vtri[fk] = -1;
+            a.vstate[fk] = VS_GONE;
+        }
+    }
+    __syncwarp();
+    for (int k = lane; k <= d; k += 32) P[k] = a.pos[U[k]];
+    // every one of the d chain edges ends with exactly one relink record,
+    // at rbase + its index (linked to a new triangle, or left as a hull edge)
+    int rbase = 0;
+    if (lane == 0 && d > 0) rbase = atomicAdd(a.nrec, d);
+    rbase = __shfl_sync(0xffffffffu, rbase, 0);
+    __syncwarp();
+    const int G = max(1, min(kFrPieces, d / kFrMinPiece));
+    int nrec_orig = 0;
+    OrientTally tally;
+    const FrRule rule{a, Fs, Fi, O, U, P, rbase, &nrec_orig};
+    // 1. each lane's piece [b0, b1]; its stack at S + b0 + lane
+    const int b0 = (int)((long long)lane * d / G), b1 = (int)((long long)(lane + 1) * d / G);
+    if (lane < G) {
+        int *LS = S + b0 + lane, *LSO = SO + b0 + lane;
+        int top = 0, used = 0;
+        for (int k = b0; k <= b1; k++)
+            top = rule.push(LS, LSO, top, k, k > b0 ? -2 - (k - 1) : -1, [&] { return Fs[b0 + used++]; },
+                            tally);
+        w.top[lane] = top;
+        w.used[lane] = used;
+    }
+    __syncwarp();
+    // 2. lane 0: the leftover stacks in order (a piece's first vertex is the
+    // previous piece's last); the stack is rebuilt in place at S[0..)
+    // (it never passes the entry being read).  Slots: the pieces' unused
+    // ones, in piece order.
+    if (lane == 0) {
+        int cl = 0, co = 0;  // next free slot: piece cl, offset co past its used ones
+        auto take = [&]() {
+            for (; cl < G; cl++, co = 0) {
+                const int pb0 = (int)((long long)cl * d / G), pb1 = (int)((long long)(cl + 1) * d / G);
+                if (pb0 + w.used[cl] + co < pb1) return Fs[pb0 + w.used[cl] + co++];
+            }
+            return -1;
+        };
+        int top2 = 0;
+        for (int L = 0; L < G; L++) {
+            const int pb0 = (int)((long long)L * d / G);
+            for (int j = L == 0 ? 0 : 1; j < w.top[L]; j++) {
+                const int idx = pb0 + L + j;
+                top2 = rule.push(S, SO, top2, S[idx], SO[idx], take, tally);
+            }
+        }
+        w.top2 = top2;
+        w.cl = cl;
+        w.co = co;
+    }
+    __syncwarp();
+    tally.flush(a.ct);
+    const int top = w.top2, cl = w.cl, co = w.co;
+    // 3. the remaining chain edges are hull edges now
+    for (int k = 1 + lane; k < top; k += 32) {
+        const int ownv = SO[k];
+        if (ownv > -2) {
+            set_link(a.tn, ownv, -1);
+        } else {
+            const int q = -2 - ownv;
+            set_fwd(a.fwd, Fs[q], Fi[q], -1);
+            a.rec[rbase + q] = Relink{-1, O[q]};
+            nrec_orig++;
+        }
+    }
+    {
+        int tot = nrec_orig;
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        if (lane == 0 && tot != d) set_err(a.ct, GPUDT_ERR_TOPOLOGY, 74);
+    }
+    {
+        // released slots: each piece's unused ones past what step 2 took
+        int mine = 0, from = 0;
+        if (lane < G && lane >= cl) {
+            from = b0 + w.used[lane] + (lane == cl ? co : 0);
+            mine = max(0, b1 - from);
+        }
+        int incl = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int nrel = __shfl_sync(0xffffffffu, incl, 31);
+        int cb = 0, fb = 0;
+        if (lane == 0) {
+            cb = atomicAdd(&a.ct->ncand, top);
+            fb = nrel || nsh ? atomicAdd(&a.ct->nfree, nrel + nsh) : 0;
+        }
+        cb = __shfl_sync(0xffffffffu, cb, 0);
+        fb = __shfl_sync(0xffffffffu, fb, 0);
+        for (int k = lane; k < top; k += 32) a.cand[cb + k] = U[S[k]];
+        for (int k = 0; k < mine; k++) {
+            const int t = Fs[from + k];
+            a.tv[t] = make_int4(-1, -1, -1, 0);
+            a.freelist[fb + incl - mine + k] = t;
+        }
+        // triangles shared by consecutive members of a run: inside the removed
+        // region.  Both members are marked here: a middle member whose fan is
+        // just its two shared triangles has no kept entry to be marked by.
+        for (int k = lane; k < nsh; k += 32) {
+            const int e = a.fan[base + d + k].x, t = dtri(e), i = dori(e);
+            const int4 w = a.tv[t];
+            const int m0 = geti(w, i), m2 = geti(w, m1(i));  // this member, the next one
+            a.vtri[m0] = -1;
+            a.vstate[m0] = VS_GONE;
+            a.vtri[m2] = -1;
+            a.vstate[m2] = VS_GONE;
+            a.tv[t] = make_int4(-1, -1, -1, 0);
+            a.freelist[fb + nrel + k] = t;
+        }
+    }
+    if (lane == 0) {
+        a.vtri[f] = -1;
+        a.vstate[f] = VS_GONE;
+    }
+}
+
 // Items whose fan has dmin..M triangles (the short and the long launch).
 __global__ void __launch_bounds__(32) k_fake_remove(FakeRemoveArgs a, const int *n_dev, int M, int dmin)
 {
     extern __shared__ __align__(16) unsigned char fr_smem[];
-    int *Fs = (int *)fr_smem, *Fi = Fs + M, *O = Fi + M, *U = O + M, *S = U + M + 1, *SO = S + M + 1 + kFrPieces;
-    double2 *P = (double2 *)(fr_smem + (fake_remove_ints(M) * sizeof(int) + 15) / 16 * 16);
-    __shared__ int s_top[kFrPieces], s_used[kFrPieces];
-    __shared__ int s_top2, s_cl, s_co;
-    const int lane = threadIdx.x;
+    __shared__ FrWarp s_warp;
     const int n = *n_dev;
     for (int item = blockIdx.x; item < n; item += gridDim.x) {
-        const int f = a.list[item], d = a.fanlen[item] & 0xffff, nsh = a.fanlen[item] >> 16,
-                  base = a.fanoff[item];
+        const int d = a.fanlen[item] & 0xffff;
         if (d < dmin || d > M) continue;  // the other launch's item
-        for (int k = lane; k < d; k += 32) {
-            const int2 q = a.fan[base + k];
-            const int t = dtri(q.x), i = dori(q.x);
-            Fs[k] = t;
-            Fi[k] = i;
-            O[k] = q.y;
-            const int4 w = a.tv[t];
-            U[k] = geti(w, p1(i));
-            if (k == d - 1) U[d] = geti(w, m1(i));
-            a.epoch[t] = a.round;
-            const int fk = geti(w, i);  // the fake of this fan triangle (a run has several)
-            if (fk != f) {
-                a.vtri[fk] = -1;
-                a.vstate[fk] = VS_GONE;
-            }
-        }
-        __syncwarp();
-        for (int k = lane; k <= d; k += 32) P[k] = a.pos[U[k]];
-        // every one of the d chain edges ends with exactly one relink record,
-        // at rbase + its index (linked to a new triangle, or left as a hull edge)
-        int rbase = 0;
-        if (lane == 0 && d > 0) rbase = atomicAdd(a.nrec, d);
-        rbase = __shfl_sync(0xffffffffu, rbase, 0);
-        __syncwarp();
-        const int G = max(1, min(kFrPieces, d / kFrMinPiece));
-        int nrec_orig = 0;
-        OrientTally tally;
-        const FrRule rule{a, Fs, Fi, O, U, P, rbase, &nrec_orig};
-        // 1. each lane's piece [b0, b1]; its stack at S + b0 + lane
-        const int b0 = (int)((long long)lane * d / G), b1 = (int)((long long)(lane + 1) * d / G);
-        if (lane < G) {
-            int *LS = S + b0 + lane, *LSO = SO + b0 + lane;
-            int top = 0, used = 0;
-            for (int k = b0; k <= b1; k++)
-                top = rule.push(LS, LSO, top, k, k > b0 ? -2 - (k - 1) : -1, [&] { return Fs[b0 + used++]; },
-                                tally);
-            s_top[lane] = top;
-            s_used[lane] = used;
-        }
-        __syncwarp();
-        // 2. lane 0: the leftover stacks in order (a piece's first vertex is the
-        // previous piece's last); the stack is rebuilt in place at S[0..)
-        // (it never passes the entry being read).  Slots: the pieces' unused
-        // ones, in piece order.
-        if (lane == 0) {
-            int cl = 0, co = 0;  // next free slot: piece cl, offset co past its used ones
-            auto take = [&]() {
-                for (; cl < G; cl++, co = 0) {
-                    const int pb0 = (int)((long long)cl * d / G), pb1 = (int)((long long)(cl + 1) * d / G);
-                    if (pb0 + s_used[cl] + co < pb1) return Fs[pb0 + s_used[cl] + co++];
-                }
-                return -1;
-            };
-            int top2 = 0;
-            for (int L = 0; L < G; L++) {
-                const int pb0 = (int)((long long)L * d / G);
-                for (int j = L == 0 ? 0 : 1; j < s_top[L]; j++) {
-                    const int idx = pb0 + L + j;
-                    top2 = rule.push(S, SO, top2, S[idx], SO[idx], take, tally);
-                }
-            }
-            s_top2 = top2;
-            s_cl = cl;
-            s_co = co;
-        }
-        __syncwarp();
-        tally.flush(a.ct);
-        const int top = s_top2, cl = s_cl, co = s_co;
-        // 3. the remaining chain edges are hull edges now
-        for (int k = 1 + lane; k < top; k += 32) {
-            const int ownv = SO[k];
-            if (ownv > -2) {
-                set_link(a.tn, ownv, -1);
-            } else {
-                const int q = -2 - ownv;
-                set_fwd(a.fwd, Fs[q], Fi[q], -1);
-                a.rec[rbase + q] = Relink{-1, O[q]};
-                nrec_orig++;
-            }
-        }
-        {
-            int tot = nrec_orig;
-            for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-            if (lane == 0 && tot != d) set_err(a.ct, GPUDT_ERR_TOPOLOGY, 74);
-        }
-        {
-            // released slots: each piece's unused ones past what step 2 took
-            int mine = 0, from = 0;
-            if (lane < G && lane >= cl) {
-                from = b0 + s_used[lane] + (lane == cl ? co : 0);
-                mine = max(0, b1 - from);
-            }
-            int incl = mine;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int nrel = __shfl_sync(0xffffffffu, incl, 31);
-            int cb = 0, fb = 0;
-            if (lane == 0) {
-                cb = atomicAdd(&a.ct->ncand, top);
-                fb = nrel || nsh ? atomicAdd(&a.ct->nfree, nrel + nsh) : 0;
-            }
-            cb = __shfl_sync(0xffffffffu, cb, 0);
-            fb = __shfl_sync(0xffffffffu, fb, 0);
-            for (int k = lane; k < top; k += 32) a.cand[cb + k] = U[S[k]];
-            for (int k = 0; k < mine; k++) {
-                const int t = Fs[from + k];
-                a.tv[t] = make_int4(-1, -1, -1, 0);
-                a.freelist[fb + incl - mine + k] = t;
-            }
-            // triangles shared by consecutive members of a run: inside the removed
-            // region.  Both members are marked here: a middle member whose fan is
-            // just its two shared triangles has no kept entry to be marked by.
-            for (int k = lane; k < nsh; k += 32) {
-                const int e = a.fan[base + d + k].x, t = dtri(e), i = dori(e);
-                const int4 w = a.tv[t];
-                const int m0 = geti(w, i), m2 = geti(w, m1(i));  // this member, the next one
-                a.vtri[m0] = -1;
-                a.vstate[m0] = VS_GONE;
-                a.vtri[m2] = -1;
-                a.vstate[m2] = VS_GONE;
-                a.tv[t] = make_int4(-1, -1, -1, 0);
-                a.freelist[fb + nrel + k] = t;
-            }
-        }
-        if (lane == 0) {
-            a.vtri[f] = -1;
-            a.vstate[f] = VS_GONE;
-        }
+        fake_remove_item(a, item, M, fr_smem, s_warp);
         __syncwarp();
     }
 }
@@ -2842,6 +2855,17 @@ int stage_constraints(Ctx &c)
     c.cons_rounds = round;
     c.st.constraintRounds = round;
     return GPUDT_OK;
+}
+
+}  // namespace galpha
+
+#include "mesh_small.cuh"
+
+namespace galpha {
+
+size_t small_mesh_scratch_bytes()
+{
+    return kSmMaxBlocks * fake_remove_smem(kMaxFanLong);
 }
 
 // ----------------------------------------------------------------- compact

@@ -27,6 +27,20 @@ constexpr int kSpinLimit = 1 << 22;              // bound of every look-back wai
 constexpr int kBlockRun = 1 << 16;
 constexpr int kShiftGroupDefault = 4, kMissingGroupDefault = 2, kFlipSyncDefault = 4;
 constexpr int kTailEnterDefault = 4096, kTailLeaveDefault = 32768;
+// Mesh stages that one launch can run in a row (mesh_small.cuh), and up to
+// which size each of them does.  Stage times in us, in one launch against
+// launches of its own (uniform points unless said otherwise, B200):
+//   shift     109 / 256 at 12,000 points, 288 / 395 at 200,000, 350 / 390 at
+//             400,000, but 873 / 764 at 400,000 clustered
+//   missing   41 / 79 at 12,000, 66 / 132 at 100,000, but 333 / 244 at 55,000
+//             clustered, about 14,000 sites: more than kSmMissLimit sites want
+//             the whole GPU
+//   boundary  198 / 343 at 12,000, 287 / 397 at 100,000, 467 / 493 at 1,000,000
+//             (1,024 ring sites), but 743 / 645 at 4,000,000 (2,048 sites, long
+//             fans)
+//   flip      85 / 124 at 12,000, 108 / 136 at 25,000, but 170 / 154 at 40,000
+enum { kSmShift = 0, kSmMissing = 1, kSmBoundary = 2, kSmFlip = 3 };
+constexpr int kSmShiftV = 262144, kSmMissLimit = 8192, kSmBoundaryF = 1024, kSmBoundaryFSmall = 4096, kSmFlipV = 28672;
 constexpr int kMaxGroup = 8;   // rounds between two counter reads
 // Per-round counts live in rings of kRing words: round k counts in word
 // k mod kRing and clears the word of round k + kRing / 2, so that the words of
@@ -99,6 +113,13 @@ struct Counters {
     int r_act[kRing];    // flip: active-list length of a round
     int r_cand[kRing];   // flip: candidates of a round
     int r_frec[kRing];   // flip: relink records of a round
+    // small meshes (one launch for the mesh stages)
+    int sm_stop;     // the error word as of a round's last phase
+    int sm_next;     // first stage not run
+    int sm_rec;      // words of r_rec taken so far
+    int sm_round;    // last operation round id
+    int sm_shift, sm_missing, sm_flip;  // rounds run
+    unsigned long long sm_ns[5];        // device time at the start of shift, missing, boundary, flip, and at the end
     // predicate stage counts, each spread over 64 counters (one per warp id mod
     // 64); last, because only a call's final read takes them along
     unsigned long long filt_spread[64];  // in-circle tests decided by the FP64 filter
@@ -207,6 +228,9 @@ struct Ctx {
     bool outtri_ready = false;          // outtri holds the current mesh (built on the first download)
     bool want_outtri = false;           // this call needs outtri: compaction writes it directly
     galphaEdgeInterval *edge_aos = nullptr;  // [2*cap] edge records for download
+    unsigned char *longfan = nullptr;  // small meshes: a fan too long for shared memory, per block
+    float small_ms[4] = {0, 0, 0, 0};  // small meshes: shift, missing, boundary, flip times on the device
+    unsigned small_mesh = 0;           // stages the current call ran that way (bit kSm*)
 
     DevBuf bufs[64];
     int nbufs = 0;
@@ -470,6 +494,8 @@ int stage_missing(Ctx &c);
 int stage_boundary(Ctx &c);
 int stage_flip(Ctx &c);
 int stage_constraints(Ctx &c);
+int stage_small(Ctx &c, int from, int to, int *next);  // stages kSm* in one launch
+size_t small_mesh_scratch_bytes();
 int stage_compact(Ctx &c);
 // ------------------------------------------------------------------ batches
 // One point set of a batch: its grid scaling, its texture cell and its
