@@ -24,6 +24,7 @@
 #include <vector>
 #include "internal.cuh"
 #include "exact.cuh"
+#include "block_sort.cuh"
 
 namespace galpha {
 
@@ -129,13 +130,16 @@ __device__ __noinline__ int attached_exact_v(double ix, double iy, double jx, do
 // double-double arithmetic allow), so a round's records are loaded one round
 // ahead, and by the wait for earlier tiles: 4 triangles per thread take 0.57
 // ms at 8.4 M triangles, 2 take 0.64, 1 takes 0.75, 8 by blocks of 128 take
-// 0.80 (longer chains ahead of the tiles that wait).  As five launches (edge
+// 0.80 (longer chains ahead of the tiles that wait).  Up to kAkFew triangles
+// there are too few tiles of four to fill the GPU and one per thread is used
+// (2,000 triangles: 20 us with four, 7 with one).  As five launches (edge
 // counts, a scan, keys, a scan over the edges, edge keys from a second gather)
 // it took 0.77 ms, and a counter read between the first and the third.
 // A status word holds kind (bits 63-62), the edges (61-31) and the unattached
 // edges (30-0) of its tile or of all tiles up to it; fewer than 2^31 edges.
 constexpr int kAkSpinLimit = 1 << 22;
-constexpr int kAkThreads = 256, kAkItems = 4, kAkTile = kAkThreads * kAkItems;
+constexpr int kAkThreads = 256, kAkItemsMany = 4;
+constexpr int kAkFew = 151552;  // 148 SMs x 4 blocks x 256
 constexpr unsigned long long kAkAgg = 1ull << 62, kAkInc = 2ull << 62, kAkVal = (1ull << 62) - 1;
 
 struct AlphaKeysArgs {
@@ -151,11 +155,17 @@ struct AlphaKeysArgs {
     int *slivers;
     unsigned long long *status;  // [tiles], zero; then the ticket
     int tiles;
+    int2 *pt;       // [N] vertex intervals, started here
+    int N;
     Counters *ct;
 };
 
+template <int kAkItems>
 __global__ void __launch_bounds__(kAkThreads, 4) k_alpha_keys(AlphaKeysArgs A)
 {
+    constexpr int kAkTile = kAkThreads * kAkItems;
+    for (int i = blockIdx.x * kAkThreads + threadIdx.x; i < A.N; i += gridDim.x * kAkThreads)
+        A.pt[i] = make_int2(-1, -1);
     __shared__ double s_rho[3 * kAkTile];  // birth time of edge i of the tile's triangle j at [i][j]
     __shared__ int s_part[kAkItems * (kAkThreads / 32)];
     __shared__ int s_tile;
@@ -237,7 +247,7 @@ __global__ void __launch_bounds__(kAkThreads, 4) k_alpha_keys(AlphaKeysArgs A)
         if (lane == 31) s_part[u * (kAkThreads / 32) + w] = x;
 #pragma unroll
         for (int q = 0; q < kAkItems; q++)
-            if (q == u) {
+            if (q == u) {  // (registers have no run-time index)
                 flags[q] = f;
                 cnt[q] = own;
                 incl[q] = x;
@@ -988,8 +998,105 @@ static int alpha_ranks(Ctx &c, AlphaSegs *segs, int nIn, bool defer)
     return GPUDT_OK;
 }
 
+// Intervals of edges and vertices; again: not for the first time since the
+// keys, which start the vertex intervals.
+static int alpha_intervals(Ctx &c, bool again)
+{
+    const int nT = c.nT_out;
+    if (again) GALPHA_CUDA(cudaMemsetAsync(c.pt_nu, 0xff, sizeof(int2) * (size_t)c.N, c.stream));
+    launch_n(c, EdgeIntervals{c.cv, c.cn, c.e_off, c.tri_ro, c.edge_ro, c.edge_nu, c.pt_nu}, nT);
+    GALPHA_CUDA(cudaGetLastError());
+    return read_counters(c);
+}
+
+// Up to kBlockSort entries: the sort, the ranks and the spectrum in one launch
+// of one block, the sorted entries kept in shared memory between them; neighbours
+// within 2 ulp are compared exactly on the spot, and a run out of exact order
+// is only counted (al_slow): the caller then redoes the ranks from the sorted
+// entries, which are written back.  (nT and the number of unattached edges are
+// on the device, so the host need not look before the launch.)  The usual
+// five digits of the key tops come first; only when they leave equal tops out
+// of order (the block knows) are all eight sorted.  1,000 points: RANK_US us,
+// where the passes, the group fix-up, the flags, the scan and the scatter were
+// 13 launches and 85 us, and a counter read.
+__global__ void __launch_bounds__(kBsThreads) k_alpha_rank_block(unsigned long long *keys, int *vals, int nT,
+                                                                 const int4 *cv, const int *edges, const double2 *P,
+                                                                 int *tri_ro, int *edge_ro, double *spectrum,
+                                                                 Counters *ct)
+{
+    extern __shared__ __align__(16) unsigned char bs_smem[];
+    typedef unsigned long long K;
+    BsSmem<K> &S = *reinterpret_cast<BsSmem<K> *>(bs_smem);
+    __shared__ int s_warp[kBsWarps];
+    const int n = nT + ct->al_unatt;
+    if (n > kBlockSort || ct->err) return;
+    auto load = [&](int i, K &k, int &v) {
+        k = keys[1 + i];
+        v = vals[1 + i];
+    };
+    auto store = [&](int i, K k, int v) {
+        keys[1 + i] = k;
+        vals[1 + i] = v;
+    };
+    block_sort(S, n, 24, 5, load, store);
+    bool off = false;  // a pair with equal tops in the wrong order
+    for (int i = 1 + threadIdx.x; i < n; i += kBsThreads) off |= S.key[i] < S.key[i - 1];
+    if (__syncthreads_or(off)) {  // stable: from the top's order as from any other
+        block_sort(S, n, 0, 8, load, store);
+        if (threadIdx.x == 0) ct->fx_many = 1;
+        __syncthreads();
+    }
+    // S.key / S.val hold the sorted entries; the warp's entries in order, 32 at a time
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rounds = (n + kBsThreads - 1) / kBsThreads, base = w * rounds * 32;
+    unsigned starts[kBlockSort / kBsThreads];
+    int before = 0;
+#pragma unroll
+    for (int r = 0; r < kBlockSort / kBsThreads; r++) {
+        if (r >= rounds) break;
+        const int i = base + r * 32 + lane;
+        bool st = i < n;
+        if (st && i > 0 && near_equal(S.key[i - 1], S.key[i])) {
+            const int cmp = exact_cmp_vals(S.val[i - 1], S.val[i], nT, cv, edges, P);
+            atomicAdd(&ct->exact_compares, 1ull);
+            if (cmp == EXACT_OVERFLOW) set_err(ct, GPUDT_ERR_EXACT, 110);
+            else if (cmp == 0) {
+                st = false;
+                atomicAdd(&ct->nties, 1);
+            } else if (cmp > 0) atomicAdd(&ct->al_slow, 1);
+        }
+        starts[r] = __ballot_sync(0xffffffffu, st);
+        before += __popc(starts[r]);
+    }
+    if (lane == 0) s_warp[w] = before;
+    __syncthreads();
+    int rank = 0, total = 0;
+    for (int q = 0; q < kBsWarps; q++) {
+        const int x = s_warp[q];
+        if (q < w) rank += x;
+        total += x;
+    }
+#pragma unroll
+    for (int r = 0; r < kBlockSort / kBsThreads; r++) {
+        if (r >= rounds) break;
+        const int i = base + r * 32 + lane;
+        if (i < n) {
+            const int k = rank + __popc(starts[r] & (0xffffffffu >> (31 - lane)));  // starts up to this entry
+            const int v = S.val[i];
+            if (v < nT) tri_ro[v] = k;
+            else edge_ro[v - nT] = k;
+            if ((starts[r] >> lane) & 1u) spectrum[k] = __longlong_as_double((long long)S.key[i]);
+        }
+        rank += __popc(starts[r]);
+    }
+    if (threadIdx.x == 0) {
+        spectrum[0] = 0.0;
+        ct->al_ranks = total;
+    }
+}
+
 // Spectrum, simplex ranks and intervals from the rank-start flags (c.aux).
-static int alpha_scatter(Ctx &c, AlphaSegs *segs, int nIn)
+static int alpha_scatter(Ctx &c, AlphaSegs *segs, int nIn, bool again = false)
 {
     const int nT = c.nT_out;
     const int *nr = c.aux;
@@ -1009,10 +1116,7 @@ static int alpha_scatter(Ctx &c, AlphaSegs *segs, int nIn)
                  nIn);
         launch_n(c, SetSentinels{segs->spec_off, c.spectrum}, segs->K);
     }
-    GALPHA_CUDA(cudaMemsetAsync(c.pt_nu, 0xff, sizeof(int2) * (size_t)c.N, c.stream));
-    launch_n(c, EdgeIntervals{c.cv, c.cn, c.e_off, c.tri_ro, c.edge_ro, c.edge_nu, c.pt_nu}, nT);
-    GALPHA_CUDA(cudaGetLastError());
-    return read_counters(c);
+    return alpha_intervals(c, again);
 }
 
 int stage_alpha(Ctx &c, AlphaSegs *segs)
@@ -1020,34 +1124,79 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
     int r;
     const int nT = c.nT_out;
     // an alpha call on a resident mesh starts without the error of an earlier
-    // failed alpha call (err and errinfo are adjacent words) and with its own
-    // counts
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->err, 0, 2 * sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->al_edges, 0, kAlphaBytes, c.stream));
-    const int tiles = (nT + kAkTile - 1) / kAkTile;
+    // failed alpha call and with its own counts
+    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->err, 0, kAlphaBytes, c.stream));
+    const bool few = nT <= kAkFew;
+    const int tile = kAkThreads * (few ? 1 : kAkItemsMany), tiles = (nT + tile - 1) / tile;
     if (nT > 0) {
-        // status words in the sort's scratch, which no sort uses yet
-        unsigned long long *status = (unsigned long long *)c.rhist;
-        GALPHA_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (size_t)(tiles + 1), c.stream));
-        k_alpha_keys<<<(unsigned)tiles, kAkThreads, 0, c.stream>>>(
-            AlphaKeysArgs{c.cv, c.cn, alpha_geom_tris(c), c.opos, nT, c.e_off, c.keys, c.vals, c.edges, c.edge_ro,
-                          c.list, status, tiles, c.ctr});
+        // status words in the counter block, or in the sort's scratch, which no sort uses yet
+        unsigned long long *status = c.ctr->al_status;
+        if (tiles + 1 > 64) {
+            status = (unsigned long long *)c.rhist;
+            GALPHA_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (size_t)(tiles + 1), c.stream));
+        }
+        const AlphaKeysArgs a{c.cv, c.cn, alpha_geom_tris(c), c.opos, nT, c.e_off, c.keys, c.vals, c.edges, c.edge_ro,
+                              c.list, status, tiles, c.pt_nu, c.N, c.ctr};
+        if (few) k_alpha_keys<1><<<(unsigned)tiles, kAkThreads, 0, c.stream>>>(a);
+        else k_alpha_keys<kAkItemsMany><<<(unsigned)tiles, kAkThreads, 0, c.stream>>>(a);
         count_launch();
+    } else if (c.N > 0) {
+        GALPHA_CUDA(cudaMemsetAsync(c.pt_nu, 0xff, sizeof(int2) * (size_t)c.N, c.stream));
     }
     // the sliver list's length stays on the device
     launch_dev(c, SliverKeys{alpha_geom_tris(c), c.opos, c.list, c.keys, c.ctr}, &c.ctr->al_sliver, nT);
-    r = read_counters(c);
+    auto sort_begins = [&]() {
+        c.sort_passes = 0;
+        if (c.events) {
+            cudaEventRecord(c.kev[8], c.stream);
+            c.kev_rec[8] = true;
+        }
+    };
+    auto sort_ends = [&]() {
+        if (c.events) {
+            cudaEventRecord(c.kev[9], c.stream);
+            c.kev_rec[9] = true;
+        }
+    };
+    auto rank_block = [&]() {
+        static bool set[64];
+        const int smem = (int)sizeof(BsSmem<unsigned long long>);
+        int e = block_sort_attr(c, k_alpha_rank_block, smem, set);
+        if (e) return e;
+        sort_begins();
+        c.sort_passes = 5;
+        k_alpha_rank_block<<<1, kBsThreads, smem, c.stream>>>(c.keys, c.vals, nT, alpha_geom_tris(c), c.edges, c.opos,
+                                                              c.tri_ro, c.edge_ro, c.spectrum, c.ctr);
+        count_launch();
+        sort_ends();
+        return alpha_intervals(c, false);
+    };
+    // a triangle owns at most three edges: this few cannot pass kBlockSort entries
+    const bool blind = !segs && 4ll * nT <= kBlockSort;
+    r = blind ? rank_block() : read_counters(c);
     if (r) return r;
     if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
     const int nE = c.hctr->al_edges;
     c.nE = nE;
     const int nIn = 1 + nT + c.hctr->al_unatt;
     c.nSpecIn = nIn;
-    c.sort_passes = 0;
-    if (c.events) {
-        cudaEventRecord(c.kev[8], c.stream);
-        c.kev_rec[8] = true;
+    if (!segs && nIn - 1 <= kBlockSort) {
+        if (!blind) r = rank_block();
+        if (r) return r;
+        c.st.sortKeys = nIn - 1;
+        if (c.hctr->fx_many) c.sort_passes += 8;
+        c.st.sortPasses = c.sort_passes;
+        if (!c.hctr->err && c.hctr->al_slow) {  // a run out of exact order: the ranks again
+            GALPHA_CUDA(cudaMemsetAsync(&c.ctr->fx_groups, 0, kRankBytes, c.stream));
+            r = alpha_ranks(c, segs, nIn, false);
+            if (!r) r = alpha_scatter(c, segs, nIn, true);
+            if (r) return r;
+        }
+        if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
+        c.nSpec = c.hctr->al_ranks + 1;
+        return GPUDT_OK;
     }
+    sort_begins();
     bool second = false;
     // entry 0 is the sentinel (no key of its own); a batch's entries are
     // regrouped after the sort, so a late look at its long groups is no option
@@ -1065,10 +1214,7 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
         c.vals2 = second ? v1 : v2;
     };
     take_sorted();
-    if (c.events) {
-        cudaEventRecord(c.kev[9], c.stream);
-        c.kev_rec[9] = true;
-    }
+    sort_ends();
     c.st.sortKeys = nIn - 1;
     c.st.sortPasses = c.sort_passes;
     if (segs) {
@@ -1102,7 +1248,7 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
         }
         GALPHA_CUDA(cudaMemsetAsync(&c.ctr->fx_groups, 0, kRankBytes, c.stream));
         r = alpha_ranks(c, segs, nIn, false);
-        if (!r) r = alpha_scatter(c, segs, nIn);
+        if (!r) r = alpha_scatter(c, segs, nIn, true);
         if (r) return r;
         if (c.hctr->err) return stage_fail(c, c.hctr->err, "alpha");
     }

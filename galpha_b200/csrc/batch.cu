@@ -514,7 +514,6 @@ int batch_setup(Ctx &c, BatchDev &B, BatchHost &bh, const double *d_xy)
     GALPHA_CUDA(cudaMemcpyAsync(B.sets, bh.sets.data(), sizeof(SetDesc) * (size_t)K, cudaMemcpyHostToDevice, c.stream));
     GALPHA_CUDA(cudaMemsetAsync(B.first, 0x7f, sizeof(int) * (size_t)K, c.stream));
     GALPHA_CUDA(cudaMemsetAsync(B.offline, 0, sizeof(int) * (size_t)K, c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.ctr, 0, sizeof(Counters), c.stream));
     launch_n(c, VertexSets{B.vbases, K, B.vset}, N);
     launch_n(c, BFirstDistinct{d_xy, B.vset, B.sets, B.first}, N);
     // atomicMin above starts from 0x7f7f7f7f; mark "none" as 0x7fffffff for the next kernel
@@ -540,18 +539,22 @@ int batch_setup(Ctx &c, BatchDev &B, BatchHost &bh, const double *d_xy)
     c.logT = 0;
     GALPHA_CUDA(cudaMemcpyAsync(B.fbases, fb.data(), sizeof(int) * (size_t)(K + 1), cudaMemcpyHostToDevice, c.stream));
     GALPHA_CUDA(cudaMemcpyAsync(B.sets, bh.sets.data(), sizeof(SetDesc) * (size_t)K, cudaMemcpyHostToDevice, c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.occ, 0, sizeof(uint32_t) * (size_t)bh.occw, c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.bandocc, 0, sizeof(uint32_t) * (size_t)bh.band, c.stream));
     // spatial numbering inside each set
     c.renumbered = N > 1;
     if (c.renumbered) {
         unsigned *k1 = (unsigned *)c.keys, *k2 = (unsigned *)c.keys2;
         launch_n(c, BSpatialKeys{d_xy, B.sets, B.vset, k1, c.perm}, N);
-        int r = radix_sort32(c, k1, c.perm, k2, c.vals2, N, c.rhist);
+        // codes of the largest cell's bits, then set numbers; no host look at
+        // which bits vary
+        int r = radix_sort32(c, k1, c.perm, k2, c.vals2, N, c.rhist, 2 * bh.classes.back().logT);
         if (r) return r;
-        launch_n(c, SetOfPerm{B.vset, c.perm, k1}, N);
-        r = radix_sort32(c, k1, c.perm, k2, c.vals2, N, c.rhist);
-        if (r) return r;
+        int bits = 1;
+        while ((1ll << bits) < K) bits++;
+        if (K > 1) {
+            launch_n(c, SetOfPerm{B.vset, c.perm, k1}, N);
+            r = radix_sort32(c, k1, c.perm, k2, c.vals2, N, c.rhist, bits);
+            if (r) return r;
+        }
     }
     BSetupSites st;
     st.xy = d_xy;
@@ -589,7 +592,6 @@ int batch_setup(Ctx &c, BatchDev &B, BatchHost &bh, const double *d_xy)
 // whose island repair cannot stay local.
 int batch_voronoi(Ctx &c, BatchDev &B, BatchHost &bh)
 {
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->ntris, 0, 2 * sizeof(int), c.stream));  // ntris, nfree
     int *const colour0 = c.colour;
     int16_t *const ycol0 = c.ycol;
     int *const idmap0 = c.idmap;

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include "internal.cuh"
 #include "exact.cuh"
+#include "snap.cuh"
 
 namespace galpha {
 
@@ -66,25 +67,6 @@ struct RingPix {
     }
 };
 
-// Pixel of input point v inside the margin (the snap SetupSites makes).
-__device__ __forceinline__ void snap_pixel(double x, double y, double sx, double sy, double scale, int D, int *ix,
-                                           int *iy)
-{
-    const double gx = floor((x - sx) / scale), gy = floor((y - sy) / scale);
-    *ix = (int)fmin(fmax(gx, 0.0), (double)(D - 1));
-    *iy = (int)fmin(fmax(gy, 0.0), (double)(D - 1));
-}
-
-__device__ __forceinline__ unsigned spread_bits14(unsigned v)
-{
-    v &= 0x3fffu;
-    v = (v | (v << 8)) & 0x00ff00ffu;
-    v = (v | (v << 4)) & 0x0f0f0f0fu;
-    v = (v | (v << 2)) & 0x33333333u;
-    v = (v | (v << 1)) & 0x55555555u;
-    return v;
-}
-
 // Morton code of each input point's pixel, with its input index as payload.
 // Sorted stably, it numbers the vertices so that neighbours in the plane
 // have nearby ids (their positions, states and incidence share cache lines),
@@ -94,20 +76,23 @@ struct SpatialKeys {
     const double *xy;
     unsigned *keys;
     int *vals;
-    double scale, sx, sy;
-    int D;
+    SnapGrid g;
     __device__ void operator()(long long i) const
     {
-        int ix, iy;
-        snap_pixel(xy[2 * i], xy[2 * i + 1], sx, sy, scale, D, &ix, &iy);
-        keys[i] = spread_bits14((unsigned)ix) | (spread_bits14((unsigned)iy) << 1);
+        keys[i] = pixel_key(xy[2 * i], xy[2 * i + 1], g);
         vals[i] = (int)i;
     }
 };
 
+// Sites come in the order of their pixels' codes, those of one pixel in input
+// order, so a pixel's owner is the first of a run of equal codes: it alone
+// writes the id map and the occupancy, and the others find it by binary search
+// (writes by every site, and two more launches to settle the lowest and to mark
+// the rest, took 0.2 and 0.1 ms at 4.2 M points).
 struct SetupSites {
     const double *xy;
-    const int *perm;  // internal vertex -> input index (nullptr: identity)
+    const int *perm;  // internal vertex -> input index
+    const unsigned *code;  // [N] sorted pixel codes
     double2 *opos, *pos;
     short2 *gpix;
     int *idmap;
@@ -122,9 +107,9 @@ struct SetupSites {
     {
         int v = (int)i;
         double2 o, p;
-        int px, py;
+        int px, py, owner = v;
         if (v < N) {
-            const int src = perm ? perm[v] : v;
+            const int src = perm[v];
             o = make_double2(xy[2 * src], xy[2 * src + 1]);
             if (!(o.x >= minX && o.x <= maxX && o.y >= minY && o.y <= maxY)) set_err(ct, GPUDT_ERR_ARG, src);
             int D = T - 2 * kMargin;
@@ -133,7 +118,25 @@ struct SetupSites {
             p = make_double2(sx + ix * scale, sy + iy * scale);
             px = ix + kMargin;
             py = iy + kMargin;
-            vstate[v] = VS_UNDECIDED;
+            const unsigned k = code[v];
+            if (v > 0 && code[v - 1] == k) {  // in the pixel of an earlier site
+                int lo = 0, hi = v - 1;       // the run starts in [lo, hi]
+                for (int step = 1; lo < hi; step *= 2) {
+                    const int j = max(lo, hi - step);
+                    if (code[j] != k) {
+                        lo = j + 1;
+                        break;
+                    }
+                    hi = j;
+                }
+                while (lo < hi) {
+                    const int j = (lo + hi) >> 1;
+                    if (code[j] == k) hi = j;
+                    else lo = j + 1;
+                }
+                owner = lo;
+            }
+            vstate[v] = owner == v ? VS_UNDECIDED : VS_MISSING;
         } else {
             short2 q = ring(v - N);
             px = q.x;
@@ -147,42 +150,12 @@ struct SetupSites {
         gpix[v] = make_short2((short)px, (short)py);
         vtri[v] = -1;
         vround[v] = v < N ? 0 : 1;  // fake ring sites never move: decided before the first priority round (id 2)
-        anchor[v] = -1;
+        anchor[v] = owner == v ? -1 : owner;
+        if (owner != v) return;
         size_t pix = ((size_t)py << logT) + px;
         idmap[pix] = v;
         atomicOr(&occ[(size_t)px * (T >> 5) + (py >> 5)], 1u << (py & 31));
         atomicOr(&bandocc[(size_t)px * W2 + (py >> 11)], 1u << ((py >> 6) & 31));
-    }
-};
-
-struct MinId {
-    const short2 *gpix;
-    int *idmap;
-    int logT;
-    __device__ void operator()(long long i) const
-    {
-        int v = (int)i;
-        short2 g = gpix[v];
-        int *slot = &idmap[((size_t)g.y << logT) + g.x];
-        if (*slot > v) atomicMin(slot, v);
-    }
-};
-
-struct ClassifySites {
-    const short2 *gpix;
-    const int *idmap;
-    int8_t *vstate;
-    int *anchor;
-    int logT;
-    __device__ void operator()(long long i) const
-    {
-        int v = (int)i;
-        short2 g = gpix[v];
-        int w = idmap[((size_t)g.y << logT) + g.x];
-        if (w != v) {
-            vstate[v] = VS_MISSING;
-            anchor[v] = w;
-        }
     }
 };
 
@@ -316,7 +289,7 @@ constexpr int kPrecheckPrefix = 1024;
 
 // The first kPrecheckPrefix points in one block, with no shared-address
 // traffic: the smallest index of a point distinct from point 0 into *first
-// (left alone when there is none) and ct->changed = 1 when one of them is
+// (0x7fffffff when there is none) and ct->changed = 1 when one of them is
 // off the line through point 0 and that point. This decides general input;
 // the grid-wide scans below then return at once.
 __global__ void __launch_bounds__(kPrecheckPrefix) k_precheck_prefix(const double *xy, int n, int *first, Counters *ct)
@@ -340,8 +313,8 @@ __global__ void __launch_bounds__(kPrecheckPrefix) k_precheck_prefix(const doubl
     }
     __syncthreads();
     const int j = jsh;
-    if (j == 0x7fffffff) return;  // the prefix is all point 0: the grid scans decide
-    if (i == 0) *first = j;
+    if (i == 0) *first = j;  // above every index when the prefix is all point 0: the grid scans decide
+    if (j == 0x7fffffff) return;
     int s = 0;
     if (in) {
         const double xj = xy[2 * j], yj = xy[2 * j + 1];
@@ -379,15 +352,18 @@ __global__ void __launch_bounds__(256) k_count_off_line(const double *xy, const 
     }
 }
 
-// Returns 1 when the input has at least one triangle.
-int has_triangles(Ctx &c, const double *d_xy, int n)
+void precheck(Ctx &c, const double *d_xy, int n)
 {
-    if (n < 3) return 0;
-    int *first = c.aux;
-    GALPHA_CUDA(cudaMemsetAsync(first, 0x7f, sizeof(int), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(&c.ctr->changed, 0, sizeof(int), c.stream));
-    k_precheck_prefix<<<1, kPrecheckPrefix, 0, c.stream>>>(d_xy, n, first, c.ctr);
+    k_precheck_prefix<<<1, kPrecheckPrefix, 0, c.stream>>>(d_xy, n, &c.ctr->pre_first, c.ctr);
     count_launch();
+}
+
+// The prefix did not decide (counters read): 1 when the input has at least one
+// triangle, found by scans of all points.
+static int has_triangles(Ctx &c, const double *d_xy, int n)
+{
+    if (n <= kPrecheckPrefix) return 0;
+    int *first = &c.ctr->pre_first;
     long long blocks = ((long long)n + 255) / 256;
     if (blocks > (long long)c.sm_count * 8) blocks = (long long)c.sm_count * 8;
     k_first_distinct<<<(unsigned)blocks, 256, 0, c.stream>>>(d_xy, n, first);
@@ -453,21 +429,28 @@ int stage_setup(Ctx &c, const double *d_xy, int n, double minX, double minY, dou
     c.V = c.N + c.F;
     grid_scaling(minX, minY, maxX, maxY, T, c.scale, c.shiftX, c.shiftY);
     int W2 = ((T >> 6) + 31) / 32;
-    GALPHA_CUDA(cudaMemsetAsync(c.occ, 0, sizeof(uint32_t) * (size_t)T * (T >> 5), c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.bandocc, 0, sizeof(uint32_t) * (size_t)T * W2, c.stream));
-    GALPHA_CUDA(cudaMemsetAsync(c.ctr, 0, sizeof(Counters), c.stream));
-    // spatial numbering of the input points (stable radix sort of pixel Morton codes)
-    c.renumbered = n > 1;
-    if (c.renumbered) {
-        unsigned *k1 = (unsigned *)c.keys, *k2 = (unsigned *)c.keys2;
-        launch_n(c, SpatialKeys{d_xy, k1, c.perm, c.scale, c.shiftX, c.shiftY, T - 2 * kMargin}, n);
-        // pixel coordinates below T: Morton codes of 2 logT bits
-        int r = radix_sort32(c, k1, c.perm, k2, c.vals2, n, c.rhist, 2 * c.logT);
-        if (r) return r;
+    // spatial numbering of the input points (stable radix sort of pixel Morton
+    // codes: pixel coordinates below T, 2 logT bits)
+    c.renumbered = true;
+    const SnapGrid g{c.scale, c.shiftX, c.shiftY, T - 2 * kMargin};
+    unsigned *code = (unsigned *)c.keys;
+    int r;
+    if (n <= kBlockSort) {
+        r = spatial_sort_block(c, d_xy, n, g, 2 * c.logT, code, c.perm);
+    } else {
+        // the last digit's pass leaves its result in (code, perm)
+        unsigned *k2 = (unsigned *)c.keys2;
+        const bool odd = sort32_digits(2 * c.logT) & 1;
+        unsigned *ka = odd ? k2 : code, *kb = odd ? code : k2;
+        int *va = odd ? c.vals2 : c.perm, *vb = odd ? c.perm : c.vals2;
+        launch_n(c, SpatialKeys{d_xy, ka, va, g}, n);
+        r = radix_sort32_inplace(c, ka, va, kb, vb, n, c.rhist, 2 * c.logT);
     }
+    if (r) return r;
     SetupSites s;
     s.xy = d_xy;
-    s.perm = c.renumbered ? c.perm : nullptr;
+    s.perm = c.perm;
+    s.code = code;
     s.opos = c.opos;
     s.pos = c.pos;
     s.gpix = c.gpix;
@@ -493,13 +476,11 @@ int stage_setup(Ctx &c, const double *d_xy, int n, double minX, double minY, dou
     s.ring = RingPix{T, nside};
     s.ct = c.ctr;
     launch_n(c, s, c.V);
-    launch_n(c, MinId{c.gpix, c.idmap, c.logT}, c.N);
-    launch_n(c, ClassifySites{c.gpix, c.idmap, c.vstate, c.anchor, c.logT}, c.N);
     GALPHA_CUDA(cudaGetLastError());
     return GPUDT_OK;
 }
 
-int stage_voronoi(Ctx &c)
+int stage_voronoi(Ctx &c, const double *d_xy, bool *empty)
 {
     const int T = c.T;
     int W2 = ((T >> 6) + 31) / 32;
@@ -510,12 +491,21 @@ int stage_voronoi(Ctx &c)
     // make the per-pixel window scan long, so they take the envelope path.
     c.fused_done = false;
     long long D = T - 2 * kMargin;
-    int occupied = 0;
-    r0 = cell_occupancy(c, c.bandocc, T, W2, 1, c.aux, &occupied);
+    const int nb = T / 64;
+    launch_n(c, CellOccupancy{c.bandocc, T, W2, nb, &c.ctr->occ_blocks}, (long long)(nb - 2) * (nb - 2));
+    r0 = read_counters(c);
     if (r0) return r0;
+    const int occupied = c.hctr->occ_blocks;
+    if (!c.hctr->changed) {  // no triangle among the first points
+        r0 = has_triangles(c, d_xy, c.N);
+        if (r0 < 0) return r0;
+        if (r0 == 0) {
+            *empty = true;
+            return GPUDT_OK;
+        }
+    }
+    if (c.hctr->err) return c.hctr->err;
     if ((long long)c.N * 256 >= D * D && occupancy_ok(T, occupied)) {
-        GALPHA_CUDA(cudaMemsetAsync(&c.ctr->ntris, 0, sizeof(int), c.stream));
-        GALPHA_CUDA(cudaMemsetAsync(&c.ctr->nisland, 0, sizeof(int), c.stream));
         r0 = launch_vd_tri(c);
         if (r0) return r0;
         r0 = read_counters(c);

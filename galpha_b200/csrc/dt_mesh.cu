@@ -209,9 +209,8 @@ int stage_links(Ctx &c)
 {
     int r;
     int nt = c.hctr->ntris;  // as the emission left it
-    int *deg = c.deg;       // [V+1]
+    int *deg = c.deg;       // [V+1], cleared when the call started
     int *start = c.aux2;    // [V+1]
-    GALPHA_CUDA(cudaMemsetAsync(deg, 0, sizeof(int) * (size_t)(c.V + 1), c.stream));
     launch_n(c, CountDeg{c.tv, deg}, nt);
     r = exclusive_scan_int(c, deg, start, c.V + 1, nullptr);
     if (r) return r;

@@ -66,17 +66,18 @@ struct Counters {
     int nlist;      // generic work-list length
     int nlist2;     // second work list
     int changed;    // generic progress flag / count
-    int err;        // first error code (GPUDT_ERR_*), 0 if none
-    int errinfo;    // stage-specific detail of the first error
     int nisland;    // island pixels
     int flips_total;
     int escalate;   // island repair could not stay local: redo the Voronoi stage globally
-    // alpha stage, cleared together when it starts (kAlphaWords from al_edges on)
+    int err;        // first error code (GPUDT_ERR_*), 0 if none
+    int errinfo;    // stage-specific detail of the first error
+    // alpha stage, cleared together with the error when it starts (kAlphaBytes from err on)
+    unsigned long long al_status[64];  // look-back words and ticket of few tiles
     int al_edges;    // edges numbered
     int al_unatt;    // of them, unattached: in the spectrum
     int al_sliver;   // triangles whose radius needs exact arithmetic
     int al_ranks;    // distinct values
-    // the rest again when the ranks are redone (kRankWords from fx_groups on)
+    // the rest again when the ranks are redone (kRankBytes from fx_groups on)
     int fx_groups;   // key sort: short groups out of order
     int fx_long;     // key sort: out-of-order pairs recorded in groups too long for one thread
     int fx_many;     // key sort: more of those than can be recorded
@@ -94,6 +95,8 @@ struct Counters {
     int tail_rounds; // flip: rounds run by the last in-block tail launch
     int nlong;       // alpha ranks: runs too long for one thread; master list: long runs
     int nhuge;       // alpha ranks: runs too long for one block, listed for the multi-block merge
+    int pre_first;   // precheck: smallest index of a point distinct from point 0
+    int occ_blocks;  // occupied interior 64 x 64 blocks of a single texture
     int sh_total;    // shift: all dropped sites listed so far
     int nbad;        // shift: sites that cannot be shifted
     int nhull;       // links: hull edges
@@ -137,7 +140,7 @@ struct Relink {
     int old;
 };
 
-constexpr size_t kAlphaBytes = offsetof(Counters, exact_orient) - offsetof(Counters, al_edges);
+constexpr size_t kAlphaBytes = offsetof(Counters, exact_orient) - offsetof(Counters, err);
 constexpr size_t kRankBytes = offsetof(Counters, exact_orient) - offsetof(Counters, fx_groups);
 
 // A grown-on-demand device buffer.
@@ -484,9 +487,11 @@ GALPHA_HD void seti(int4 &v, int i, int x)
 }
 
 // Stage entry points (dt_grid.cu, dt_mesh.cu, alpha.cu)
-int has_triangles(Ctx &c, const double *d_xy, int n);
+// Starts the check whether the input has a triangle; stage_voronoi reads it
+// and sets *empty when there is none.
+void precheck(Ctx &c, const double *d_xy, int n);
 int stage_setup(Ctx &c, const double *d_xy, int n, double minX, double minY, double maxX, double maxY, int T);
-int stage_voronoi(Ctx &c);
+int stage_voronoi(Ctx &c, const double *d_xy, bool *empty);
 int stage_triangles(Ctx &c);
 int stage_links(Ctx &c);
 int stage_shift(Ctx &c);
@@ -601,6 +606,19 @@ int radix_sort_finish(Ctx &c, unsigned long long *keys, int *vals, unsigned long
                       bool *in_second, bool fresh);
 int radix_sort32(Ctx &c, unsigned int *keys, int *vals, unsigned int *keys2, int *vals2, int n, int *scratch,
                  int key_bits = 0);
+// The same for keys of key_bits bits, leaving the result in (keys2, vals2)
+// after an odd number of digits (sort32_digits), in (keys, vals) after an even
+// one, with no copy.
+int radix_sort32_inplace(Ctx &c, unsigned int *keys, int *vals, unsigned int *keys2, int *vals2, int n, int *scratch,
+                         int key_bits);
+inline int sort32_digits(int key_bits) { return (key_bits + 7) / 8; }
+// Snap of a point to its pixel (dt_grid.cu) for the sorts that make their own keys.
+struct SnapGrid {
+    double scale, sx, sy;
+    int D;
+};
+constexpr int kBlockSort = 8192;  // entries that one block sorts in one launch
+int spatial_sort_block(Ctx &c, const double *xy, int n, const SnapGrid &g, int key_bits, unsigned *keys, int *perm);
 // Stable sort by the low nbits of 32-bit set ids, moving (keys, vals) along;
 // the result ends in (skey, keys, vals).
 int radix_sort_set_kv(Ctx &c, unsigned *skey, unsigned *skey2, unsigned long long *keys, int *vals,

@@ -25,7 +25,7 @@ namespace galpha {
 constexpr int kSmThreads = 512;   // per block: 128 registers per thread
 constexpr int kSmMaxBlocks = 16;  // largest cluster
 constexpr int kSmFrWarps = 8;     // warps per block that remove fakes (shared memory)
-constexpr int kSmPerBlock = 512;  // vertices per block
+constexpr int kSmPerBlock = 256;  // vertices per block
 
 struct SmallMesh {
     // arrays of Ctx

@@ -15,6 +15,8 @@
 #include <mutex>
 #include <vector>
 #include "internal.cuh"
+#include "snap.cuh"
+#include "block_sort.cuh"
 
 namespace galpha {
 
@@ -781,6 +783,41 @@ int radix_sort_finish(Ctx &c, unsigned long long *keys, int *vals, unsigned long
             launch_n(c, CopyElems<int>{rv + g.x, fv}, len);
         }
     }
+    GALPHA_CUDA(cudaGetLastError());
+    return GPUDT_OK;
+}
+
+int radix_sort32_inplace(Ctx &c, unsigned int *keys, int *vals, unsigned int *keys2, int *vals2, int n, int *scratch,
+                         int key_bits)
+{
+    bool sec = false;
+    return radix_sort_keys<unsigned int>(c, keys, vals, keys2, vals2, n, scratch, 0, &sec, key_bits);
+}
+
+// Points in the order of their pixels' codes: (sorted code, input index).
+__global__ void __launch_bounds__(kBsThreads) k_spatial_sort(const double *__restrict__ xy, int n, SnapGrid g,
+                                                             int passes, unsigned *keys, int *perm)
+{
+    extern __shared__ __align__(16) unsigned char bs_smem[];
+    block_sort(*reinterpret_cast<BsSmem<unsigned> *>(bs_smem), n, 0, passes,
+               [&](int i, unsigned &k, int &v) {
+                   k = pixel_key(xy[2 * i], xy[2 * i + 1], g);
+                   v = i;
+               },
+               [&](int i, unsigned k, int v) {
+                   keys[i] = k;
+                   perm[i] = v;
+               });
+}
+
+int spatial_sort_block(Ctx &c, const double *xy, int n, const SnapGrid &g, int key_bits, unsigned *keys, int *perm)
+{
+    static bool set[64];
+    const int smem = (int)sizeof(BsSmem<unsigned>);
+    int r = block_sort_attr(c, k_spatial_sort, smem, set);
+    if (r) return r;
+    k_spatial_sort<<<1, kBsThreads, smem, c.stream>>>(xy, n, g, sort32_digits(key_bits), keys, perm);
+    count_launch();
     GALPHA_CUDA(cudaGetLastError());
     return GPUDT_OK;
 }

@@ -77,3 +77,53 @@ def test_handles_in_parallel():
     for t in th:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("n,fbo", [(8191, 512), (8192, 512), (8193, 512), (8193, 4096), (3000, 16384)])
+def test_spatial_sort_sizes(engine, n, fbo):
+    """One block sorts up to 8,192 points, digit passes more; odd and even
+    numbers of digits."""
+    pts = D.uniform_points(n, 3)
+    pts[1::3] = pts[::3][:len(pts[1::3])] + 1e-9  # pixels with several sites
+    _check(engine, pts, fbo)
+
+
+@pytest.mark.parametrize("n", [1030, 1034, 1038, 2092, 2098, 2102, 2106, 2112])
+def test_ranks_in_one_block(engine, n):
+    """Spectrum lengths on both sides of what one block sorts, and of what it
+    sorts without a look at the length."""
+    from alphacheck import compare_alpha
+
+    pts = D.uniform_points(n, 5)
+    dt = engine.triangulate(G.GPUDTParams(pts, fboSize=512))
+    ok, rep = compare_alpha(pts, dt.vtx, dt.tri, engine.alpha_resident(), 4)
+    assert ok, rep
+
+
+def test_ties_in_one_block(engine):
+    """A lattice (exact ties) with a few points moved by far less than an ulp of
+    the radii (near ties whose keys may be out of exact order)."""
+    from alphacheck import compare_alpha
+
+    g = np.stack(np.meshgrid(np.arange(20.0), np.arange(20.0)), axis=-1).reshape(-1, 2) / 3.0
+    g[21::37] *= 1.0 + 2.0 ** -51
+    dt = engine.triangulate(G.GPUDTParams(g, fboSize=256))
+    ok, rep = compare_alpha(g, dt.vtx, dt.tri, engine.alpha_resident(), 4)
+    assert ok, rep
+
+
+@pytest.mark.parametrize("n", [3, 700, 1024, 1025, 3000])
+def test_degenerate_inputs(engine, n):
+    """Copies of one point, and collinear points, with the deciding point first,
+    in the first 1,024 or after them: an empty mesh, or a triangulation."""
+    for pts in (np.ones((n, 2)), np.stack([np.arange(n) * 0.5, np.arange(n) * 0.25], axis=1)):
+        assert engine.triangulate(G.GPUDTParams(pts, fboSize=256)).nTris == 0
+        assert len(engine.alpha_resident()["spectrum"]) == 1
+        last = pts.copy()
+        last[-1] += [0.3, 0.9]
+        dt = engine.triangulate(G.GPUDTParams(last, fboSize=256))
+        if len(np.unique(last, axis=0)) < 3:
+            assert dt.nTris == 0
+        else:
+            ok, rep = compare_dt(last, dt.vtx, dt.tri)
+            assert ok, rep
