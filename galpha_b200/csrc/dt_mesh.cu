@@ -1079,20 +1079,17 @@ int stage_missing(Ctx &c)
 // ---------------------------------------------------------------- boundary
 // Fan of a hull vertex f: from the clockwise-most triangle (whose edge f->u0 is
 // a hull edge) counterclockwise to the triangle whose edge ud->f is a hull edge.
-// Fake ring sites are removed class by class (ring index mod 4 in the order
-// 0, 2, 1, 3): sites of one class are separated along the border by sites of
-// other classes that are still present, so they are not adjacent and their
-// fans are disjoint; the priority test below only matters in the rare case of
-// an edge cutting a texture corner.
+// Fake ring sites are removed in runs (below); what a pass of runs leaves is
+// removed by further ones, and by priority among neighbours when a pass of runs
+// finds none it can take.
 constexpr int kMaxChain = 256;
 
-// Selection of fake sites to remove together: a fake whose fan (walked once
-// each way from vtri) holds no competing fake of lower priority -- in the
-// first pass only fakes of its ring class (ring position modulo 4) compete,
-// later every remaining fake does.  The selected fake's fan is stored (slot
-// and index of f, packed, and the outer neighbour across the chain edge) so
-// that the removal reads it with independent loads instead of walking again;
-// fans of selected fakes are disjoint, so they stay valid until the removal.
+// Selection of fake sites to remove together, one by one: a fake whose fan
+// (walked once each way from vtri) holds no fake of lower priority.  The
+// selected fake's fan is stored (slot and index of f, packed, and the outer
+// neighbour across the chain edge) so that the removal reads it with
+// independent loads instead of walking again; fans of selected fakes are
+// disjoint, so they stay valid until the removal.
 constexpr int kMaxFanLong = 4096;  // longest fan a fake may have (error beyond)
 
 struct FakeSelect {
@@ -1102,11 +1099,11 @@ struct FakeSelect {
     int *list, *fanoff, *fanlen;
     int2 *fan;
     int *count, *fan_n;
-    int N, cls;  // cls < 0: every remaining fake competes by priority
+    int N;
     Counters *ct;
     __device__ bool conflicts(int g, uint32_t pf) const
     {
-        return g >= N && vstate[g] == VS_FAKE && (cls < 0 || ((g - N) & 3) == cls) && prio((uint32_t)g) < pf;
+        return g >= N && vstate[g] == VS_FAKE && prio((uint32_t)g) < pf;
     }
     __device__ void operator()(long long ii) const
     {
@@ -1114,7 +1111,7 @@ struct FakeSelect {
         constexpr int M = kMaxChain;
         int2 E[2 * M];  // (packed f-corner, outer neighbour) per fan triangle, fans of up to M
         int lo = M, hi = M, nccw = 0, ncw = 0, ecw = -1;
-        bool pick = (cls < 0 || ((int)ii & 3) == cls) && vstate[f] == VS_FAKE;
+        bool pick = vstate[f] == VS_FAKE;
         if (pick) {
             const uint32_t pf = prio((uint32_t)f);
             const int e0 = vtri[f];
@@ -1185,42 +1182,48 @@ struct FakeSelect {
     }
 };
 
-// Runs of fake sites removed as one unit.  Removing one ring class after
-// another leaves the last class as a chain: collinear fakes on a side of the
-// texture become hull neighbours through the chords their removed neighbours
-// leave, so every fake of the last class touches the next one and the
-// priority rounds take out only about a third of the chain per round.  A run
-// -- selected fakes that follow each other along the hull -- has as outer
-// boundary the concatenation of its members' fan chains without the one
-// triangle each consecutive pair shares; the stack rule patches that chain
-// exactly as it patches one fake's.  Selection by separator levels over the
-// class's chain (j = ring position / 4): level l takes the fakes with j a
-// multiple of 16^l but not of 16^(l+1), so the kept multiples separate the
-// runs of one level (level 0: runs of 15 between every 16th fake).  The
-// leader (the member whose clockwise hull neighbour is not selected) stores
-// the kept fan entries followed by the shared triangles (outer link -1);
-// fanlen holds kept | shared << 16.  A run whose fans touch a selected fake
-// of another run, or that closes on itself, is left to the priority rounds.
+// Runs of fake sites removed as one unit.  Fakes that follow each other along
+// the hull (ring neighbours at first, later those whose removed neighbours left
+// a chord between them) have as outer boundary the concatenation of their fans'
+// chains without the one triangle each consecutive pair shares; the stack rule
+// patches that chain exactly as it patches one fake's: a chain vertex sees its
+// own fake, and the fakes see their chains in the same order.
+// Selection by separator levels over the ring (j = ring position): level l
+// takes the fakes with j a multiple of 16^l but not of 16^(l+1), so the kept
+// multiples separate the runs of one level (level 0: runs of 15 between every
+// 16th fake); level -1 takes every fake that is left.  Of two selected fakes
+// that see each other across a chain (one strictly inside the other's, over an
+// empty corner, say) the one of higher priority value is left out; it ends the
+// run on either side and waits for a later pass.  The leader (the member whose
+// clockwise hull neighbour is no member) stores the kept fan entries followed
+// by the shared triangles (outer link -1); fanlen holds kept | shared << 16.
+// A run that closes on itself (fakes all along the hull) is taken without its
+// member of lowest id.
+// Before, three of four ring classes were removed fake by fake, the last class
+// as runs that one such pair left out whole, and the rest by priority, about a
+// third of it per pass: 12 passes of 35 us at 12,000 points in a disk (390 us of
+// boundary stage, now 225), 20 at 262,145 clustered points (593 us, now 350).
 constexpr int kMaxRunMembers = 64;
 
-// Separator-level selection of the fakes of one ring class (see above).
-__device__ __forceinline__ bool run_selected(const int8_t *vstate, int N, int cls, int level, int g)
+// Separator-level selection (see above).
+__device__ __forceinline__ bool run_selected(const int8_t *vstate, int N, int level, int g)
 {
-    if (g < N || vstate[g] != VS_FAKE || ((g - N) & 3) != cls) return false;
-    const int j = (g - N) >> 2, sh = 4 * level;
+    if (g < N || vstate[g] != VS_FAKE) return false;
+    if (level < 0) return true;
+    const int j = g - N, sh = 4 * level;
     return (j & ((1 << sh) - 1)) == 0 && ((j >> sh) & 15) != 0;
 }
 
 // Per selected fake, its own fan: the entries (clockwise end first) in the
 // staging array, and a record {offset, length, clockwise end vertex U[0],
-// counterclockwise end vertex U[d], valid}.  A fan holding a selected fake
-// strictly inside its chain is not valid (it touches another run).  Each
-// thread walks one fan, so the latency is that of one fan, not of a run.
+// counterclockwise end vertex U[d], valid}.  A fan holding a selected fake of
+// lower priority strictly inside its chain is not valid.  Each thread walks one
+// fan, so the latency is that of one fan, not of a run.
 struct FakeRunStage {
     const int4 *tv, *tn;
     const int8_t *vstate;
     const int *vtri;
-    int N, cls, level;
+    int N, level;
     int2 *stage;
     int *stage_n;
     int *rec;  // 5 ints per ring position
@@ -1228,44 +1231,53 @@ struct FakeRunStage {
     __device__ void operator()(long long ii) const
     {
         const int f = N + (int)ii;
-        const bool sel = run_selected(vstate, N, cls, level, f);
-        int ecw = -1, d = 0, a0 = -1, bend = -1;
+        const bool sel = run_selected(vstate, N, level, f);
+        const uint32_t pf = prio((uint32_t)f);
+        auto yields = [&](int g) { return run_selected(vstate, N, level, g) && prio((uint32_t)g) < pf; };
+        constexpr int M = kMaxChain;
+        int2 E[2 * M];  // fan entries around the first one walked to
+        int lo = M, hi = M, nccw = 0, ncw = 0, a0 = -1, bend = -1, ecw = -1;
         bool ok = sel;
         if (ok) {
             const int e0 = vtri[f];
             int e = e0;
-            for (int g = 0;; g++) {  // clockwise to the hull edge (f, U[0])
-                const int nx = geti(tn[dtri(e)], m1(dori(e)));
+            for (;;) {  // counterclockwise from e0 to the hull edge (U[d], f)
+                const int t = dtri(e), i = dori(e);
+                const int4 w = tv[t], n = tn[t];
+                if (nccw == 0) a0 = geti(w, p1(i));
+                bend = geti(w, m1(i));
+                if (hi < 2 * M) E[hi++] = make_int2(e, geti(n, i));
+                nccw++;
+                const int nx = geti(n, p1(i));
                 if (nx < 0) break;
-                e = enc(dtri(nx), m1(dori(nx)));
-                if (e == e0 || g > kMaxFanLong) {
-                    e = -1;
-                    break;
-                }
-            }
-            ecw = e;
-            ok = ecw >= 0;
-        }
-        if (ok) {
-            int ee = ecw;
-            for (;;) {  // counterclockwise: count, ends, foreign selected fakes
-                const int t = dtri(ee), i = dori(ee);
-                const int4 w = tv[t];
-                if (d == 0) a0 = geti(w, p1(i));
-                const int bv = geti(w, m1(i));
-                bend = bv;
-                d++;
-                const int nx = geti(tn[t], p1(i));
-                if (nx < 0) break;
-                if (run_selected(vstate, N, cls, level, bv) || d > kMaxFanLong) {  // U[k] inside the chain
+                e = enc(dtri(nx), p1(dori(nx)));
+                if (e == e0 || nccw > kMaxFanLong || yields(bend)) {  // bend is inside the chain
                     ok = false;
                     break;
                 }
-                ee = enc(dtri(nx), p1(dori(nx)));
+            }
+            e = ecw = e0;
+            while (ok) {  // clockwise from e0 to the hull edge (f, U[0])
+                const int nx = geti(tn[dtri(e)], m1(dori(e)));
+                if (nx < 0) break;
+                if (yields(a0)) {  // a0 is inside the chain
+                    ok = false;
+                    break;
+                }
+                e = enc(dtri(nx), m1(dori(nx)));
+                const int t = dtri(e), i = dori(e);
+                a0 = geti(tv[t], p1(i));
+                if (lo > 0) E[--lo] = make_int2(e, geti(tn[t], i));
+                ncw++;
+                ecw = e;
+                if (nccw + ncw > kMaxFanLong) ok = false;
             }
         }
+        const int d = nccw + ncw;
         const int off = warp_reserve(stage_n, ok ? d : 0);
-        if (ok) {
+        if (ok && nccw <= M && ncw <= M) {
+            for (int k = 0; k < d; k++) stage[off + k] = E[lo + k];
+        } else if (ok) {  // a long fan: walked again from its clockwise end, into the store
             int ee = ecw;
             for (int k = 0; k < d; k++) {
                 const int t = dtri(ee), i = dori(ee);
@@ -1287,30 +1299,42 @@ struct FakeRunStage {
     }
 };
 
-// Per run leader (a selected fake whose clockwise hull neighbour is not
-// selected): follows the members through their records, checks that each
+// Per run leader: follows the members through their records, checks that each
 // next member's clockwise end is the current one, and copies the kept
 // entries followed by the shared triangles (outer link -1) into the fan
 // store; fanlen = kept | shared << 16.
 struct FakeRunJoin {
     const int8_t *vstate;
-    int N, cls, level;
+    int N, level;
     const int2 *stage;
     const int *rec;
     int *list, *fanoff, *fanlen;
     int2 *fan;
     int *count, *fan_n;
     Counters *ct;
-    // members and counts of the run led by ring position ii; 0 if invalid
-    __device__ int scan(int ii, int *kept, int *nsh) const
+    __device__ bool valid(int g) const
     {
-        const int f = N + ii;
+        return run_selected(vstate, N, level, g) && rec[5 * (g - N) + 4];
+    }
+    // a fake between two hull neighbours that share its one triangle: it goes
+    // first, alone, since it cuts the pair's common triangle off
+    __device__ bool ear(int g) const { return valid(g) && rec[5 * (g - N) + 1] == 1; }
+    __device__ bool member(int g) const
+    {
+        if (!valid(g)) return false;
+        const int *r = rec + 5 * (g - N);
+        if (r[1] > 1) return !ear(r[2]) && !ear(r[3]);
+        return (!ear(r[2]) || g < r[2]) && (!ear(r[3]) || g < r[3]);
+    }
+    // Members and counts of the run from ring position ii on, which ends before
+    // a fake that is no member, or before the fake `last`; 0 if it is not one.
+    __device__ int scan(int ii, int last, int *kept, int *nsh) const
+    {
         int m = ii, nk = 0, ns = 0;
         for (int mi = 0; mi < kMaxRunMembers; mi++) {
             const int *r = rec + 5 * m;
-            if (!r[4] || (mi > 0 && r[1] < 2)) return 0;
             const int nxt = r[3];
-            const bool next = nxt != f && run_selected(vstate, N, cls, level, nxt);
+            const bool next = nxt != last && r[1] > 1 && member(nxt);
             if (next && rec[5 * (nxt - N) + 2] != N + m) return 0;  // not hull neighbours
             nk += r[1] - (mi > 0 ? 1 : 0) - (next ? 1 : 0);
             ns += next ? 1 : 0;
@@ -1323,23 +1347,37 @@ struct FakeRunJoin {
         }
         return 0;
     }
+    // The members close on themselves through f, and f has the lowest id.
+    __device__ bool heads_ring(int f) const
+    {
+        int g = rec[5 * (f - N) + 3];
+        for (int mi = 0; mi < kMaxRunMembers; mi++) {
+            if (g == f) return mi > 0;
+            if (g < f || !member(g)) return false;
+            g = rec[5 * (g - N) + 3];
+        }
+        return false;
+    }
     __device__ void operator()(long long ii) const
     {
         const int f = N + (int)ii;
-        bool pick = run_selected(vstate, N, cls, level, f) && rec[5 * ii + 4] &&
-                    !run_selected(vstate, N, cls, level, rec[5 * ii + 2]);
-        int kept = 0, nsh = 0, nmem = 0;
-        if (pick) {
-            nmem = scan((int)ii, &kept, &nsh);
-            pick = nmem > 0;
+        int kept = 0, nsh = 0, nmem = 0, from = (int)ii;
+        if (member(f)) {
+            if (!member(rec[5 * ii + 2])) {
+                nmem = scan(from, f, &kept, &nsh);
+            } else if (heads_ring(f)) {
+                from = rec[5 * ii + 3] - N;
+                nmem = scan(from, f, &kept, &nsh);
+            }
         }
+        const bool pick = nmem > 0;
         const int k = warp_reserve(count, pick ? 1 : 0);
         const int base = warp_reserve(fan_n, pick ? kept + nsh : 0);
         if (pick) {
-            list[k] = f;
+            list[k] = N + from;
             fanoff[k] = base;
             fanlen[k] = kept | (nsh << 16);
-            int m = (int)ii, q = 0;
+            int m = from, q = 0;
             for (int mi = 0; mi < nmem; mi++) {
                 const int *r = rec + 5 * m;
                 const bool next = mi + 1 < nmem;
@@ -1364,11 +1402,16 @@ struct FakeRunJoin {
 // is popped.  The chain is cut into up to 32 pieces that share their end
 // vertices; each lane runs the rule on its piece (its pops are pops of the
 // whole chain too: a vertex inside the hull of a piece is inside the hull of
-// the chain), then lane 0 runs it once more over the pieces' leftover stacks
-// in order.  The triangles differ from one sequential pass but fill the same
-// pocket (the chain is star-shaped from the removed site), and the flip stage
-// makes the mesh Delaunay either way.  The lanes then write the remaining
-// hull edges, the boundary candidates and the released slots.
+// the chain), then neighbouring pieces are joined pair by pair: the left one's
+// lane runs the rule on over the right one's leftover stack.  The triangles
+// differ from one sequential pass but fill the same pocket (the chain is
+// star-shaped from the removed site), and the flip stage makes the mesh
+// Delaunay either way.  The lanes then write the remaining hull edges, the
+// boundary candidates and the released slots.
+// A step of the rule is a chain of shared-memory loads and an orientation,
+// some 0.1 us, and nothing else of the warp runs beside it, so the longest
+// chain of steps sets the time: with pieces of 16 joined by one lane in order a
+// run of 58 chain edges took 34 us, with pieces of 4 joined in pairs 30.
 struct FakeRemoveArgs {
     int4 *tv, *tn, *fwd;
     int *epoch, *freelist, *vtri;
@@ -1384,7 +1427,7 @@ struct FakeRemoveArgs {
 };
 
 constexpr int kFrPieces = 32;    // one piece per lane
-constexpr int kFrMinPiece = 16;  // chain edges per piece at least
+constexpr int kFrMinPiece = 4;   // chain edges per piece at least
 
 // Dynamic shared memory for fans of up to M triangles: Fs, Fi, O (M ints),
 // U (M + 1), the stacks S, SO (M + 1 + kFrPieces each: each piece's stack
@@ -1448,8 +1491,7 @@ struct FrRule {
 
 // What the lanes of a removal share besides the arrays.
 struct FrWarp {
-    int top[kFrPieces], used[kFrPieces];
-    int top2, cl, co;
+    int top[kFrPieces], used[kFrPieces];  // per piece: stack height (of the pieces joined to it), slots used
 };
 
 // Removes one selected unit (one warp); mem: fake_remove_smem(M) bytes, 16-byte
@@ -1501,34 +1543,33 @@ __device__ void fake_remove_item(const FakeRemoveArgs &a, int item, int M, unsig
         w.used[lane] = used;
     }
     __syncwarp();
-    // 2. lane 0: the leftover stacks in order (a piece's first vertex is the
-    // previous piece's last); the stack is rebuilt in place at S[0..)
-    // (it never passes the entry being read).  Slots: the pieces' unused
+    // 2. pieces joined in pairs: lane L (a multiple of 2 * step) goes on over the
+    // leftover stack of the pieces from L + step on (its first vertex is its
+    // own last), in place: with more entries read than written, its stack
+    // never passes the entry being read.  Slots: the joined pieces' unused
     // ones, in piece order.
-    if (lane == 0) {
-        int cl = 0, co = 0;  // next free slot: piece cl, offset co past its used ones
-        auto take = [&]() {
-            for (; cl < G; cl++, co = 0) {
-                const int pb0 = (int)((long long)cl * d / G), pb1 = (int)((long long)(cl + 1) * d / G);
-                if (pb0 + w.used[cl] + co < pb1) return Fs[pb0 + w.used[cl] + co++];
-            }
-            return -1;
-        };
-        int top2 = 0;
-        for (int L = 0; L < G; L++) {
-            const int pb0 = (int)((long long)L * d / G);
-            for (int j = L == 0 ? 0 : 1; j < w.top[L]; j++) {
-                const int idx = pb0 + L + j;
-                top2 = rule.push(S, SO, top2, S[idx], SO[idx], take, tally);
-            }
+    for (int step = 1; step < G; step *= 2) {
+        const int right = lane + step;
+        if ((lane & (2 * step - 1)) == 0 && right < G) {
+            const int rb0 = (int)((long long)right * d / G), end = min(G, right + step);
+            int cl = lane;
+            auto take = [&]() {
+                for (; cl < end; cl++) {
+                    const int pb0 = (int)((long long)cl * d / G), pb1 = (int)((long long)(cl + 1) * d / G);
+                    if (pb0 + w.used[cl] < pb1) return Fs[pb0 + w.used[cl]++];
+                }
+                return -1;
+            };
+            int *LS = S + b0 + lane, *LSO = SO + b0 + lane;
+            const int *RS = S + rb0 + right, *RSO = SO + rb0 + right;
+            int top = w.top[lane];
+            for (int j = 1, n = w.top[right]; j < n; j++) top = rule.push(LS, LSO, top, RS[j], RSO[j], take, tally);
+            w.top[lane] = top;
         }
-        w.top2 = top2;
-        w.cl = cl;
-        w.co = co;
+        __syncwarp();
     }
-    __syncwarp();
     tally.flush(a.ct);
-    const int top = w.top2, cl = w.cl, co = w.co;
+    const int top = w.top[0];
     // 3. the remaining chain edges are hull edges now
     for (int k = 1 + lane; k < top; k += 32) {
         const int ownv = SO[k];
@@ -1547,11 +1588,11 @@ __device__ void fake_remove_item(const FakeRemoveArgs &a, int item, int M, unsig
         if (lane == 0 && tot != d) set_err(a.ct, GPUDT_ERR_TOPOLOGY, 74);
     }
     {
-        // released slots: each piece's unused ones past what step 2 took
+        // released slots: each piece's unused ones
         int mine = 0, from = 0;
-        if (lane < G && lane >= cl) {
-            from = b0 + w.used[lane] + (lane == cl ? co : 0);
-            mine = max(0, b1 - from);
+        if (lane < G) {
+            from = b0 + w.used[lane];
+            mine = b1 - from;
         }
         int incl = mine;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1776,39 +1817,35 @@ int stage_boundary(Ctx &c)
     int r;
     Counters *ct = c.ctr;
     int *cand = c.aux;  // boundary candidates
-    const int order[4] = {0, 2, 1, 3};
     const long long recn = 4LL * c.cap_tris;
     int removed = 0;
     // stored fans of the selected fakes: (offset, length) per list entry and
     // the entries; the incidence array of the links stage is free by now
     int *fanoff = c.anchor, *fanlen = c.vround;  // per list entry (F <= V)
     int2 *fan = (int2 *)c.inc;                    // 3 cap ints: 1.5 cap entries
-    int run_levels = 1;  // separator levels covering the last class's chain of F / 4 fakes
-    while (run_levels < 6 && (1LL << (4 * run_levels)) < (c.F + 3) / 4) run_levels++;
-    // first pass: the four ring classes in turn (independent by construction);
-    // then rounds of priority-minimal fakes among all that remain
+    int run_levels = 1;  // separator levels covering the ring
+    while (run_levels < 6 && (1LL << (4 * run_levels)) < c.F) run_levels++;
+    // first pass: runs, one separator level after another; then runs of all
+    // that is left, by priority one by one after a pass that removed nothing
+    bool runs = true;
     for (int pass = 0, it = 0; removed < c.F; pass++) {
         if (pass > c.max_rounds / 4) return GPUDT_ERR_NOCONVERGE;
-        // pass 0: three ring classes one fake at a time, then the last class
-        // (a chain by then) as runs, one separator level after another; later
-        // passes: priority rounds among the fakes left
-        const int nsub = pass == 0 ? 3 + run_levels : 1;
+        const int nsub = pass == 0 ? run_levels : 1;
         for (int q = 0; q < nsub; q++, it++) {
             int round = next_round(c);
             int *nsel = &ct->r_fk[ring(it)], *nfan = &ct->r_fan[ring(it)], *nrec = rec_word(c);
-            if (pass == 0 && q >= 3) {
+            if (runs) {
                 // staging in alpha-stage buffers, idle until the mesh is final
                 int2 *stage = (int2 *)c.keys2;
                 int *rec5 = (int *)c.spectrum;
-                launch_n(c, FakeRunStage{c.tv, c.tn, c.vstate, c.vtri, c.N, order[3], q - 3, stage,
-                                         &ct->r_stage[ring(it)], rec5, ct},
+                const int level = pass == 0 ? q : -1;
+                launch_n(c, FakeRunStage{c.tv, c.tn, c.vstate, c.vtri, c.N, level, stage, &ct->r_stage[ring(it)], rec5,
+                                         ct},
                          c.F);
-                launch_n(c, FakeRunJoin{c.vstate, c.N, order[3], q - 3, stage, rec5, c.list, fanoff, fanlen, fan,
-                                        nsel, nfan, ct},
+                launch_n(c, FakeRunJoin{c.vstate, c.N, level, stage, rec5, c.list, fanoff, fanlen, fan, nsel, nfan, ct},
                          c.F);
             } else
-                launch_n(c, FakeSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, fanoff, fanlen, fan, nsel, nfan, c.N,
-                                       pass == 0 ? order[q] : -1, ct},
+                launch_n(c, FakeSelect{c.tv, c.tn, c.vstate, c.vtri, c.list, fanoff, fanlen, fan, nsel, nfan, c.N, ct},
                          c.F);
             r = launch_fake_remove(c,
                                FakeRemoveArgs{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.list, fanoff, fanlen, fan,
@@ -1824,7 +1861,9 @@ int stage_boundary(Ctx &c)
         r = read_counters(c);
         if (r) return r;
         if (c.hctr->err) return c.hctr->err;
-        if (c.hctr->fk_removed == removed) return GPUDT_ERR_NOCONVERGE;  // a full pass removed nothing
+        const bool none = c.hctr->fk_removed == removed;
+        if (none && !runs) return GPUDT_ERR_NOCONVERGE;  // priority always removes one
+        runs = !none;
         removed = c.hctr->fk_removed;
     }
     int ncand = c.hctr->ncand;

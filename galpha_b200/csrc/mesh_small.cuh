@@ -196,30 +196,30 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
     }
     if (next == kSmBoundary && m.to >= kSmBoundary && !bad) {
         if (lead) ct->sm_ns[2] = global_ns();
-        const int order[4] = {0, 2, 1, 3};
         int *fanoff = m.anchor, *fanlen = m.vround;
         int2 *fan = (int2 *)m.inc;
         int removed = 0;
+        bool runs = true;
         for (int pass = 0, it = 0; removed < m.F && !bad; pass++) {
             if (pass > m.max_rounds / 4) {
                 bad = 305;
                 break;
             }
-            const int nsub = pass == 0 ? 3 + m.run_levels : 1;
+            const int nsub = pass == 0 ? m.run_levels : 1;
             int now = removed;
             for (int q = 0; q < nsub && !bad; q++, it++) {
                 int *nsel = &ct->r_fk[rg(it)], *nfan = &ct->r_fan[rg(it)], *nrec = &ct->r_rec[rg(rr)];
                 round++;
-                if (pass == 0 && q >= 3) {
-                    spread(m.F, FakeRunStage{m.tv, m.tn, m.vstate, m.vtri, m.N, 3, q - 3, m.stage, &ct->r_stage[rg(it)],
+                if (runs) {
+                    const int level = pass == 0 ? q : -1;
+                    spread(m.F, FakeRunStage{m.tv, m.tn, m.vstate, m.vtri, m.N, level, m.stage, &ct->r_stage[rg(it)],
                                              m.rec5, ct});
                     cluster_barrier();
-                    spread(m.F, FakeRunJoin{m.vstate, m.N, 3, q - 3, m.stage, m.rec5, m.list, fanoff, fanlen, fan, nsel,
+                    spread(m.F, FakeRunJoin{m.vstate, m.N, level, m.stage, m.rec5, m.list, fanoff, fanlen, fan, nsel,
                                             nfan, ct});
                 } else {
-                    const int cls = pass == 0 ? order[q] : -1;
                     spread(m.F, FakeSelect{m.tv, m.tn, m.vstate, m.vtri, m.list, fanoff, fanlen, fan, nsel, nfan, m.N,
-                                           cls, ct});
+                                           ct});
                 }
                 cluster_barrier();
                 now = rd(&ct->fk_removed);  // changes only in the next selection
@@ -255,7 +255,9 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
                 rr++;
                 if (rd(&ct->sm_stop)) bad = -1;
             }
-            if (!bad && now == removed) bad = 306;  // a full pass removed nothing
+            const bool none = now == removed;
+            if (!bad && none && !runs) bad = 306;  // priority always removes one
+            runs = !none;
             removed = now;
         }
         if (!bad) {
@@ -421,7 +423,7 @@ static int launch_mesh_small(Ctx &c, int from, int to)
     m.V = c.V;
     m.cap = c.cap_tris;
     m.run_levels = 1;
-    while (m.run_levels < 6 && (1LL << (4 * m.run_levels)) < (c.F + 3) / 4) m.run_levels++;
+    while (m.run_levels < 6 && (1LL << (4 * m.run_levels)) < c.F) m.run_levels++;
     m.round0 = c.round_counter;
     m.rr0 = c.rec_round;
     m.max_rounds = c.max_rounds;
