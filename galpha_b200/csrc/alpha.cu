@@ -109,13 +109,39 @@ __device__ __forceinline__ double rho_tri(double2 A, double2 B, double2 C, bool 
 }
 
 // ------------------------------------------------------------------ kernels
-// The exact attached test, called with coordinates by value: the caller then
-// keeps its operands in registers (an array argument would have to live in
-// local memory on the hot path, for a call that almost never happens).
-__device__ __noinline__ int attached_exact_v(double ix, double iy, double jx, double jy, double kx, double ky)
+// The owned edges (mask `und`) of triangle t that the filter leaves undecided:
+// returns the mask of those that are unattached.  A call that reads its operands
+// again, after the loop over a thread's triangles: what lives across a call, and
+// what the exact test takes by address, is kept in local memory, and in that loop
+// every triangle stored and loaded it there (more L1 sectors than its gathers).
+__device__ __noinline__ unsigned attached_hard(const int4 *gv, const int4 *cn, const double2 *P, long long t,
+                                               unsigned und, Counters *ct)
 {
-    const double i[2] = {ix, iy}, j[2] = {jx, jy}, k[2] = {kx, ky};
-    return attached_exact(i, j, k);
+    const int4 g = gv[t], n = cn[t];
+    unsigned un = 0;
+    for (int i = 0; i < 3; i++) {
+        if (!((und >> i) & 1u)) continue;
+        const double2 pa = P[geti(g, p1(i))], pb = P[geti(g, m1(i))], pk = P[geti(g, i)];
+        const double qa[2] = {pa.x, pa.y}, qb[2] = {pb.x, pb.y}, qk[2] = {pk.x, pk.y};
+        int att = attached_filter(qa, qb, qk);
+        if (att == 2) {
+            atomicAdd(&ct->exact_attached, 1ull);
+            att = attached_exact(qa, qb, qk);
+        }
+        const int nb = geti(n, i);
+        if (att == 0 && nb >= 0) {
+            const double2 po = P[((const int *)gv)[4ll * dtri(nb) + dori(nb)]];
+            const double qo[2] = {po.x, po.y};
+            att = attached_filter(qa, qb, qo);
+            if (att == 2) {
+                atomicAdd(&ct->exact_attached, 1ull);
+                att = attached_exact(qa, qb, qo);
+            }
+        }
+        if (att == EXACT_OVERFLOW) set_err(ct, GPUDT_ERR_EXACT, 100);
+        if (!att) un |= 1u << i;
+    }
+    return un;
 }
 
 // Triangle keys, edge numbering, attached tests and edge keys in one pass over
@@ -126,11 +152,12 @@ __device__ __noinline__ int attached_exact_v(double ix, double iy, double jx, do
 // it writes the tile's edges and edge keys at their places.  The loads are a
 // triangle's three records, its corners and, for an owned edge its own corner
 // leaves unattached, the corner across it; bound by the latency of those
-// gathers (issue slots 38 % busy at 32 warps per SM, which the registers of the
+// gathers (issue slots 40 % busy at 32 warps per SM, which the registers of the
 // double-double arithmetic allow), so a round's records are loaded one round
-// ahead, and by the wait for earlier tiles: 4 triangles per thread take 0.57
-// ms at 8.4 M triangles, 2 take 0.64, 1 takes 0.75, 8 by blocks of 128 take
-// 0.80 (longer chains ahead of the tiles that wait).  Up to kAkFew triangles
+// ahead, and by the wait for earlier tiles: 4 triangles per thread took 0.57
+// ms at 8.0 M triangles, 2 took 0.64, 1 took 0.75, 8 by blocks of 128 took
+// 0.80 (longer chains ahead of the tiles that wait); 0.48 since the exact tests
+// are made after the loop.  Up to kAkFew triangles
 // there are too few tiles of four to fill the GPU and one per thread is used
 // (2,000 triangles: 20 us with four, 7 with one).  As five launches (edge
 // counts, a scan, keys, a scan over the edges, edge keys from a second gather)
@@ -174,7 +201,7 @@ __global__ void __launch_bounds__(kAkThreads, 4) k_alpha_keys(AlphaKeysArgs A)
     if (threadIdx.x == 0) s_tile = atomicAdd((int *)(A.status + A.tiles), 1);
     __syncthreads();
     const int tile = s_tile;
-    unsigned flags[kAkItems];  // bits 0-2 owned edges, 3-5 unattached ones
+    unsigned flags[kAkItems];  // bits 0-2 owned edges, 3-5 unattached ones, 6-8 undecided ones
     int incl[kAkItems], cnt[kAkItems];  // owned | unattached << 16
     const long long t0 = (long long)tile * kAkTile + threadIdx.x;
     int4 v, n, g;  // the next triangle's records, loaded one round ahead
@@ -217,41 +244,35 @@ __global__ void __launch_bounds__(kAkThreads, 4) k_alpha_keys(AlphaKeysArgs A)
             for (int i = 0; i < 3; i++) {
                 if (!((f >> i) & 1u)) continue;
                 const double2 pa = Q[p1(i)], pb = Q[m1(i)], pk = Q[i], po = O[i];
-                double qa[2] = {pa.x, pa.y}, qb[2] = {pb.x, pb.y}, qk[2] = {pk.x, pk.y};
+                const double qa[2] = {pa.x, pa.y}, qb[2] = {pb.x, pb.y}, qk[2] = {pk.x, pk.y};
                 int att = attached_filter(qa, qb, qk);
-                if (att == 2) {
-                    atomicAdd(&A.ct->exact_attached, 1ull);
-                    att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, pk.x, pk.y);
-                }
                 if (att == 0 && opp[i] >= 0) {
-                    double qo[2] = {po.x, po.y};
+                    const double qo[2] = {po.x, po.y};
                     att = attached_filter(qa, qb, qo);
-                    if (att == 2) {
-                        atomicAdd(&A.ct->exact_attached, 1ull);
-                        att = attached_exact_v(pa.x, pa.y, pb.x, pb.y, po.x, po.y);
-                    }
                 }
-                if (att == EXACT_OVERFLOW) set_err(A.ct, GPUDT_ERR_EXACT, 100);
-                if (!att) {
-                    f |= 8u << i;
-                    s_rho[i * kAkTile + j] = rho_edge(pa, pb);
-                }
+                f |= (att == 0 ? 8u : att == 2 ? 64u : 0u) << i;
+                if (att != 1) s_rho[i * kAkTile + j] = rho_edge(pa, pb);
             }
         }
-        const int own = __popc(f & 7u) | (__popc(f & 56u) << 16);
-        int x = own;
+#pragma unroll
+        for (int q = 0; q < kAkItems; q++)
+            if (q == u) flags[q] = f;  // (registers have no run-time index)
+    }
+#pragma unroll
+    for (int u = 0; u < kAkItems; u++) {
+        if (flags[u] >> 6) flags[u] |= attached_hard(A.gv, A.cn, A.P, t0 + u * kAkThreads, flags[u] >> 6, A.ct) << 3;
+    }
+#pragma unroll
+    for (int u = 0; u < kAkItems; u++) {
+        const unsigned f = flags[u];
+        int x = __popc(f & 7u) | (__popc(f & 56u) << 16);
+        cnt[u] = x;
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
         if (lane == 31) s_part[u * (kAkThreads / 32) + w] = x;
-#pragma unroll
-        for (int q = 0; q < kAkItems; q++)
-            if (q == u) {  // (registers have no run-time index)
-                flags[q] = f;
-                cnt[q] = own;
-                incl[q] = x;
-            }
+        incl[u] = x;
     }
     __syncthreads();
     if (w == 0) {

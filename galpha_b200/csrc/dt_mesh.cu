@@ -1934,6 +1934,72 @@ __device__ __forceinline__ bool cons_has(const unsigned long long *h, unsigned m
     return false;
 }
 
+// The two filter stages of the in-circle test: 2 when undecided, else the sign;
+// *n64 counts a call the FP64 stage decided.
+__device__ __forceinline__ int incircle_fast(double2 A, double2 B, double2 C, double2 D, int *n64)
+{
+    const double pa[2] = {A.x, A.y}, pb[2] = {B.x, B.y}, pc[2] = {C.x, C.y}, pd[2] = {D.x, D.y};
+    int s = incircle_filter32(pa, pb, pc, pd);
+    if (s == 2) {
+        s = incircle_filter(pa, pb, pc, pd);
+        *n64 += s != 2;
+    }
+    return s;
+}
+
+// A triangle's vote for the flip of its edge i (the neighbour across is u).
+__device__ __forceinline__ void flip_vote(int t, int i, int u, int *prop, int *target, int *vote)
+{
+    prop[t] = i;
+    target[t] = u;
+    // votes carry a hashed priority (prio is a bijection on 32 bits):
+    // chains of competing flips then resolve in about log rounds
+    // instead of one step per round along increasing slot ids
+    const unsigned pt = prio((uint32_t)t);
+    atomicMin((unsigned *)&vote[t], pt);
+    atomicMin((unsigned *)&vote[u], pt);
+}
+
+// A triangle whose edges (mask `want`) the filters do not all decide: the edges in
+// order, up to the first one that is not locally Delaunay, with the exact stage.
+// All of the triangle's work, in a call that shares no value with the caller: what
+// lives across a call is kept in local memory, and the exact stage takes its points
+// by address; with either in the common path each test stored and loaded them there
+// (three quarters of the L1 sectors of a round, at 4,000,000 uniform points).
+__device__ __noinline__ void flip_check_hard(const int4 *tv, const int4 *tn, const double2 *pos, int t, int want,
+                                             int8_t *eflag, int *prop, int *target, int *vote, int *cands,
+                                             int *cand_n, Counters *ct)
+{
+    const int4 v = tv[t], n = tn[t];
+    int ci = -1, ntest = 0, nfilt = 0;
+    for (int i = 0; i < 3 && ci < 0; i++) {
+        if (!((want >> i) & 1)) continue;
+        const int e = geti(n, i);
+        const double2 A = pos[geti(v, p1(i))], B = pos[geti(v, m1(i))], C = pos[geti(v, i)];
+        const double2 D = pos[geti(tv[dtri(e)], dori(e))];
+        ntest++;
+        int s = incircle_fast(A, B, C, D, &nfilt);
+        if (s == 2) {
+            atomicAdd(&ct->exact_incircle, 1ull);
+            const double pa[2] = {A.x, A.y}, pb[2] = {B.x, B.y}, pc[2] = {C.x, C.y}, pd[2] = {D.x, D.y};
+            s = incircle_exact(pa, pb, pc, pd);
+            if (s == EXACT_OVERFLOW) {
+                set_err(ct, GPUDT_ERR_EXACT, 90);
+                break;
+            }
+        }
+        if (s > 0) ci = i;
+    }
+    warp_add_spread(ct->icc_spread, ntest);
+    warp_add_spread(ct->filt_spread, nfilt);
+    if (ci < 0) {
+        if (eflag) eflag[t] = 0;
+        return;
+    }
+    flip_vote(t, ci, dtri(geti(n, ci)), prop, target, vote);
+    cands[atomicAdd(cand_n, 1)] = t;
+}
+
 struct FlipCheck {
     const int4 *tv, *tn;
     const double2 *pos;
@@ -1950,7 +2016,6 @@ struct FlipCheck {
         // a list entry of -1 is a hole left by a fixed-slot FlipApply: nothing to test
         const int4 v = t >= 0 ? tv[t] : make_int4(-1, -1, -1, 0);
         int ci = -1, cu = -1, ntest = 0, nfilt = 0;
-        bool err = false;
         // the first round tests every edge once (from the lower slot); later
         // rounds test the edges a flip or a lost vote left marked
         const int fl = t < 0 ? 0 : (act ? eflag[t] : 7);
@@ -1973,45 +2038,29 @@ struct FlipCheck {
             double2 D[3];
 #pragma unroll
             for (int i = 0; i < 3; i++) D[i] = want[i] ? pos[geti(tu[i], dori(nb[i]))] : make_double2(0.0, 0.0);
+            bool hard = false;
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                if (ci >= 0 || err) break;
-                if (!want[i]) continue;
-                const double2 A = P[p1(i)], B = P[m1(i)], C = P[i];
-                double pa[2] = {A.x, A.y}, pb[2] = {B.x, B.y}, pc[2] = {C.x, C.y}, pd[2] = {D[i].x, D[i].y};
+                if (ci >= 0 || hard || !want[i]) continue;
+                const int s = incircle_fast(P[p1(i)], P[m1(i)], P[i], D[i], &nfilt);
+                hard = s == 2;
                 ntest++;
-                int s = incircle_filter32(pa, pb, pc, pd);
-                if (s == 2) {
-                    s = incircle_filter(pa, pb, pc, pd);
-                    if (s == 2) {
-                        atomicAdd(&ct->exact_incircle, 1ull);
-                        s = incircle_exact(pa, pb, pc, pd);
-                        if (s == EXACT_OVERFLOW) err = true;
-                    } else {
-                        nfilt++;
-                    }
-                }
-                if (!err && s > 0) {
+                if (s == 1) {
                     ci = i;
                     cu = dtri(nb[i]);
                 }
             }
+            if (hard) {
+                flip_check_hard(tv, tn, pos, t, (want[0] ? 1 : 0) | (want[1] ? 2 : 0) | (want[2] ? 4 : 0),
+                                act ? eflag : nullptr, prop, target, vote, cands, cand_n, ct);
+                return;
+            }
         }
-        if (err) set_err(ct, GPUDT_ERR_EXACT, 90);
         warp_add_spread(ct->icc_spread, ntest);
         warp_add_spread(ct->filt_spread, nfilt);
         const bool has = ci >= 0;
         if (act && !has && fl) eflag[t] = 0;  // every marked edge is locally Delaunay
-        if (has) {
-            prop[t] = ci;
-            target[t] = cu;
-            // votes carry a hashed priority (prio is a bijection on 32 bits):
-            // chains of competing flips then resolve in about log rounds
-            // instead of one step per round along increasing slot ids
-            const unsigned pt = prio((uint32_t)t);
-            atomicMin((unsigned *)&vote[t], pt);
-            atomicMin((unsigned *)&vote[cu], pt);
-        }
+        if (has) flip_vote(t, ci, cu, prop, target, vote);
         const int slot = warp_reserve(cand_n, has ? 1 : 0);
         if (has) cands[slot] = t;
     }
@@ -2275,8 +2324,11 @@ int stage_flip(Ctx &c)
         for (int k = 0; k < c.flip_sync; k++) {
             const int p = rounds & 1, w = ring(rounds), w1 = ring(rounds + 1), ahead = ring(rounds + kRing / 2);
             int round = next_round(c);
+            // 64 registers a thread in the first round too: left to itself the
+            // compiler takes 40 there and keeps the rest in local memory (600 us
+            // at 8.0 M triangles, 531 with 64)
             if (rounds == 0)
-                launch_n(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &ct->r_cand[w], ct,
+                launch_occ<4>(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &ct->r_cand[w], ct,
                                       c.eflag, c.chash, c.cmask},
                          nt);
             else

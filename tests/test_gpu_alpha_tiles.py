@@ -40,3 +40,22 @@ def test_alpha_smallest(engine, n):
     dt = engine.triangulate(G.GPUDTParams(pts, fboSize=256))
     ok, rep = compare_alpha(pts, dt.vtx, dt.tri, engine.alpha_resident(), 4)
     assert ok, rep
+
+
+@pytest.mark.parametrize("n", [500, 80000])
+def test_undecided_predicates(engine, n):
+    """Points of an integer grid: right and straight angles and cocircular fours
+    everywhere, so the filters of the in-circle and the attached test leave much
+    to the exact stage, with one triangle per thread and with four."""
+    import numpy as np
+    from dtcheck import compare_dt
+
+    side = int(2 * n ** 0.5)
+    ids = np.random.default_rng(n).permutation(side * side)[:n]
+    pts = np.stack([ids % side, ids // side], axis=1) / 1024.0
+    dt = engine.triangulate(G.GPUDTParams(pts, fboSize=1024))
+    ok, rep = compare_dt(pts, dt.vtx, dt.tri)
+    assert ok, rep
+    assert dt.status.exactIncircle > 0
+    ok, rep = compare_alpha(pts, dt.vtx, dt.tri, engine.alpha_resident(), 4)
+    assert ok, rep
