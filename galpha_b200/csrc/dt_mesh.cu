@@ -282,12 +282,6 @@ static int ring(int k)
 {
     return k % kRing;
 }
-// Marks the k ids after `first` (first + 1 .. first + k) as used by rounds
-// that device code numbered itself.
-static void skip_rounds(Ctx &c, int first, int k)
-{
-    if (first + k > c.round_counter) c.round_counter = first + k;
-}
 
 // ------------------------------------------------------------------- shift
 // A fan walk around interior vertex v: calls f(t, i, a, b) for every
@@ -1904,9 +1898,22 @@ int stage_boundary(Ctx &c)
 // The first round tests every edge once, from the triangle with the lower
 // slot.  A flip replaces edge (b, c) of the quad (a, b, d, c) by (a, d); only
 // the quad's four outer edges can then have stopped being locally Delaunay,
-// so the two new triangles are listed with their outer edges marked
-// (eflag), and later rounds test marked edges only.  A candidate that loses
-// its vote keeps its marks (all three after the one-sided first round).
+// so the two new triangles are listed with their outer edges marked, and later
+// rounds test marked edges only.  A candidate that loses its vote keeps its
+// marks (all three after the one-sided first round).
+//
+// What the stage keeps of a triangle is the smallest vote of the round (unsigned,
+// all ones: none) and an int2, in an array of the alpha stage that is idle here:
+//   x  (round + 1) << 4 | flipped in that round << 3 | marked edges, written when
+//      the triangle is put on the next round's list
+//   y  enc(the other triangle of the flip, the index of the flipped edge)
+// Rounds past the first are gathers and scattered stores at 300 to 500 ns each
+// with nothing between them, so the sectors a candidate touches set their time.
+// With stamps, marks, epochs and forwarding links in arrays of their own, the
+// proposed edge and its neighbour in two more, and a triangle of each vertex kept
+// up to date (nothing past the constraints reads it), a flip touched some 24
+// sectors, now 10.  The votes stay apart: the first round's go to a third of all
+// triangles, and in an array of four bytes each they stay in L2.
 // Set of constrained edges: open addressing over keys (min id << 32 | max id),
 // empty slots ~0 (constraints, section below).
 __device__ __forceinline__ unsigned long long cons_key(int a, int b)
@@ -1947,11 +1954,9 @@ __device__ __forceinline__ int incircle_fast(double2 A, double2 B, double2 C, do
     return s;
 }
 
-// A triangle's vote for the flip of its edge i (the neighbour across is u).
-__device__ __forceinline__ void flip_vote(int t, int i, int u, int *prop, int *target, int *vote)
+// The votes of triangle t for the flip with its neighbour u.
+__device__ __forceinline__ void flip_vote(int *vote, int t, int u)
 {
-    prop[t] = i;
-    target[t] = u;
     // votes carry a hashed priority (prio is a bijection on 32 bits):
     // chains of competing flips then resolve in about log rounds
     // instead of one step per round along increasing slot ids
@@ -1967,8 +1972,7 @@ __device__ __forceinline__ void flip_vote(int t, int i, int u, int *prop, int *t
 // by address; with either in the common path each test stored and loaded them there
 // (three quarters of the L1 sectors of a round, at 4,000,000 uniform points).
 __device__ __noinline__ void flip_check_hard(const int4 *tv, const int4 *tn, const double2 *pos, int t, int want,
-                                             int8_t *eflag, int *prop, int *target, int *vote, int *cands,
-                                             int *cand_n, Counters *ct)
+                                             int *vote, int2 *cands, int *cand_n, Counters *ct)
 {
     const int4 v = tv[t], n = tn[t];
     int ci = -1, ntest = 0, nfilt = 0;
@@ -1992,35 +1996,37 @@ __device__ __noinline__ void flip_check_hard(const int4 *tv, const int4 *tn, con
     }
     warp_add_spread(ct->icc_spread, ntest);
     warp_add_spread(ct->filt_spread, nfilt);
-    if (ci < 0) {
-        if (eflag) eflag[t] = 0;
-        return;
-    }
-    flip_vote(t, ci, dtri(geti(n, ci)), prop, target, vote);
-    cands[atomicAdd(cand_n, 1)] = t;
+    if (ci < 0) return;
+    const int u = dtri(geti(n, ci));
+    flip_vote(vote, t, u);
+    cands[atomicAdd(cand_n, 1)] = make_int2(enc(t, ci), u);
 }
 
 struct FlipCheck {
     const int4 *tv, *tn;
     const double2 *pos;
     const int *act;
-    int *vote, *prop, *target, *cands;
+    const int2 *st;
+    int *vote;
+    int2 *cands;  // (triangle and edge, neighbour)
     int *cand_n;
     Counters *ct;
-    int8_t *eflag;
     const unsigned long long *chash;  // constrained edges, never flipped (null: none)
     unsigned cmask;
     __device__ void operator()(long long ii) const
     {
         const int t = act ? act[ii] : (int)ii;  // no list: every slot (the first round)
         // a list entry of -1 is a hole left by a fixed-slot FlipApply: nothing to test
-        const int4 v = t >= 0 ? tv[t] : make_int4(-1, -1, -1, 0);
+        int4 v = make_int4(-1, -1, -1, 0), n = v;
+        if (t >= 0) {
+            v = tv[t];
+            n = tn[t];
+        }
         int ci = -1, cu = -1, ntest = 0, nfilt = 0;
         // the first round tests every edge once (from the lower slot); later
         // rounds test the edges a flip or a lost vote left marked
-        const int fl = t < 0 ? 0 : (act ? eflag[t] : 7);
+        const int fl = t < 0 ? 0 : (act ? st[t].x & 7 : 7);
         if (v.x >= 0 && fl) {
-            const int4 n = tn[t];
             const int nb[3] = {n.x, n.y, n.z};
             const double2 P[3] = {pos[v.x], pos[v.y], pos[v.z]};  // once per triangle, not per edge
             // the neighbours and their apexes of every edge to be tested are
@@ -2052,17 +2058,16 @@ struct FlipCheck {
             }
             if (hard) {
                 flip_check_hard(tv, tn, pos, t, (want[0] ? 1 : 0) | (want[1] ? 2 : 0) | (want[2] ? 4 : 0),
-                                act ? eflag : nullptr, prop, target, vote, cands, cand_n, ct);
+                                vote, cands, cand_n, ct);
                 return;
             }
         }
         warp_add_spread(ct->icc_spread, ntest);
         warp_add_spread(ct->filt_spread, nfilt);
         const bool has = ci >= 0;
-        if (act && !has && fl) eflag[t] = 0;  // every marked edge is locally Delaunay
-        if (has) flip_vote(t, ci, cu, prop, target, vote);
+        if (has) flip_vote(vote, t, cu);
         const int slot = warp_reserve(cand_n, has ? 1 : 0);
-        if (has) cands[slot] = t;
+        if (has) cands[slot] = make_int2(enc(t, ci), cu);
     }
 };
 
@@ -2073,70 +2078,57 @@ struct FlipCheck {
 // returning atomics per candidate (record, flip and list reservations) --
 // the tail of the kernel's latency chain -- by plain stores.
 struct FlipApply {
-    int4 *tv, *tn, *fwd;
-    int *epoch, *vtri, *vote, *stamp, *next;
+    int4 *tv, *tn;
+    int2 *st;
+    const int *vote;
+    int *next;
     int *next_n;
-    const int *prop, *target, *cands;
+    const int2 *cands;
     Relink *rec;
-    int round;
+    int stamp;  // round + 1
     Counters *ct;
-    int8_t *eflag;
     bool first;  // first round: a losing candidate was tested one-sided, so all its edges stay marked
     const int *cand_n;  // candidates of the round (the launch count)
     int *rec_n;         // relink records of the round
     long long rec_cap;  // relink records the array holds
-    __device__ bool fresh(int x) const { return x >= 0 && atomicExch(&stamp[x], round) != round; }
     __device__ void operator()(long long ii) const
     {
-        const int t = cands[ii];
-        const int u = target[t];
-        const unsigned pt = prio((uint32_t)t);
+        const int2 cd = cands[ii];
+        const int t = dtri(cd.x), i = dori(cd.x), u = cd.y;
+        const int pt = (int)prio((uint32_t)t);
         // the vote words and both triangles are loaded together (a winner
         // needs all of them; the kernel is bound by these gathers' latency)
-        const unsigned vt = (unsigned)vote[t], vu = (unsigned)vote[u];
-        const int i = prop[t];
+        const int vt = vote[t], vu = vote[u], ts = st[t].x;
         const int4 tvv = tv[t], tnn = tn[t], uvv = tv[u], unn = tn[u];
         const bool win = vt == pt && vu == pt;
-        int nx[6], nn = 0;
+        int nx[2], nn = 0;
         Relink r4[4];
         if (!win) {
-            if (first) eflag[t] = 7;
-            if (fresh(t)) nx[nn++] = t;
+            // listed again with its marks, unless the winner that takes it as its
+            // neighbour has listed it, or does so later (with the marks of a flip)
+            const int x = (stamp << 4) | (first ? 7 : ts & 7);
+            if (ts >> 4 != stamp && atomicCAS(&st[t].x, ts, x) == ts) nx[nn++] = t;
         } else {
             const int e = geti(tnn, i);
             const int j = dori(e);
             const int a = geti(tvv, i), b = geti(tvv, p1(i)), cc = geti(tvv, m1(i)), d = geti(uvv, j);
             const int ot1 = geti(tnn, p1(i)), ot2 = geti(tnn, m1(i));
             const int ou1 = geti(unn, p1(j)), ou2 = geti(unn, m1(j));
-            epoch[t] = round;
-            epoch[u] = round;
             tv[t] = make_int4(a, b, d, 0);
             tv[u] = make_int4(d, cc, a, 0);
             tn[t] = make_int4(-1, enc(u, 1), -1, 0);
             tn[u] = make_int4(-1, enc(t, 1), -1, 0);
-            int4 ft = make_int4(0, 0, 0, 0), fu = make_int4(0, 0, 0, 0);
-            seti(ft, i, -1);
-            seti(ft, p1(i), enc(u, 0));
-            seti(ft, m1(i), enc(t, 2));
-            seti(fu, j, -1);
-            seti(fu, p1(j), enc(t, 0));
-            seti(fu, m1(j), enc(u, 2));
-            fwd[t] = ft;
-            fwd[u] = fu;
             r4[0] = Relink{enc(t, 0), ou1};
             r4[1] = Relink{enc(t, 2), ot2};
             r4[2] = Relink{enc(u, 0), ot1};
             r4[3] = Relink{enc(u, 2), ou2};
-            vtri[a] = enc(t, 0);
-            vtri[b] = enc(t, 1);
-            vtri[d] = enc(t, 2);
-            vtri[cc] = enc(u, 1);
             // only the four outer edges of the new pair can have stopped being
             // locally Delaunay: edges 0 and 2 of t and of u
-            eflag[t] = 5;
-            eflag[u] = 5;
-            if (fresh(t)) nx[nn++] = t;
-            if (fresh(u)) nx[nn++] = u;
+            const int x = (stamp << 4) | 8 | 5;
+            st[t] = make_int2(x, enc(u, i));  // no other candidate lists t
+            st[u].y = enc(t, j);
+            nx[nn++] = t;
+            if (atomicExch(&st[u].x, x) >> 4 != stamp) nx[nn++] = u;  // (u itself may be a losing candidate)
         }
         const int nc = *cand_n;  // the same for every thread of the launch
         if (4ll * nc <= rec_cap) {
@@ -2163,21 +2155,48 @@ struct FlipApply {
     }
 };
 
-struct FlipReset {
-    int *vote;
-    const int *target, *cands;
+// The outer links of the flips of a round, both sides at once; a neighbour that
+// was flipped in the same round says where its edge went.
+struct FlipRelink {
+    int4 *tn;
+    const int2 *st;
+    const Relink *rec;
+    int stamp;
     __device__ void operator()(long long ii) const
     {
-        int t = cands[ii];
-        vote[t] = -1;  // 0xffffffff: no unsigned vote yet
-        vote[target[t]] = -1;
+        const Relink r = rec[ii];
+        if (r.loc < 0) return;
+        if (r.old < 0) {
+            set_link(tn, r.loc, -1);
+            return;
+        }
+        const int u = dtri(r.old), b = dori(r.old);
+        const int2 s = st[u];
+        if (s.x >> 3 == (stamp << 1 | 1)) {
+            const int k = dori(s.y);
+            set_link(tn, r.loc, b == p1(k) ? enc(dtri(s.y), 0) : b == m1(k) ? enc(u, 2) : -1);
+        } else {
+            set_link(tn, r.loc, r.old);
+            set_link(tn, r.old, r.loc);
+        }
+    }
+};
+
+struct FlipReset {
+    int *vote;
+    const int2 *cands;
+    __device__ void operator()(long long ii) const
+    {
+        const int2 c = cands[ii];
+        vote[dtri(c.x)] = -1;  // 0xffffffff: no unsigned vote yet
+        vote[c.y] = -1;
     }
 };
 
 // The last launch of a flip round: the relinks and, independent of them, the
 // votes of the round's candidates taken back; it clears the words of the round
 // kRing / 2 ahead.
-__global__ void __launch_bounds__(256) k_flip_finish(Relinker rl, const int *nrec, FlipReset rs, const int *ncand,
+__global__ void __launch_bounds__(256) k_flip_finish(FlipRelink rl, const int *nrec, FlipReset rs, const int *ncand,
                                                      Clears z)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2195,7 +2214,7 @@ __global__ void __launch_bounds__(256) k_flip_finish(Relinker rl, const int *nre
 // inside ONE block, with __syncthreads between their phases instead of a launch
 // per phase (long flip chains -- a retriangulated hull pocket, a dense cluster
 // -- otherwise cost three launches per round for a handful of flips).  The same
-// functors run in the same phase order with consecutive round ids, so the mesh
+// functors run in the same phase order with the same stamps, so the mesh
 // is the one the launched rounds produce.  The block stops when the list
 // empties, when a round's list exceeds `leave` (the host goes back to launched
 // rounds) or after max_rounds; no thread ever waits on another block.  It
@@ -2205,9 +2224,8 @@ constexpr int kTailThreads = 1024;
 // c.tail_enter: the host hands over at or below this many active triangles;
 // c.tail_leave: the block hands back above this many.
 
-__global__ void __launch_bounds__(kTailThreads) k_flip_tail(FlipCheck ck, FlipApply ap, Relinker rl, FlipReset rs,
-                                                             int *l0, int *l1, int k0, int round0,
-                                                             int max_rounds, int leave)
+__global__ void __launch_bounds__(kTailThreads, 1) k_flip_tail(FlipCheck ck, FlipApply ap, FlipRelink rl, FlipReset rs,
+                                                             int *l0, int *l1, int k0, int max_rounds, int leave)
 {
     Counters *ct = ck.ct;
     int k = 0;
@@ -2221,7 +2239,6 @@ __global__ void __launch_bounds__(kTailThreads) k_flip_tail(FlipCheck ck, FlipAp
             ct->r_act[w1] = 0;
         }
         __syncthreads();
-        const int round = round0 + k;
         const bool odd = (k0 + k) & 1;
         ck.act = odd ? l1 : l0;
         ck.cand_n = &ct->r_cand[w];
@@ -2232,11 +2249,10 @@ __global__ void __launch_bounds__(kTailThreads) k_flip_tail(FlipCheck ck, FlipAp
         ap.next_n = &ct->r_act[w1];
         ap.cand_n = &ct->r_cand[w];
         ap.rec_n = &ct->r_frec[w];
-        ap.round = round;
+        ap.stamp = rl.stamp = k0 + k + 1;
         for (int i = threadIdx.x; i < nc; i += kTailThreads) ap(i);
         __syncthreads();
         const int nr = *(volatile int *)&ct->r_frec[w];
-        rl.round = round;
         for (int i = threadIdx.x; i < nr; i += kTailThreads) rl(i);
         for (int i = threadIdx.x; i < nc; i += kTailThreads) rs(i);  // independent of the relinks
         __syncthreads();
@@ -2250,34 +2266,20 @@ __global__ void __launch_bounds__(kTailThreads) k_flip_tail(FlipCheck ck, FlipAp
     if (threadIdx.x == 0) ct->tail_rounds = k;
 }
 
-// Start of the stage, four slots per thread: no vote (unsigned words start at
-// the maximum), no stamp, and the edges still to be tested: none marked before
-// a first launched round (it tests all), all when the in-block rounds start
-// from the list of live slots, made here (the arrays are 256-byte aligned).
+// Start of the stage: no vote (unsigned words start at the maximum), no stamp, and
+// the edges still to be tested: none marked before a first launched round (it
+// tests all), all when the in-block rounds start from the list of live slots,
+// made here.
 struct FlipInit {
     const int4 *tv;
-    int *vote, *stamp;
-    int8_t *eflag;
+    int2 *st;
+    int *vote;
     int *list, *count;  // live slots (null: not wanted)
-    int nt, cap;
-    __device__ void operator()(long long q) const
+    __device__ void operator()(long long t) const
     {
-        const int s = 4 * (int)q;
-        const unsigned char e = list ? 7 : 0;
-        if (s + 3 < cap) {
-            *(int4 *)(stamp + s) = make_int4(-1, -1, -1, -1);
-            *(uchar4 *)(eflag + s) = make_uchar4(e, e, e, e);
-        } else {
-            for (int k = s; k < cap; k++) {
-                stamp[k] = -1;
-                eflag[k] = (int8_t)e;
-            }
-        }
-        if (s + 3 < nt) *(int4 *)(vote + s) = make_int4(-1, -1, -1, -1);
-        for (int k = s; k < min(s + 4, nt); k++) {
-            if (s + 3 >= nt) vote[k] = -1;
-            if (list && tv[k].x >= 0) list[atomicAdd(count, 1)] = k;
-        }
+        st[t] = make_int2(list ? 7 : 0, 0);
+        vote[t] = -1;
+        if (list && tv[t].x >= 0) list[atomicAdd(count, 1)] = (int)t;
     }
 };
 
@@ -2289,33 +2291,28 @@ int stage_flip(Ctx &c)
     Counters *ct = c.ctr;
     int nt = c.hctr->ntris;
     int *lists[2] = {c.list, c.list2};
-    int *prop = c.aux, *target = c.aux2, *cands = c.inc, *stamp = c.stamp;
+    int2 *st = (int2 *)c.keys2;
+    int2 *cands = (int2 *)c.inc;
     // the first launched round tests every slot directly; the in-block tail
     // (small meshes) starts from a list of the live slots
-    launch_n(c, FlipInit{c.tv, c.vote, stamp, c.eflag, nt <= c.tail_enter ? lists[0] : nullptr, &ct->r_act[0], nt,
-                         c.cap_tris},
-             ((long long)c.cap_tris + 3) / 4);
+    launch_n(c, FlipInit{c.tv, st, c.vote, nt <= c.tail_enter ? lists[0] : nullptr, &ct->r_act[0]}, nt);
     const long long capn = c.cap_tris, recn = 4LL * c.cap_tris;
     int rounds = 0;
     long long known = nt;  // active-list length at `rounds`, as last read (nt bounds the first)
     while (known > 0) {
         if (known <= c.tail_enter) {
-            const int round0 = next_round(c);
             k_flip_tail<<<1, kTailThreads, 0, c.stream>>>(
-                FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, nullptr, ct, c.eflag, c.chash,
-                          c.cmask},
-                FlipApply{c.tv, c.tn, c.fwd, c.epoch, c.vtri, c.vote, stamp, nullptr, nullptr, prop, target, cands,
-                          c.rec, 0, ct, c.eflag, false, nullptr, nullptr, 3ll * c.cap_tris},
-                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, 0, ct}, FlipReset{c.vote, target, cands},
-                lists[0], lists[1], rounds, round0, c.max_rounds + 1 - rounds, c.tail_leave);
+                FlipCheck{c.tv, c.tn, c.pos, nullptr, st, c.vote, cands, nullptr, ct, c.chash, c.cmask},
+                FlipApply{c.tv, c.tn, st, c.vote, nullptr, nullptr, cands, c.rec, 0, ct, false, nullptr, nullptr,
+                          3ll * c.cap_tris},
+                FlipRelink{c.tn, st, c.rec, 0}, FlipReset{c.vote, cands}, lists[0], lists[1], rounds,
+                c.max_rounds + 1 - rounds, c.tail_leave);
             count_launch();
             GALPHA_CUDA(cudaGetLastError());
             r = read_counters(c);
             if (r) return r;
             if (c.hctr->err) return c.hctr->err;
-            const int k = c.hctr->tail_rounds;
-            skip_rounds(c, round0, k - 1);
-            rounds += k;
+            rounds += c.hctr->tail_rounds;
             known = c.hctr->r_act[ring(rounds)];
             if (known == 0) break;
             if (rounds > c.max_rounds) return GPUDT_ERR_NOCONVERGE;
@@ -2323,26 +2320,21 @@ int stage_flip(Ctx &c)
         }
         for (int k = 0; k < c.flip_sync; k++) {
             const int p = rounds & 1, w = ring(rounds), w1 = ring(rounds + 1), ahead = ring(rounds + kRing / 2);
-            int round = next_round(c);
-            // 64 registers a thread in the first round too: left to itself the
-            // compiler takes 40 there and keeps the rest in local memory (600 us
-            // at 8.0 M triangles, 531 with 64)
+            const int stamp = rounds + 1;
             if (rounds == 0)
-                launch_occ<4>(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, c.vote, prop, target, cands, &ct->r_cand[w], ct,
-                                      c.eflag, c.chash, c.cmask},
-                         nt);
+                launch_occ<4>(c, FlipCheck{c.tv, c.tn, c.pos, nullptr, st, c.vote, cands, &ct->r_cand[w], ct, c.chash,
+                                           c.cmask},
+                              nt);
             else
-                launch_dev(c, FlipCheck{c.tv, c.tn, c.pos, lists[p], c.vote, prop, target, cands, &ct->r_cand[w], ct,
-                                        c.eflag, c.chash, c.cmask},
-                           &ct->r_act[w], capn);
-            launch_dev(c, FlipApply{c.tv, c.tn, c.fwd, c.epoch, c.vtri, c.vote, stamp, lists[1 - p], &ct->r_act[w1],
-                                    prop, target, cands, c.rec, round, ct, c.eflag, rounds == 0, &ct->r_cand[w],
-                                    &ct->r_frec[w], 3ll * c.cap_tris},
+                launch_dev_occ<4>(c, FlipCheck{c.tv, c.tn, c.pos, lists[p], st, c.vote, cands, &ct->r_cand[w], ct,
+                                               c.chash, c.cmask},
+                                  &ct->r_act[w], capn);
+            launch_dev(c, FlipApply{c.tv, c.tn, st, c.vote, lists[1 - p], &ct->r_act[w1], cands, c.rec, stamp, ct, rounds == 0,
+                                    &ct->r_cand[w], &ct->r_frec[w], 3ll * c.cap_tris},
                        &ct->r_cand[w], capn);
             const long long blocks = std::max(1ll, std::min((recn + 255) / 256, (long long)c.sm_count * 8));
             k_flip_finish<<<(unsigned)blocks, 256, 0, c.stream>>>(
-                Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, &ct->r_frec[w],
-                FlipReset{c.vote, target, cands}, &ct->r_cand[w],
+                FlipRelink{c.tn, st, c.rec, stamp}, &ct->r_frec[w], FlipReset{c.vote, cands}, &ct->r_cand[w],
                 Clears{{&ct->r_act[ahead], &ct->r_cand[ahead], &ct->r_frec[ahead]}});
             count_launch();
             rounds++;

@@ -186,7 +186,6 @@ struct Ctx {
     int *freelist = nullptr;   // [cap]
     Relink *rec = nullptr;     // [3*cap]
     int *vtri = nullptr;       // [V] one incident oriented triangle
-    int8_t *eflag = nullptr;   // [cap] flip: edges of a triangle still to be tested (bit i: edge opposite vtx[i])
     int *perm = nullptr;       // [V] single-set path: internal (spatially sorted) vertex -> input index
     bool renumbered = false;   // the mesh stages ran on spatially sorted ids (perm); outputs use input ids
     int8_t *vstate = nullptr;  // [V]
@@ -347,7 +346,7 @@ struct Clears {
 // Grid-stride launch over [0, *n) with the count read on the device, so a
 // round of kernels can run without the host learning its size.
 template <class F>
-__global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n, Clears z)
+__device__ __forceinline__ void for_each_dev(const F &f, const int *n, const Clears &z)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
 #pragma unroll
@@ -361,6 +360,19 @@ __global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n, Clears 
 }
 
 template <class F>
+__global__ void __launch_bounds__(256) k_for_each_dev(F f, const int *n, Clears z)
+{
+    for_each_dev(f, n, z);
+}
+
+// The same with at least MINB resident blocks per SM asked for.
+template <class F, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_for_each_dev_occ(F f, const int *n, Clears z)
+{
+    for_each_dev(f, n, z);
+}
+
+template <class F>
 inline void launch_dev(const Ctx &c, F f, const int *n_dev, long long max_n, const Clears &z = Clears())
 {
     if (max_n <= 0) return;
@@ -368,6 +380,17 @@ inline void launch_dev(const Ctx &c, F f, const int *n_dev, long long max_n, con
     long long maxb = (long long)c.sm_count * 8;
     if (blocks > maxb) blocks = maxb;
     k_for_each_dev<<<(unsigned)blocks, 256, 0, c.stream>>>(f, n_dev, z);
+    count_launch();
+}
+
+template <int MINB, class F>
+inline void launch_dev_occ(const Ctx &c, F f, const int *n_dev, long long max_n, const Clears &z = Clears())
+{
+    if (max_n <= 0) return;
+    long long blocks = (max_n + 255) / 256;
+    long long maxb = (long long)c.sm_count * 8;
+    if (blocks > maxb) blocks = maxb;
+    k_for_each_dev_occ<F, MINB><<<(unsigned)blocks, 256, 0, c.stream>>>(f, n_dev, z);
     count_launch();
 }
 

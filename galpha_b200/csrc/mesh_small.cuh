@@ -33,9 +33,9 @@ struct SmallMesh {
     int4 *tv, *tn, *fwd;
     int *epoch, *vote, *stamp, *freelist, *vtri, *vround, *anchor;
     int *list, *list2, *aux, *aux2, *inc;
-    int8_t *vstate, *eflag;
+    int8_t *vstate;
     Relink *rec;
-    int2 *stage;      // fake runs: staged fan entries
+    int2 *stage;      // fake runs: staged fan entries; flips: the triangles' states
     int *rec5;        // fake runs: records
     unsigned char *longfan;  // fake_remove_smem(kMaxFanLong) bytes per block
     const unsigned long long *chash;
@@ -304,13 +304,14 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
     if (next == kSmFlip && m.to >= kSmFlip && !bad) {
         if (lead) ct->sm_ns[3] = global_ns();
         const int nt = rd(&ct->ntris);
-        each((m.cap + 3) / 4, FlipInit{m.tv, m.vote, m.stamp, m.eflag, m.list, &ct->r_act[0], nt, m.cap});
+        int2 *st = m.stage;
+        int2 *cands = (int2 *)m.inc;
+        each(nt, FlipInit{m.tv, st, m.vote, m.list, &ct->r_act[0]});
         cluster_barrier();
-        FlipCheck ck{m.tv, m.tn, m.pos, nullptr, m.vote, aux, aux2, m.inc, nullptr, ct, m.eflag, m.chash, m.cmask};
-        FlipApply ap{m.tv, m.tn, m.fwd, m.epoch, m.vtri, m.vote, m.stamp, nullptr, nullptr, aux, aux2, m.inc, m.rec, 0,
-                     ct, m.eflag, false, nullptr, nullptr, 3ll * m.cap};
-        Relinker rl{m.tn, m.fwd, m.epoch, m.rec, m.tv, m.vtri, 0, ct};
-        const FlipReset rs{m.vote, aux2, m.inc};
+        FlipCheck ck{m.tv, m.tn, m.pos, nullptr, st, m.vote, cands, nullptr, ct, m.chash, m.cmask};
+        FlipApply ap{m.tv, m.tn, st, m.vote, nullptr, nullptr, cands, m.rec, 0, ct, false, nullptr, nullptr, 3ll * m.cap};
+        FlipRelink rl{m.tn, st, m.rec, 0};
+        const FlipReset rs{m.vote, cands};
         // one round: the whole cluster, or block 0 alone (by = its threads, sync its barrier)
         auto flips = [&](int k, int n, int first, int by, auto sync) {
             const int w = rg(k), w1 = rg(k + 1), ahead = rg(k + kRing / 2);
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
             ap.next_n = &ct->r_act[w1];
             ap.cand_n = &ct->r_cand[w];
             ap.rec_n = &ct->r_frec[w];
-            ap.round = rl.round = round + 1 + k;
+            ap.stamp = rl.stamp = k + 1;
             for (int i = first; i < nc; i += by) ap(i);
             sync();
             const int nr = rd(&ct->r_frec[w]);
@@ -362,7 +363,6 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
             k = rd(&ct->tail_rounds);
         }
         flip_rounds = k;
-        round += 1 + k;
         next = kSmFlip + 1;
     }
     if (lead) {
@@ -410,7 +410,6 @@ static int launch_mesh_small(Ctx &c, int from, int to)
     m.aux2 = c.aux2;
     m.inc = c.inc;
     m.vstate = c.vstate;
-    m.eflag = c.eflag;
     m.rec = c.rec;
     m.stage = (int2 *)c.keys2;  // alpha-stage buffers, idle until the mesh is final
     m.rec5 = (int *)c.spectrum;
