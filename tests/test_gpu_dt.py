@@ -280,3 +280,21 @@ def test_schedule_rejects_out_of_range(engine):
             engine.set_schedule(*bad)
     assert engine.schedule() == dict(shift_group=4, missing_group=2, flip_sync=4, flip_tail_enter=4096,
                                      flip_tail_leave=32768)
+
+
+@pytest.mark.parametrize("fbo", [256, 512, 8192])
+@pytest.mark.parametrize("n", [3, 40, 3000])
+def test_colouring_near_and_far(engine, n, fbo):
+    """Owners of the texture's pixels up to 16 columns and 4,000 rows away are
+    found by the scan in shared memory, others by the one in global memory:
+    sparse sets whose sites lie further off than either, a dense cluster beside
+    empty space, and a column and a row of sites."""
+    rng = np.random.default_rng(n + fbo)
+    sparse = rng.random((n, 2))
+    cluster = np.concatenate([rng.random((n, 2)) * 0.02, rng.random((5, 2))])
+    column = np.stack([0.5 + 1e-4 * rng.random(n), rng.random(n)], axis=1)
+    row = np.concatenate([column[:, ::-1], [[0.1, 0.1], [0.9, 0.95]]])
+    for pts in (sparse, cluster, np.concatenate([column, [[0.1, 0.2], [0.95, 0.8]]]), row):
+        dt = engine.triangulate(G.GPUDTParams(pts, fboSize=fbo))
+        ok, rep = compare_dt(pts, dt.vtx, dt.tri)
+        assert ok, rep
