@@ -59,3 +59,21 @@ def test_undecided_predicates(engine, n):
     assert dt.status.exactIncircle > 0
     ok, rep = compare_alpha(pts, dt.vtx, dt.tri, engine.alpha_resident(), 4)
     assert ok, rep
+
+
+@pytest.mark.parametrize("n", [302000, 304500])
+def test_vertex_intervals_by_block(engine, n):
+    """Either side of 606,208 triangles, from where a block combines its
+    triangles' contributions to a vertex before they go to global memory; a hub
+    of high degree and a far cluster make vertices that many blocks share."""
+    import numpy as np
+
+    th = np.linspace(0.0, 2.0 * np.pi, 200, endpoint=False)
+    ring = np.stack([np.cos(th), np.sin(th)], axis=1) * 0.3
+    rest = D.uniform_points(n - 201, n) * 2.0 - 1.0
+    rest = rest[np.hypot(rest[:, 0], rest[:, 1]) > 0.31]
+    pts = np.concatenate([ring, [[1e-4, 2e-4]], rest, D.uniform_points(n - 201 - len(rest), n + 1) * 0.01 + 0.9])
+    dt = engine.triangulate(G.GPUDTParams(pts, fboSize=2048))
+    assert (dt.nTris < 606208) == (n < 303000)
+    ok, rep = compare_alpha(pts, dt.vtx, dt.tri, engine.alpha_resident(), 4)
+    assert ok, rep
