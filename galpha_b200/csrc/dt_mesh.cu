@@ -671,8 +671,8 @@ int stage_shift(Ctx &c)
                     launch_dev(c, ShiftCheckTris{c.tv, c.pos, c.opos, cand, drop, cur, curn, ct}, &ct->ntris,
                                c.cap_tris);
                 else
-                    launch_dev(c, ShiftCheckFans{c.tv, c.tn, c.vtri, c.pos, c.opos, cand, prev, drop, cur, curn, ct},
-                               prevn, c.V);
+                    launch_spread(c, ShiftCheckFans{c.tv, c.tn, c.vtri, c.pos, c.opos, cand, prev, drop, cur, curn, ct},
+                                  prevn, c.V);
                 launch_dev(c, ShiftDropList{cur, cand, drop, dropped, &ct->sh_total, c.N, ct}, curn, c.V,
                            Clears{{&ct->r_drop[ring(it + kRing / 2)]}});
             }
@@ -723,9 +723,9 @@ int stage_shift(Ctx &c)
             const int round = next_round(c);
             // a round selects at most the bad sites left (the grid is sized by them:
             // an empty round of this local-memory-heavy kernel then stays cheap)
-            launch_dev(c, BadRemove{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.anchor, c.list, c.pos,
-                                    c.vstate, c.rec, nrec, round, c.N, ct},
-                       nsel, badCount);
+            launch_spread(c, BadRemove{c.tv, c.tn, c.fwd, c.epoch, c.freelist, c.vtri, c.anchor, c.list, c.pos,
+                                       c.vstate, c.rec, nrec, round, c.N, ct},
+                          nsel, badCount);
             launch_dev(c, Relinker{c.tn, c.fwd, c.epoch, c.rec, c.tv, c.vtri, round, ct}, nrec, recn);
             c.rec_round++;
         }
