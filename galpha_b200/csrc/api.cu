@@ -311,7 +311,7 @@ static int mesh_stages(Ctx &c)
             int to = s;
             while (to < kSmFlip && one[to + 1] && !(to == kSmBoundary && c.n_cons > 0)) to++;
             r = stage_small(c, s, to, &next);
-            if (r) return stage_fail(c, r, to > s ? "mesh" : stage);
+            if (r) return stage_fail(c, r, s == kSmShift && next == s ? "links" : to > s ? "mesh" : stage);
             for (int k = s; k < next; k++) c.small_mesh |= 1u << k;
             if (next <= to) one[next] = false;  // too many missing sites for it
             for (int k = s; k < next; k++) c.reads_at[4 + k] = c.host_reads;

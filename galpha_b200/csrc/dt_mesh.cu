@@ -218,8 +218,16 @@ int stage_links(Ctx &c)
     launch_n(c, FillInc{c.tv, start, deg, inc}, nt);
     launch_n(c, MatchLinks{c.tv, c.tn, start, inc, c.vtri, c.ctr}, nt);
     GALPHA_CUDA(cudaGetLastError());
+    // the launch that runs the next stages of a small mesh makes the check itself
+    // before anything else (a read costs it 11 us here)
+    if (c.V <= kSmShiftV) return GPUDT_OK;
     r = read_counters(c);
     if (r) return r;
+    return links_result(c);
+}
+
+int links_result(Ctx &c)
+{
     if (c.hctr->err) return c.hctr->err;
     // the only hull edges are the F edges of the fake ring
     if (c.hctr->nhull != c.F) {

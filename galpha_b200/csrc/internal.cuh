@@ -553,6 +553,7 @@ int stage_setup(Ctx &c, const double *d_xy, int n, double minX, double minY, dou
 int stage_voronoi(Ctx &c, const double *d_xy, bool *empty);
 int stage_triangles(Ctx &c);
 int stage_links(Ctx &c);
+int links_result(Ctx &c);  // the check of the links, from counters read after their launches
 int stage_shift(Ctx &c);
 int stage_missing(Ctx &c);
 int stage_boundary(Ctx &c);

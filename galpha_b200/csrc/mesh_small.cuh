@@ -90,7 +90,9 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
     int shift_rounds = 0, missing_rounds = 0, flip_rounds = 0;
     int *const aux = m.aux, *const aux2 = m.aux2;
 
-    if (next == kSmShift) {
+    // broken links (links_result) reach no stage
+    if (next == kSmShift && (rd(&ct->err) || rd(&ct->nhull) != m.F)) bad = -1;
+    if (next == kSmShift && !bad) {
         if (lead) ct->sm_ns[0] = global_ns();
         {
             int8_t *cand = (int8_t *)m.list2;
@@ -459,9 +461,10 @@ int stage_small(Ctx &c, int from, int to, int *next)
     const Counters &h = *c.hctr;
     c.round_counter = std::max(c.round_counter, h.sm_round);
     c.rec_round = h.sm_rec;
+    *next = h.sm_next;
+    if (from == kSmShift && h.sm_next == kSmShift && (r = links_result(c))) return r;
     if (h.err) return h.err;
     if (h.ntris > c.cap_tris) return GPUDT_ERR_NOMEM;
-    *next = h.sm_next;
     for (int s = from; s < h.sm_next; s++) c.small_ms[s] = (float)((double)(h.sm_ns[s + 1] - h.sm_ns[s]) * 1e-6);
     if (from <= kSmShift) {
         c.st.shiftRounds = h.sm_shift;
