@@ -31,15 +31,16 @@ constexpr int kTailEnterDefault = 4096, kTailLeaveDefault = 32768;
 // Mesh stages that one launch can run in a row (mesh_small.cuh), and up to
 // which size each of them does.  Stage times in us, in one launch against
 // launches of its own (uniform points unless said otherwise, B200):
-//   shift     109 / 256 at 12,000 points, 288 / 395 at 200,000, 350 / 390 at
-//             400,000, but 873 / 764 at 400,000 clustered
-//   missing   41 / 79 at 12,000, 66 / 132 at 100,000, but 333 / 244 at 55,000
+//   shift     111 / 216 at 12,000 points, 285 / 321 at 200,000 (669 / 603
+//             clustered), 445 / 442 at 1,000,000 (797 / 778)
+//   missing   39 / 76 at 12,000, 62 / 121 at 100,000, but 333 / 244 at 55,000
 //             clustered, about 14,000 sites: more than kSmMissLimit sites want
 //             the whole GPU
-//   boundary  198 / 343 at 12,000, 287 / 397 at 100,000, 467 / 493 at 1,000,000
-//             (1,024 ring sites), but 743 / 645 at 4,000,000 (2,048 sites, long
-//             fans)
-//   flip      85 / 124 at 12,000, 108 / 136 at 25,000, but 170 / 154 at 40,000
+//   boundary  189 / 293 at 12,000, 269 / 369 at 100,000, 465 / 580 at 1,000,000
+//             (1,024 ring sites; 410 / 704 clustered), but 743 / 645 at
+//             4,000,000 (2,048 sites, long fans; before the runs of the whole
+//             ring)
+//   flip      62 / 106 at 12,000, 90 / 106 at 25,000, but 126 / 113 at 40,000
 enum { kSmShift = 0, kSmMissing = 1, kSmBoundary = 2, kSmFlip = 3 };
 constexpr int kSmShiftV = 262144, kSmMissLimit = 8192, kSmBoundaryF = 1024, kSmBoundaryFSmall = 4096, kSmFlipV = 28672;
 constexpr int kMaxGroup = 8;   // rounds between two counter reads
