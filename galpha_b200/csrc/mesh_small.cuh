@@ -10,10 +10,10 @@
 // barrier (whose blocks are resident together by construction, so nothing
 // spins), and the loop conditions are read on the device.  The mesh may differ
 // from the launched stages' only where two launched runs may differ.  A call of
-// 1,000 points takes 0.66 ms, with launched stages 0.97; 12,000 points 0.90 and
-// 1.30 (sizes up to which each stage is run this way: kSmShiftV and below).
+// 12,000 points takes 0.80 ms, with launched stages 1.12; 100,000 points 1.15 and
+// 1.41 (sizes up to which each stage is run this way: kSmShiftV and below).
 // What bounds it is the latency of the phases' gathers, and of one warp's chain
-// of triangles in fake removal (0.15 of 0.21 ms at 1,000 points); 16 blocks of
+// of triangles in fake removal (0.12 of 0.23 ms at 1,000 points); 16 blocks of
 // 512 threads hide it for up to some 10,000 items per phase.
 //
 // Every thread must take the same branches, so a counter word that decides one
