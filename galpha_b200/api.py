@@ -172,6 +172,7 @@ def load(path=None):
     L.galphaBatchSets.argtypes = [vp, vp]
     L.galphaSetBatchDensity.argtypes = [vp, ctypes.c_double]
     L.galphaSetSchedule.argtypes = [vp, ip, ip, ip, ip, ip]
+    L.galphaSetClusterLimit.argtypes = [vp, ip]
     L.galphaGetSchedule.argtypes = [vp, ctypes.POINTER(ip)]
     L.galphaBatchCopy.argtypes = [vp, vp, vp, vp, vp, vp]
     L.galphaBatchQuery.argtypes = [vp, vp, ip, vp]
@@ -496,6 +497,12 @@ class Engine:
         flip_tail_enter) keeps the default.  Tuned by galpha_b200.autotune."""
         _check(self._L.galphaSetSchedule(self._h, int(shift_group), int(missing_group), int(flip_sync),
                                          int(flip_tail_enter), int(flip_tail_leave)), "galphaSetSchedule")
+
+    def set_cluster_limit(self, max_blocks=-1):
+        """Largest thread-block cluster that runs the mesh stages of a small mesh
+        in one launch (galphaSetClusterLimit; default 16).  0: each stage always
+        runs as launches of its own.  No value changes a result."""
+        _check(self._L.galphaSetClusterLimit(self._h, int(max_blocks)), "galphaSetClusterLimit")
 
     def schedule(self):
         """The schedule in force, as a dict (galphaGetSchedule)."""

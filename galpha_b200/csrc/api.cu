@@ -296,12 +296,13 @@ int stage_fail(Ctx &c, int r, const char *stage)
 }
 
 // Shifting to flipping: each stage as launches of its own, or, while the mesh
-// is small for that stage, in one launch with its neighbours.
+// is small for that stage and the device can place the cluster that it takes,
+// in one launch with its neighbours.
 static int mesh_stages(Ctx &c)
 {
     static const char *const names[] = {"shift", "missing", "boundary", "flip"};
-    const bool few = c.V <= kSmShiftV;
-    bool one[] = {few, few, c.F <= (few ? kSmBoundaryFSmall : kSmBoundaryF), c.V <= kSmFlipV};
+    const bool fits = small_mesh_fits(c), few = shift_in_one(c);
+    bool one[] = {few, few, fits && c.F <= (few ? kSmBoundaryFSmall : kSmBoundaryF), fits && c.V <= kSmFlipV};
     c.small_mesh = 0;
     int r;
     for (int s = kSmShift; s <= kSmFlip;) {
@@ -697,6 +698,14 @@ int galphaGetSchedule(galphaHandle h, int *out5)
     out5[2] = c.flip_sync;
     out5[3] = c.tail_enter;
     out5[4] = c.tail_leave;
+    return GPUDT_OK;
+}
+
+int galphaSetClusterLimit(galphaHandle h, int maxBlocks)
+{
+    if (!h || maxBlocks > kSmMaxBlocks) return GPUDT_ERR_ARG;
+    std::lock_guard<std::mutex> lk(h->mu);
+    h->H.c.sm_limit = maxBlocks >= 0 ? maxBlocks : kSmMaxBlocks;
     return GPUDT_OK;
 }
 

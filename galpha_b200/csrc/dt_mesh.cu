@@ -220,7 +220,7 @@ int stage_links(Ctx &c)
     GALPHA_CUDA(cudaGetLastError());
     // the launch that runs the next stages of a small mesh makes the check itself
     // before anything else (a read costs it 11 us here)
-    if (c.V <= kSmShiftV) return GPUDT_OK;
+    if (shift_in_one(c)) return GPUDT_OK;
     r = read_counters(c);
     if (r) return r;
     return links_result(c);

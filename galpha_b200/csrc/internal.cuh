@@ -42,6 +42,7 @@ constexpr int kTailEnterDefault = 4096, kTailLeaveDefault = 32768;
 //             ring)
 //   flip      62 / 106 at 12,000, 90 / 106 at 25,000, but 126 / 113 at 40,000
 enum { kSmShift = 0, kSmMissing = 1, kSmBoundary = 2, kSmFlip = 3 };
+constexpr int kSmMaxBlocks = 16;  // largest cluster
 constexpr int kSmShiftV = 262144, kSmMissLimit = 8192, kSmBoundaryF = 1024, kSmBoundaryFSmall = 4096, kSmFlipV = 28672;
 constexpr int kMaxGroup = 8;   // rounds between two counter reads
 // Per-round counts live in rings of kRing words: round k counts in word
@@ -235,6 +236,8 @@ struct Ctx {
     unsigned char *longfan = nullptr;  // small meshes: a fan too long for shared memory, per block
     float small_ms[4] = {0, 0, 0, 0};  // small meshes: shift, missing, boundary, flip times on the device
     unsigned small_mesh = 0;           // stages the current call ran that way (bit kSm*)
+    int sm_fit = -1;                   // largest cluster the device places for it (-1: not asked yet, 0: none)
+    int sm_limit = kSmMaxBlocks;       // largest cluster allowed (galphaSetClusterLimit)
 
     DevBuf bufs[64];
     int nbufs = 0;
@@ -561,6 +564,8 @@ int stage_boundary(Ctx &c);
 int stage_flip(Ctx &c);
 int stage_constraints(Ctx &c);
 int stage_small(Ctx &c, int from, int to, int *next);  // stages kSm* in one launch
+bool small_mesh_fits(Ctx &c);  // whether that launch's cluster can be placed
+inline bool shift_in_one(Ctx &c) { return c.V <= kSmShiftV && small_mesh_fits(c); }
 size_t small_mesh_scratch_bytes();
 int stage_compact(Ctx &c);
 // ------------------------------------------------------------------ batches

@@ -23,7 +23,6 @@
 namespace galpha {
 
 constexpr int kSmThreads = 512;   // per block: 128 registers per thread
-constexpr int kSmMaxBlocks = 16;  // largest cluster
 constexpr int kSmFrWarps = 8;     // warps per block that remove fakes (shared memory)
 constexpr int kSmPerBlock = 256;  // vertices per block
 
@@ -379,20 +378,56 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
     }
 }
 
+constexpr size_t kSmSmem = kSmFrWarps * fake_remove_smem(kMaxChain);
+
+// Launch of one cluster of `blocks` blocks; at: filled in for it.
+static cudaLaunchConfig_t small_mesh_config(const Ctx &c, int blocks, cudaLaunchAttribute *at)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kSmThreads);
+    cfg.dynamicSmemBytes = kSmSmem;
+    cfg.stream = c.stream;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = blocks;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+static int small_mesh_blocks(int V)
+{
+    int blocks = 1;
+    while (blocks < kSmMaxBlocks && blocks * kSmPerBlock < V) blocks *= 2;
+    return blocks;
+}
+
+// A block takes a whole SM, so a mesh of over 2,048 vertices needs 16 free ones
+// in one GPC, which a whole B200 has and a part of one need not: the device is
+// asked once per handle, and where the mesh's cluster does not fit (or is
+// larger than allowed) the stages run as launches of their own.
+bool small_mesh_fits(Ctx &c)
+{
+    if (c.sm_fit < 0) {
+        cudaFuncSetAttribute(k_mesh_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmSmem);
+        const bool large =
+            cudaFuncSetAttribute(k_mesh_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        int fit = large ? kSmMaxBlocks : 8;
+        for (; fit > 0; fit /= 2) {
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = small_mesh_config(c, fit, at);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_mesh_small, &cfg) == cudaSuccess && clusters > 0) break;
+        }
+        cudaGetLastError();  // an answer "cannot" is no error of the call
+        c.sm_fit = fit;
+    }
+    return small_mesh_blocks(c.V) <= std::min(c.sm_fit, c.sm_limit);
+}
+
 static int launch_mesh_small(Ctx &c, int from, int to)
 {
-    const int smem = (int)(kSmFrWarps * fake_remove_smem(kMaxChain));
-    {
-        static std::mutex mu;
-        static bool attr_set[64];
-        const int dv = c.device >= 0 && c.device < 64 ? c.device : 0;
-        std::lock_guard<std::mutex> lk(mu);
-        if (!attr_set[dv]) {
-            GALPHA_CUDA(cudaFuncSetAttribute(k_mesh_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            GALPHA_CUDA(cudaFuncSetAttribute(k_mesh_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            attr_set[dv] = true;
-        }
-    }
     SmallMesh m{};
     m.opos = c.opos;
     m.pos = c.pos;
@@ -431,19 +466,8 @@ static int launch_mesh_small(Ctx &c, int from, int to)
     m.from = from;
     m.to = to;
     m.miss_limit = kSmMissLimit;
-    int blocks = 1;
-    while (blocks < kSmMaxBlocks && blocks * kSmPerBlock < c.V) blocks *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kSmThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = c.stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = blocks;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = small_mesh_config(c, small_mesh_blocks(c.V), at);
     GALPHA_CUDA(cudaLaunchKernelEx(&cfg, k_mesh_small, m));
     count_launch();
     return GPUDT_OK;

@@ -295,6 +295,18 @@ int galphaSetSchedule(galphaHandle h, int shiftGroup, int missingGroup, int flip
                       int flipTailLeave);
 int galphaGetSchedule(galphaHandle h, int *out5);
 
+/* The mesh stages of a small mesh (shifting and missing sites up to 262,144
+ * vertices, ring sites included, the fake ring up to 1,024 sites, flips up to
+ * 28,672 vertices) run as one launch of one thread-block cluster of up to 16
+ * blocks, a whole SM each; they run as launches of their own where the device
+ * cannot place the cluster that the mesh takes (one block per 256 vertices,
+ * rounded up to a power of two).  maxBlocks (0..16; negative restores 16)
+ * lowers the largest cluster of the handle's later calls; 0: always launches
+ * of their own, which is also where the loop schedule above has an effect.  No
+ * value changes a result; above 16: GPUDT_ERR_ARG.  No counterpart in the
+ * reference. */
+int galphaSetClusterLimit(galphaHandle h, int maxBlocks);
+
 /* Text of the last error on the calling thread (cleared when a compute call
  * -- RunDevice, Triangulate, Compute*, RunBatch*, gpudtComputeDTEx -- starts). */
 const char *galphaLastError(void);
