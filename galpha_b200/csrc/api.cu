@@ -314,14 +314,14 @@ static int mesh_stages(Ctx &c)
             r = stage_small(c, s, to, &next);
             if (r) return stage_fail(c, r, s == kSmShift && next == s ? "links" : to > s ? "mesh" : stage);
             for (int k = s; k < next; k++) c.small_mesh |= 1u << k;
-            if (next <= to) one[next] = false;  // too many missing sites for it
+            if (next <= to) one[next] = false;  // too many missing sites or exact tests for it
             for (int k = s; k < next; k++) c.reads_at[4 + k] = c.host_reads;
         } else {
             r = s == kSmShift ? stage_shift(c) : s == kSmMissing ? stage_missing(c) : s == kSmBoundary ? stage_boundary(c)
                                                                                                   : stage_flip(c);
             if (r) return stage_fail(c, r, stage);
         }
-        if (next == kSmFlip) {
+        if (s < kSmFlip && next == kSmFlip) {
             r = stage_constraints(c);
             if (r) return stage_fail(c, r, "constraints");
         }

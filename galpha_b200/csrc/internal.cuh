@@ -124,6 +124,7 @@ struct Counters {
     int sm_next;     // first stage not run
     int sm_rec;      // words of r_rec taken so far
     int sm_round;    // last operation round id
+    int sm_hard;     // flips: looked-at triangles with an edge that the filters leave undecided
     int sm_shift, sm_missing, sm_flip;  // rounds run
     unsigned long long sm_ns[5];        // device time at the start of shift, missing, boundary, flip, and at the end
     // predicate stage counts, each spread over 64 counters (one per warp id mod

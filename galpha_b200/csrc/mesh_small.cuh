@@ -58,6 +58,23 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
+// Whether the filters leave an edge of triangle t undecided.
+__device__ __forceinline__ bool flip_undecided(const int4 *tv, const int4 *tn, const double2 *pos, int t)
+{
+    const int4 v = tv[t];
+    if (v.x < 0) return false;
+    const int4 n = tn[t];
+    bool hard = false;
+    for (int i = 0; i < 3; i++) {
+        const int e = geti(n, i);
+        if (e < 0) continue;
+        int n64 = 0;
+        hard |= incircle_fast(pos[geti(v, p1(i))], pos[geti(v, m1(i))], pos[geti(v, i)],
+                              pos[geti(tv[dtri(e)], dori(e))], &n64) == 2;
+    }
+    return hard;
+}
+
 __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
 {
     extern __shared__ __align__(16) unsigned char sm_mem[];
@@ -302,13 +319,30 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
         }
         next = kSmFlip;
     }
+    bool exact = false;
     if (next == kSmFlip && m.to >= kSmFlip && !bad) {
         if (lead) ct->sm_ns[3] = global_ns();
         const int nt = rd(&ct->ntris);
         int2 *st = m.stage;
-        int2 *cands = (int2 *)m.inc;
         each(nt, FlipInit{m.tv, st, m.vote, m.list, &ct->r_act[0]});
+        // Exact tests are arithmetic, some 80 us each on coordinates that are no
+        // multiples of a power of two, and want the whole GPU when there are more
+        // of them than threads here (a lattice of spacing 1/3: 8,100 points 177
+        // us, now 85; 25,600 points 663, now 112): each thread looks at one
+        // triangle of an even spread (2.5 us), and by their share the flips are
+        // handed back to launches.
+        if (nt > nthr) {
+            const bool hard = flip_undecided(m.tv, m.tn, m.pos, (int)((long long)tid * nt / nthr));
+            const unsigned b = __ballot_sync(0xffffffffu, hard);
+            if (lane == 0 && b) atomicAdd(&ct->sm_hard, __popc(b));
+        }
         cluster_barrier();
+        exact = (long long)rd(&ct->sm_hard) * nt > (long long)nthr * nthr;
+        if (exact && lead) ct->r_act[0] = 0;
+    }
+    if (next == kSmFlip && m.to >= kSmFlip && !bad && !exact) {
+        int2 *st = m.stage;
+        int2 *cands = (int2 *)m.inc;
         FlipCheck ck{m.tv, m.tn, m.pos, nullptr, st, m.vote, cands, nullptr, ct, m.chash, m.cmask};
         FlipApply ap{m.tv, m.tn, st, m.vote, nullptr, nullptr, cands, m.rec, 0, ct, false, nullptr, nullptr, 3ll * m.cap};
         FlipRelink rl{m.tn, st, m.rec, 0};
@@ -474,8 +508,8 @@ static int launch_mesh_small(Ctx &c, int from, int to)
 }
 
 // Runs the stages `from` .. `to` in one launch and one counter read; *next is
-// the first stage that has not been run (to + 1, or kSmMissing when there are
-// too many missing sites).
+// the first stage that has not been run (to + 1; kSmMissing when there are too
+// many missing sites; kSmFlip when there are too many exact tests).
 int stage_small(Ctx &c, int from, int to, int *next)
 {
     int r = launch_mesh_small(c, from, to);

@@ -74,6 +74,28 @@ def test_alpha_after_launched_stages(limited):
         assert ok, rep
 
 
+@pytest.mark.parametrize("side,spacing,launched", [(60, 3.0, False), (66, 3.0, True), (120, 3.0, True), (120, 1.0, True)])
+def test_flips_with_many_exact_tests(engine, side, spacing, launched):
+    """A lattice leaves an edge of every triangle to the exact in-circle test: with
+    more triangles than the cluster has threads (8,192) the flips are handed back
+    to launches.  With constraints they are handed back after those."""
+    g = np.stack(np.meshgrid(np.arange(float(side)), np.arange(float(side))), axis=-1).reshape(-1, 2) / spacing
+    for cons in (None, np.array([[0, side * (side - 1) + 1], [side - 1, side * (side - 1) + side - 2]], np.int32)):
+        dt = engine.triangulate(G.GPUDTParams(g, fboSize=1024, constraints=cons))
+        if cons is None:
+            assert (dt.status.hostReadsStage[FLIP] >= 1) == launched
+            ok, rep = compare_dt(g, dt.vtx, dt.tri)
+            assert ok, rep
+            assert dt.status.exactIncircle >= (side - 1) ** 2  # a diagonal per cell
+        else:
+            v = np.concatenate([dt.vtx[:, [0, 1]], dt.vtx[:, [1, 2]], dt.vtx[:, [2, 0]]])
+            edges = set(map(tuple, v.tolist())) | set(map(tuple, v[:, ::-1].tolist()))
+            assert all(tuple(c) in edges for c in cons.tolist())
+            assert dt.nTris == 2 * side * side - 2 - 4 * (side - 1)
+    pts = D.uniform_points(12000, 4)  # the same size, nothing undecided
+    assert engine.triangulate(G.GPUDTParams(pts, fboSize=512)).status.hostReadsStage[FLIP] == 0
+
+
 def test_limit_out_of_range(engine):
     with pytest.raises(G.GpudtError):
         engine.set_cluster_limit(17)
