@@ -302,7 +302,7 @@ static int mesh_stages(Ctx &c)
 {
     static const char *const names[] = {"shift", "missing", "boundary", "flip"};
     const bool fits = small_mesh_fits(c), few = shift_in_one(c);
-    bool one[] = {few, few, fits && c.F <= (few ? kSmBoundaryFSmall : kSmBoundaryF), fits && c.V <= kSmFlipV};
+    bool one[] = {few, few, fits && c.F <= (c.V <= kSmBoundaryV ? kSmBoundaryFSmall : kSmBoundaryF), fits && c.V <= kSmFlipV};
     c.small_mesh = 0;
     int r;
     for (int s = kSmShift; s <= kSmFlip;) {

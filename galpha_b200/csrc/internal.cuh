@@ -31,19 +31,29 @@ constexpr int kTailEnterDefault = 4096, kTailLeaveDefault = 32768;
 // Mesh stages that one launch can run in a row (mesh_small.cuh), and up to
 // which size each of them does.  Stage times in us, in one launch against
 // launches of its own (uniform points unless said otherwise, B200):
-//   shift     111 / 216 at 12,000 points, 285 / 321 at 200,000 (669 / 603
-//             clustered), 445 / 442 at 1,000,000 (797 / 778)
+//   shift     92 / 198 at 16,000 points, 225 / 303 at 140,000, 277 / 312 at
+//             200,000; where many sites are left to the priority rounds (16
+//             pixels per point and less: blobs, a small texture) the rounds
+//             want the whole GPU sooner: 457 / 447 at 140,000 (64 blobs of
+//             sigma 0.01, 4,200 unshiftable sites), 632 / 579 at 200,000, 658 /
+//             577 at 220,000.  With the links' read and the missing sites, which
+//             go along, ten kinds of sets are 24 to 155 us faster or even up
+//             to 180,000 points but for the blobs (25 us behind at worst); from
+//             200,000 on three of ten, from 220,000 on seven are slower, by up
+//             to 79 us
 //   missing   39 / 76 at 12,000, 62 / 121 at 100,000, but 333 / 244 at 55,000
 //             clustered, about 14,000 sites: more than kSmMissLimit sites want
 //             the whole GPU
 //   boundary  189 / 293 at 12,000, 269 / 369 at 100,000, 465 / 580 at 1,000,000
-//             (1,024 ring sites; 410 / 704 clustered), but 743 / 645 at
+//             (1,024 ring sites; 410 / 704 clustered), at 240,000 371 / 413
+//             with 2,048 sites and 403 / 445 with 4,096, but 743 / 645 at
 //             4,000,000 (2,048 sites, long fans; before the runs of the whole
 //             ring)
 //   flip      62 / 106 at 12,000, 90 / 106 at 25,000, but 126 / 113 at 40,000
 enum { kSmShift = 0, kSmMissing = 1, kSmBoundary = 2, kSmFlip = 3 };
 constexpr int kSmMaxBlocks = 16;  // largest cluster
-constexpr int kSmShiftV = 262144, kSmMissLimit = 8192, kSmBoundaryF = 1024, kSmBoundaryFSmall = 4096, kSmFlipV = 28672;
+constexpr int kSmShiftV = 196608, kSmMissLimit = 8192, kSmFlipV = 28672;
+constexpr int kSmBoundaryF = 1024, kSmBoundaryV = 262144, kSmBoundaryFSmall = 4096;  // any mesh; meshes up to that size
 constexpr int kMaxGroup = 8;   // rounds between two counter reads
 // Per-round counts live in rings of kRing words: round k counts in word
 // k mod kRing and clears the word of round k + kRing / 2, so that the words of

@@ -295,9 +295,9 @@ int galphaSetSchedule(galphaHandle h, int shiftGroup, int missingGroup, int flip
                       int flipTailLeave);
 int galphaGetSchedule(galphaHandle h, int *out5);
 
-/* The mesh stages of a small mesh (shifting and missing sites up to 262,144
- * vertices, ring sites included, the fake ring up to 1,024 sites, flips up to
- * 28,672 vertices) run as one launch of one thread-block cluster of up to 16
+/* The mesh stages of a small mesh (shifting and missing sites up to 196,608
+ * vertices, ring sites included, the fake ring up to 1,024 sites, or 4,096 up
+ * to 262,144 vertices, flips up to 28,672 vertices) run as one launch of one thread-block cluster of up to 16
  * blocks, a whole SM each; they run as launches of their own where the device
  * cannot place the cluster that the mesh takes (one block per 256 vertices,
  * rounded up to a power of two).  maxBlocks (0..16; negative restores 16)

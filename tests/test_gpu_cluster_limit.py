@@ -96,6 +96,16 @@ def test_flips_with_many_exact_tests(engine, side, spacing, launched):
     assert engine.triangulate(G.GPUDTParams(pts, fboSize=512)).status.hostReadsStage[FLIP] == 0
 
 
+# 256 ring sites: 196,608 vertices is the last size that shifts in the one launch
+@pytest.mark.parametrize("n,one", [(196352, True), (196353, False)])
+def test_shift_size_limit(engine, n, one):
+    pts = D.gaussian_blobs(n, 9, nblobs=64, sigma=0.01)
+    dt = engine.triangulate(G.GPUDTParams(pts, fboSize=1024))
+    reads = list(dt.status.hostReadsStage)
+    assert (reads[SHIFT] == 1) == one and reads[BOUNDARY] == 1  # the fake ring is in one launch either way
+    assert canon_set(dt.vtx) == canon_set(O.dt(pts)[0])
+
+
 def test_limit_out_of_range(engine):
     with pytest.raises(G.GpudtError):
         engine.set_cluster_limit(17)
