@@ -165,7 +165,6 @@ static size_t plan(const Sizes &z, Ctx *c, Arena *A)
     TAKE(outtri, gpudtTriangle, cap);
     TAKE(edge_aos, galphaEdgeInterval, 2 * cap);
     TAKE(qclass, uint8_t, V + 3 * cap);
-    TAKE(longfan, unsigned char, small_mesh_scratch_bytes());
     TAKE(ctr, Counters, 1);
 #undef TAKE
     return total + 4096;

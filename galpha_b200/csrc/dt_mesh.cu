@@ -2953,11 +2953,6 @@ int stage_constraints(Ctx &c)
 
 namespace galpha {
 
-size_t small_mesh_scratch_bytes()
-{
-    return kSmMaxBlocks * fake_remove_smem(kMaxFanLong);
-}
-
 // ----------------------------------------------------------------- compact
 struct MarkAlive {
     const int4 *tv;

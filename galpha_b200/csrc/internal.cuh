@@ -244,7 +244,6 @@ struct Ctx {
     bool outtri_ready = false;          // outtri holds the current mesh (built on the first download)
     bool want_outtri = false;           // this call needs outtri: compaction writes it directly
     galphaEdgeInterval *edge_aos = nullptr;  // [2*cap] edge records for download
-    unsigned char *longfan = nullptr;  // small meshes: a fan too long for shared memory, per block
     float small_ms[4] = {0, 0, 0, 0};  // small meshes: shift, missing, boundary, flip times on the device
     unsigned small_mesh = 0;           // stages the current call ran that way (bit kSm*)
     int sm_fit = -1;                   // largest cluster the device places for it (-1: not asked yet, 0: none)
@@ -577,7 +576,6 @@ int stage_constraints(Ctx &c);
 int stage_small(Ctx &c, int from, int to, int *next);  // stages kSm* in one launch
 bool small_mesh_fits(Ctx &c);  // whether that launch's cluster can be placed
 inline bool shift_in_one(Ctx &c) { return c.V <= kSmShiftV && small_mesh_fits(c); }
-size_t small_mesh_scratch_bytes();
 int stage_compact(Ctx &c);
 // ------------------------------------------------------------------ batches
 // One point set of a batch: its grid scaling, its texture cell and its

@@ -26,6 +26,14 @@ constexpr int kSmThreads = 512;   // per block: 128 registers per thread
 constexpr int kSmFrWarps = 8;     // warps per block that remove fakes (shared memory)
 constexpr int kSmPerBlock = 256;  // vertices per block
 
+// The stored fans of a round are disjoint, fewer entries than triangle slots,
+// so the long ones (over kMaxChain) find room, each at its own place, in an
+// array of two edge records per slot that the mesh stages leave idle.
+constexpr int kSmFanBytes = 42;
+static_assert((size_t)kSmFanBytes * (kMaxChain + 1) >= fake_remove_smem(kMaxChain + 1) + 15, "a place holds its fan");
+static_assert((size_t)kSmFanBytes * kMaxFanLong >= fake_remove_smem(kMaxFanLong) + 15, "a place holds its fan");
+static_assert(kSmFanBytes <= 2 * sizeof(galphaEdgeInterval), "the array holds every place");
+
 struct SmallMesh {
     // arrays of Ctx
     double2 *opos, *pos;
@@ -36,7 +44,8 @@ struct SmallMesh {
     Relink *rec;
     int2 *stage;      // fake runs: staged fan entries; flips: the triangles' states
     int *rec5;        // fake runs: records
-    unsigned char *longfan;  // fake_remove_smem(kMaxFanLong) bytes per block
+    unsigned char *longfan;  // fans too long for shared memory, each at kSmFanBytes times its place in the store
+    long long longfan_bytes;
     const unsigned long long *chash;
     unsigned cmask;
     Counters *ct;
@@ -254,9 +263,13 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
                 if (warp == 0)  // fans too long for the shared arrays
                     for (int item = cta; item < n; item += ncta) {
                         const int d = fanlen[item] & 0xffff;
-                        if (d > kMaxChain)
-                            fake_remove_item(fr, item, kMaxFanLong, m.longfan + cta * fake_remove_smem(kMaxFanLong),
-                                             s_fr[0]);
+                        if (d > kMaxChain) {
+                            const long long at = ((long long)kSmFanBytes * fanoff[item] + 15) & ~15ll;
+                            if (at + (long long)fake_remove_smem(d) <= m.longfan_bytes)
+                                fake_remove_item(fr, item, d, m.longfan + at, s_fr[0]);
+                            else if (lane == 0)
+                                set_err(ct, GPUDT_ERR_TOPOLOGY, 76);  // the fans overlap: a broken mesh
+                        }
                         __syncwarp();
                     }
                 cluster_barrier();
@@ -484,7 +497,8 @@ static int launch_mesh_small(Ctx &c, int from, int to)
     m.rec = c.rec;
     m.stage = (int2 *)c.keys2;  // alpha-stage buffers, idle until the mesh is final
     m.rec5 = (int *)c.spectrum;
-    m.longfan = c.longfan;
+    m.longfan = (unsigned char *)c.edge_aos;  // idle until an alpha result is downloaded
+    m.longfan_bytes = 2ll * c.cap_tris * (long long)sizeof(galphaEdgeInterval);
     m.chash = c.chash;
     m.cmask = c.cmask;
     m.ct = c.ctr;
