@@ -582,6 +582,9 @@ static int handle_init(galpha_ctx *h, int device, long long budget)
     }
     GALPHA_CUDA(cudaMalloc(&c.scan_buf, kScanBufBytes));
     GALPHA_CUDA(cudaMemsetAsync(c.scan_buf, 0, kScanBufBytes, c.stream));
+    // the first scan may run on a caller's stream (galphaSetStream), which is not
+    // ordered after this one, and would take words of an earlier handle for its own
+    GALPHA_CUDA(cudaStreamSynchronize(c.stream));
     for (int k = 0; k < GALPHA_STAGE_TOTAL + 2; k++) GALPHA_CUDA(cudaEventCreate(&c.ev[k]));
     for (int k = 0; k < 10; k++) GALPHA_CUDA(cudaEventCreate(&c.kev[k]));
     c.events = true;
