@@ -321,6 +321,8 @@ static int mesh_stages(Ctx &c)
             if (r) return stage_fail(c, r, stage);
         }
         if (s < kSmFlip && next == kSmFlip) {
+            if ((c.small_mesh >> kSmBoundary) & 1u && c.events)
+                cudaEventRecord(c.ev[GALPHA_STAGE_BOUNDARY], c.stream);  // what the launch does not time: the constraints
             r = stage_constraints(c);
             if (r) return stage_fail(c, r, "constraints");
         }
@@ -480,6 +482,8 @@ static void fill_times(Ctx &c, int last)
         float ms = 0.f;
         if (k >= 3 && k < 7 && ((c.small_mesh >> (k - 3)) & 1u)) {  // inside a launch: the device's own clock
             c.st.ms[k] = c.small_ms[k - 3];
+            if (k == GALPHA_STAGE_BOUNDARY && c.chash && cudaEventElapsedTime(&ms, c.ev[k], c.ev[k + 1]) == cudaSuccess)
+                c.st.ms[k] += ms;  // constraints belong to this stage
             c.st.hostReadsStage[k] = c.reads_at[k + 1] - c.reads_at[k];
             continue;
         }

@@ -62,7 +62,7 @@ typedef struct galpha_ctx *galphaHandle;
 #define GALPHA_STAGE_TRIANGLES 2  /* Voronoi vertices -> triangles + links */
 #define GALPHA_STAGE_SHIFT     3  /* shifting + bad-case removal */
 #define GALPHA_STAGE_MISSING   4  /* missing-site insertion */
-#define GALPHA_STAGE_BOUNDARY  5  /* fake ring removal + hull */
+#define GALPHA_STAGE_BOUNDARY  5  /* fake ring removal + hull + constrained edges */
 #define GALPHA_STAGE_FLIP      6  /* Lawson flipping */
 #define GALPHA_STAGE_COMPACT   7  /* compaction / output layout */
 #define GALPHA_STAGE_ALPHA     8  /* birth times + attached + sort + ranks + intervals */

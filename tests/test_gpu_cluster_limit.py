@@ -96,6 +96,21 @@ def test_flips_with_many_exact_tests(engine, side, spacing, launched):
     assert engine.triangulate(G.GPUDTParams(pts, fboSize=512)).status.hostReadsStage[FLIP] == 0
 
 
+def test_constraint_time_in_the_boundary_stage(engine):
+    """gpudtStatus.ms[boundary] holds the constraints' time too, with the fake
+    ring in the one launch as with launches (some 500 us against 200)."""
+    pts = D.uniform_points(20000, 6)
+    band = np.floor(pts[:, 1] * 141).astype(int)
+    lines = [np.nonzero(band == b)[0] for b in range(4, 140, 12)]
+    lines = [i[np.argsort(pts[i, 0])] for i in lines]
+    cons = np.concatenate([np.stack([i[:-1], i[1:]], axis=1) for i in lines]).astype(np.int32)
+    ms = {}
+    for name, c in (("plain", None), ("constrained", cons)):
+        ms[name] = np.median([engine.triangulate(G.GPUDTParams(pts, fboSize=1024, constraints=c)).status.ms[BOUNDARY]
+                              for _ in range(5)])
+    assert ms["constrained"] > 1.5 * ms["plain"]
+
+
 # 256 ring sites: 196,608 vertices is the last size that shifts in the one launch
 @pytest.mark.parametrize("n,one", [(196352, True), (196353, False)])
 def test_shift_size_limit(engine, n, one):
