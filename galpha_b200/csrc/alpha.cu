@@ -157,7 +157,7 @@ __device__ __noinline__ unsigned attached_hard(const int4 *gv, const int4 *cn, c
 // ahead, and by the wait for earlier tiles: 4 triangles per thread took 0.57
 // ms at 8.0 M triangles, 2 took 0.64, 1 took 0.75, 8 by blocks of 128 took
 // 0.80 (longer chains ahead of the tiles that wait); 0.48 since the exact tests
-// are made after the loop.  Up to kAkFew triangles
+// are made after the loop.  Up to kAkFew triangles per SM (151,552 on 148)
 // there are too few tiles of four to fill the GPU and one per thread is used
 // (2,000 triangles: 20 us with four, 7 with one).  As five launches (edge
 // counts, a scan, keys, a scan over the edges, edge keys from a second gather)
@@ -166,7 +166,7 @@ __device__ __noinline__ unsigned attached_hard(const int4 *gv, const int4 *cn, c
 // edges (30-0) of its tile or of all tiles up to it; fewer than 2^31 edges.
 constexpr int kAkSpinLimit = 1 << 22;
 constexpr int kAkThreads = 256, kAkItemsMany = 4;
-constexpr int kAkFew = 151552;  // 148 SMs x 4 blocks x 256
+constexpr int kAkFew = 4 * kAkThreads;  // triangles per SM: its resident blocks, one each
 constexpr unsigned long long kAkAgg = 1ull << 62, kAkInc = 2ull << 62, kAkVal = (1ull << 62) - 1;
 
 struct AlphaKeysArgs {
@@ -830,10 +830,11 @@ struct EdgeIntervals {
 // atomics), and 1,024 consecutive triangles, which lie together, reach some 650
 // vertices 2,560 times.  A vertex that finds no slot of the table in kEiProbes
 // steps goes to global memory at once.  231 us at 8.0 M triangles.  Below kEiMany
-// triangles, fewer tiles than four per SM, the plain form: its threads all start
-// at once there and the atomics no longer bound it (100,000 triangles: 6 us).
+// triangles per SM (606,208 on 148), fewer tiles than four each, the plain form:
+// its threads all start at once there and the atomics no longer bound it
+// (100,000 triangles: 6 us).
 constexpr int kEiThreads = 256, kEiItems = 4, kEiSlots = 2048, kEiProbes = 4;
-constexpr int kEiMany = 148 * 4 * kEiThreads * kEiItems;
+constexpr int kEiMany = 4 * kEiThreads * kEiItems;  // triangles per SM
 
 __global__ void __launch_bounds__(kEiThreads) k_edge_intervals(EdgeIntervals f, int nT)
 {
@@ -871,7 +872,7 @@ __global__ void __launch_bounds__(kEiThreads) k_edge_intervals(EdgeIntervals f, 
 
 static void launch_edge_intervals(Ctx &c, const EdgeIntervals &f, int nT)
 {
-    if (nT < kEiMany) {
+    if (nT < kEiMany * c.sm_count) {
         launch_n(c, f, nT);
         return;
     }
@@ -1209,7 +1210,7 @@ int stage_alpha(Ctx &c, AlphaSegs *segs)
     // an alpha call on a resident mesh starts without the error of an earlier
     // failed alpha call and with its own counts
     GALPHA_CUDA(cudaMemsetAsync(&c.ctr->err, 0, kAlphaBytes, c.stream));
-    const bool few = nT <= kAkFew;
+    const bool few = nT <= kAkFew * c.sm_count;
     const int tile = kAkThreads * (few ? 1 : kAkItemsMany), tiles = (nT + tile - 1) / tile;
     if (nT > 0) {
         // status words in the counter block, or in the sort's scratch, which no sort uses yet
