@@ -287,7 +287,8 @@ int galphaSetBlockRun(galphaHandle h, int entries);
  * 32,768): the length above which that block hands them back.  A round past
  * the end of a loop does nothing and the in-block rounds are the launched
  * rounds' functors, so no value changes a result, only the time and
- * gpudtStatus.hostReads; 0 (-1 for flipTailEnter) restores a default, values
+ * gpudtStatus.hostReads (and neither where a stage runs in one launch, see
+ * galphaSetClusterLimit); 0 (-1 for flipTailEnter) restores a default, values
  * out of range return GPUDT_ERR_ARG.  galphaGetSchedule fills out5 with the
  * five values in force.  The autotuner (galpha_b200.autotune) picks them per
  * workload.  No counterpart in the reference. */

@@ -85,3 +85,19 @@ def test_schedule_keeps_the_default_within_noise():
     eng = FakeScheduleEngine(lambda s: 100.0 - 0.5 * (s["flip_sync"] == 8))  # 0.5 % better: below min_gain
     best, _ = A.tune_schedule(eng, eng.run, reps=1)
     assert best == FakeScheduleEngine.DEFAULT
+
+
+@pytest.mark.parametrize("reads,tuned", [([1, 0, 0, 0], False), ([1, 0, 0, 2], True), ([4, 2, 1, 3], True)])
+def test_schedule_without_launched_loops_is_left_alone(reads, tuned):
+    """A workload whose loops all run inside one launch (one counter read) does
+    not depend on the schedule: the differences are noise and are not followed."""
+    eng = FakeScheduleEngine(lambda s: 100.0 - 5.0 * (s["flip_sync"] == 8))
+
+    def run():
+        st = eng.run()
+        st.hostReadsStage = [0, 1, 1] + reads + [1, 2, 0, 0, 0]
+        return st
+
+    best, table = A.tune_schedule(eng, run, reps=1)
+    assert best["flip_sync"] == (8 if tuned else 4) and eng.s == best
+    assert (len(table) == 1) == (not tuned)
