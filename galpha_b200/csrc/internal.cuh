@@ -234,8 +234,8 @@ struct Ctx {
     int nMaster = 0, nSpecPtr = 0;
     bool have_master = false;
     int *hist = nullptr;       // scratch of scans over more than kScanMaxTiles tiles
-    // single-launch scans: status words, then the tile ticket (own allocation,
-    // made with the handle); scans started so far
+    // single-launch scans: status words, then the tile ticket (behind the counter
+    // block, made with the handle); scans started so far
     unsigned long long *scan_buf = nullptr;
     unsigned scan_no = 0;
     int *rhist = nullptr;      // radix sort histograms

@@ -34,6 +34,11 @@ static_assert((size_t)kSmFanBytes * (kMaxChain + 1) >= fake_remove_smem(kMaxChai
 static_assert((size_t)kSmFanBytes * kMaxFanLong >= fake_remove_smem(kMaxFanLong) + 15, "a place holds its fan");
 static_assert(kSmFanBytes <= 2 * sizeof(galphaEdgeInterval), "the array holds every place");
 
+__device__ __noinline__ void fake_remove_long(const FakeRemoveArgs &a, int item, int d, unsigned char *mem, FrWarp &w)
+{
+    fake_remove_item(a, item, d, mem, w);
+}
+
 struct SmallMesh {
     // arrays of Ctx
     double2 *opos, *pos;
@@ -266,7 +271,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mesh_small(const SmallMesh m)
                         if (d > kMaxChain) {
                             const long long at = ((long long)kSmFanBytes * fanoff[item] + 15) & ~15ll;
                             if (at + (long long)fake_remove_smem(d) <= m.longfan_bytes)
-                                fake_remove_item(fr, item, d, m.longfan + at, s_fr[0]);
+                                fake_remove_long(fr, item, d, m.longfan + at, s_fr[0]);
                             else if (lane == 0)
                                 set_err(ct, GPUDT_ERR_TOPOLOGY, 76);  // the fans overlap: a broken mesh
                         }
