@@ -584,11 +584,12 @@ static int handle_init(galpha_ctx *h, int device, long long budget)
         c.hmail_dev = (char *)dp + ctr_bytes;
     }
     {
-        // Counter block and scan words, one allocation for the handle's life.  Which
-        // of the two dies' L2 holds the counters (it changes from one 4 KB to the
-        // next) is worth 4 to 12 % of the one-launch mesh stages, whose cluster sits
-        // on one die: 1,000 points 176 us or 189, 12,289 in a disk 450 or 478.  In the
-        // arena they moved with every size; here a handle keeps them where they are.
+        // Counter block and scan words, one allocation for the handle's life.  The
+        // one-launch mesh stages take 4 to 12 % longer at some addresses of the
+        // counters than at others, two states that change from one 4 KB to the next
+        // (most likely the die whose L2 holds them; the cluster sits on one): 1,000
+        // points 176 us or 189, 12,289 in a disk 450 or 478.  In the arena they moved
+        // with every size; here a handle keeps them where they are.
         const size_t ctr_bytes = (sizeof(Counters) + 4095) & ~(size_t)4095;
         char *p = nullptr;
         GALPHA_CUDA(cudaMalloc(&p, ctr_bytes + kScanBufBytes));

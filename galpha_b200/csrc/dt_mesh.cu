@@ -1920,8 +1920,10 @@ int stage_boundary(Ctx &c)
 // With stamps, marks, epochs and forwarding links in arrays of their own, the
 // proposed edge and its neighbour in two more, and a triangle of each vertex kept
 // up to date (nothing past the constraints reads it), a flip touched some 24
-// sectors, now 10.  The votes stay apart: the first round's go to a third of all
+// sectors, now 10 (its loads and stores, counted; FlipApply at 4,000,000 points 547
+// us, now 341).  The votes stay apart: the first round's go to a third of all
 // triangles, and in an array of four bytes each they stay in L2.
+//
 // Set of constrained edges: open addressing over keys (min id << 32 | max id),
 // empty slots ~0 (constraints, section below).
 __device__ __forceinline__ unsigned long long cons_key(int a, int b)

@@ -1,10 +1,10 @@
 // noalloc.cu -- galphaEdgeListNoAlloc: the alpha stage's edge numbering of a
 // device-resident triangle-neighbour mesh, computed without allocating.
 //
-// The handle path numbers edges in three launches over arena scratch
-// (EdgeCount -> exclusive_scan_int -> the edge writes of TriKeys, which
-// restate computeTriEdgeCount + thrust::exclusive_scan + the edge fill of
-// Alpha_Shapes_2D.cu:170-199).  This variant does the same in ONE kernel: each
+// The handle path numbers edges in the launch that computes the alpha keys
+// (k_alpha_keys, look-back words in the arena; computeTriEdgeCount +
+// thrust::exclusive_scan + the edge fill of Alpha_Shapes_2D.cu:170-199).  This
+// variant only numbers them, from gpudtTriangle records, without an arena: each
 // block takes the next tile of triangles from a ticket, counts the edges its
 // triangles own, finds the tile's global offset by a single-pass decoupled
 // look-back over the per-tile descriptors of earlier tiles, and writes the
@@ -58,7 +58,7 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 // Owned edges of one triangle record staged in shared memory (9 ints: tri[3],
 // vtx[3], tmp[3]): edge i = (vtx[i+1], vtx[i+2]) belongs to the triangle when
 // its first vertex has the smaller index or it lies on the hull (kernel.cu's
-// computeTriEdgeCount rule, the same test as EdgeCount in alpha.cu).
+// computeTriEdgeCount rule, the same test as in alpha.cu's k_alpha_keys).
 __device__ __forceinline__ int owned_mask(const int *r)
 {
     int m = 0;

@@ -416,7 +416,8 @@ __device__ __forceinline__ unsigned owner_scan(const int16_t *__restrict__ row, 
 }
 
 // The near part of the scan from shared memory.  The arithmetic of the scan bounds
-// the kernels that use it (issue slots 82 % busy), so what does not depend on the
+// the kernels that use it (84 % of the issue slots without these words, 81 with
+// them, at 1,048,576 sites), so what does not depend on the
 // pixel is done once per column candidate: a word (y - ycol)^2 << 8 | tile column,
 // kScanNone where there is none (or further than kScanDy rows off, which leaves
 // room for the shift).  A word plus k^2 << 8 then orders the candidates by (d,

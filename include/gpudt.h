@@ -99,7 +99,8 @@ typedef struct {
                                 [0] colour + dual-triangle kernel (k_vd_tri; k_row_pass on
                                 the envelope path), [1] column pass,
                                 [2] triangle emission (count + write),
-                                [3] spectrum key sort (all radix passes, alpha stage) */
+                                [3] spectrum key sort (all radix passes, alpha stage; with
+                                the ranks where one block does both: up to 8,192 keys) */
     long long sortKeys;      /* keys of the spectrum sort */
     int sortPasses;          /* radix passes it took (8-bit digits) */
     int hostReads;           /* device -> host reads of the call, each one stream synchronisation
