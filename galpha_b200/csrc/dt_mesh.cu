@@ -510,6 +510,12 @@ struct BadSelectList {
 // Remove vertex v (interior) and triangulate its star hole by ear clipping
 // with the kernel point K = pos[v] (cudaShifting.cu:350-450 semantics: an ear
 // (A,B,C) is cut when ccw(A,B,C) > 0 and K is strictly left of A->C).
+// A site's fan grows with every neighbour that is removed before it, by the ears
+// that happen to be cut at it, so its length has no small bound: with room for 64
+// triangles one in a hundred batches of 1,024 sets at 4 pixels per point failed.
+// Any fan that can be walked can be removed.
+constexpr int kMaxHole = 4 * kMaxFan;
+
 struct BadRemove {
     int4 *tv, *tn, *fwd;
     int *epoch, *freelist, *vtri, *anchor;
@@ -523,17 +529,16 @@ struct BadRemove {
     __device__ void operator()(long long ii) const
     {
         int v = list[ii];
-        int U[kMaxFan], Fs[kMaxFan], Fi[kMaxFan], O[kMaxFan];
+        int U[kMaxHole], F[kMaxHole], O[kMaxHole];  // per fan triangle: first rim vertex, corner of v, outer link
         int d = 0;
         bool over = false;
         bool fine = walk_fan(tv, tn, vtri[v], [&](int t, int i, int a, int b) {
-            if (d >= kMaxFan) {
+            if (d >= kMaxHole) {
                 over = true;
                 return false;
             }
             U[d] = a;
-            Fs[d] = t;
-            Fi[d] = i;
+            F[d] = enc(t, i);
             O[d] = geti(tn[t], i);
             d++;
             return true;
@@ -544,24 +549,25 @@ struct BadRemove {
         }
         double2 K = pos[v];
         // polygon ring with owners of each current edge (U[k] -> U[next])
-        int nxt[kMaxFan], prv[kMaxFan], own[kMaxFan];  // own: -2-k original edge k, else loc
+        short nxt[kMaxHole], prv[kMaxHole];
+        int own[kMaxHole];  // -2-k original edge k, else loc
         for (int k = 0; k < d; k++) {
-            nxt[k] = (k + 1) % d;
-            prv[k] = (k + d - 1) % d;
+            nxt[k] = (short)((k + 1) % d);
+            prv[k] = (short)((k + d - 1) % d);
             own[k] = -2 - k;
         }
         int used = 0, remaining = d, cur = 0, stall = 0;
         auto owner_link = [&](int ownv, int loc) {
             if (ownv <= -2) {
                 int k = -2 - ownv;
-                set_fwd(fwd, Fs[k], Fi[k], loc);
+                set_fwd(fwd, dtri(F[k]), dori(F[k]), loc);
                 push_rec(rec, nrec, loc, O[k]);
             } else {
                 set_link(tn, loc, ownv);
                 set_link(tn, ownv, loc);
             }
         };
-        for (int k = 0; k < d; k++) epoch[Fs[k]] = round;
+        for (int k = 0; k < d; k++) epoch[dtri(F[k])] = round;
         // strict pass first (K strictly inside what remains); when a full
         // cycle finds no such ear, K lies on a candidate diagonal and the
         // closed test is used (the rest stays star-shaped from K)
@@ -578,7 +584,7 @@ struct BadRemove {
                 ear = orientp(pos[U[A]], pos[U[C]], pos[U[D]], ct) > 0;
             }
             if (ear) {
-                int s = Fs[used++];
+                int s = dtri(F[used++]);
                 tv[s] = make_int4(U[A], U[B], U[C], 0);
                 tn[s] = make_int4(-1, -1, -1, 0);
                 // edges: opp A (0) = B->C owned by own[B]; opp C (2) = A->B owned by own[A];
@@ -589,8 +595,8 @@ struct BadRemove {
                 vtri[U[A]] = enc(s, 0);
                 vtri[U[B]] = enc(s, 1);
                 vtri[U[C]] = enc(s, 2);
-                nxt[A] = C;
-                prv[C] = A;
+                nxt[A] = (short)C;
+                prv[C] = (short)A;
                 remaining--;
                 cur = C;
                 stall = 0;
@@ -614,7 +620,7 @@ struct BadRemove {
                 set_err(ct, GPUDT_ERR_TOPOLOGY, 52);
                 return;
             }
-            int s = Fs[used++];
+            int s = dtri(F[used++]);
             tv[s] = make_int4(U[A], U[B], U[C], 0);
             tn[s] = make_int4(-1, -1, -1, 0);
             owner_link(own[B], enc(s, 0));
@@ -624,7 +630,7 @@ struct BadRemove {
             vtri[U[B]] = enc(s, 1);
             vtri[U[C]] = enc(s, 2);
         }
-        for (int k = used; k < d; k++) free_slot(tv, freelist, ct, Fs[k]);
+        for (int k = used; k < d; k++) free_slot(tv, freelist, ct, dtri(F[k]));
         int an = U[0];
         for (int k = 0; k < d; k++)
             if (U[k] < nreal) {

@@ -44,3 +44,21 @@ def test_hull_vertex_with_a_long_fan(engine, row):
     dt = engine.triangulate(G.GPUDTParams(pts, fboSize=4096))
     ok, rep = compare_dt(pts, dt.vtx, dt.tri)
     assert ok, rep
+
+
+@pytest.mark.parametrize("limit", [-1, 0])
+@pytest.mark.parametrize("n,fbo", [(2500, 1024), (5500, 1024), (6500, 1024), (9500, 4096)])
+def test_bad_sites_with_long_fans(engine, n, fbo, limit):
+    """Points on a circle: thousands of unshiftable sites side by side, whose fans
+    grow with every neighbour removed before them, past 64 triangles (the length
+    that removal once had room for).  In one launch and in launches."""
+    th = np.linspace(0.0, 2.0 * np.pi, n, endpoint=False) + 0.001
+    pts = np.stack([np.cos(th), np.sin(th)], axis=1)
+    engine.set_cluster_limit(limit)
+    try:
+        dt = engine.triangulate(G.GPUDTParams(pts, fboSize=fbo))
+    finally:
+        engine.set_cluster_limit(-1)
+    assert dt.status.nBadShift > 1000
+    ok, rep = compare_dt(pts, dt.vtx, dt.tri)
+    assert ok, rep
