@@ -292,13 +292,18 @@ static int ring(int k)
 }
 
 // ------------------------------------------------------------------- shift
+// A fan has no small bound (points in one pixel are all inserted from the site that
+// owns it, and a hub sees its whole ring), so walks around a vertex are bounded
+// only against a broken mesh.
+constexpr int kMaxFanWalk = 1 << 20;
+
 // A fan walk around interior vertex v: calls f(t, i, a, b) for every
-// triangle (v, a, b) counterclockwise; returns false on a fan over kMaxFan*4.
+// triangle (v, a, b) counterclockwise; returns false on a broken mesh.
 template <class Fn>
 __device__ __forceinline__ bool walk_fan(const int4 *tv, const int4 *tn, int start, Fn f)
 {
     int e = start;
-    for (int guard = 0; guard < 4 * kMaxFan; guard++) {
+    for (int guard = 0; guard < kMaxFanWalk; guard++) {
         int t = dtri(e), i = dori(e);
         int4 w = tv[t];
         if (!f(t, i, geti(w, p1(i)), geti(w, m1(i)))) return true;
@@ -513,8 +518,7 @@ struct BadSelectList {
 // A site's fan grows with every neighbour that is removed before it, by the ears
 // that happen to be cut at it, so its length has no small bound: with room for 64
 // triangles one in a hundred batches of 1,024 sets at 4 pixels per point failed.
-// Any fan that can be walked can be removed.
-constexpr int kMaxHole = 4 * kMaxFan;
+constexpr int kMaxHole = 256;
 
 struct BadRemove {
     int4 *tv, *tn, *fwd;
@@ -781,7 +785,7 @@ __device__ int locate_walk(const int4 *tv, const int4 *tn, const double2 *P, con
         int e = vtri[a], t = -1, ia = 0;
         for (int dir = 0; dir < 2 && t < 0; dir++) {
             e = vtri[a];
-            for (int guard = 0; guard < 4 * kMaxFan; guard++) {
+            for (int guard = 0; guard < kMaxFanWalk; guard++) {
                 int tt = dtri(e), i = dori(e);
                 int4 w = tv[tt];
                 int b = geti(w, p1(i)), c = geti(w, m1(i));

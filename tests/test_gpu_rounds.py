@@ -62,3 +62,36 @@ def test_bad_sites_with_long_fans(engine, n, fbo, limit):
     assert dt.status.nBadShift > 1000
     ok, rep = compare_dt(pts, dt.vtx, dt.tri)
     assert ok, rep
+
+
+@pytest.mark.parametrize("limit", [-1, 0])
+@pytest.mark.parametrize("n,fbo", [(3500, 2048), (5000, 512), (7000, 2048)])
+def test_points_in_one_pixel(engine, n, fbo, limit):
+    """Three clusters that each fall into a pixel or two: all their points are
+    located from the one site that owns the pixel, whose fan grows past 256
+    triangles (the length after which location once gave up)."""
+    c = D.uniform_points(n, 4) * 0.001
+    pts = np.concatenate([c, c + [0.9, 0.9], c * [1, -1] + [0.0, 0.9]])
+    engine.set_cluster_limit(limit)
+    try:
+        dt = engine.triangulate(G.GPUDTParams(pts, fboSize=fbo))
+    finally:
+        engine.set_cluster_limit(-1)
+    assert dt.status.nMissing > 2 * n
+    assert canon_set(dt.vtx) == canon_set(O.dt(pts)[0])
+
+
+@pytest.mark.parametrize("limit", [-1, 0])
+@pytest.mark.parametrize("n,fbo", [(300, 512), (1500, 2048), (6000, 4096)])
+def test_hub_of_a_ring(engine, n, fbo, limit):
+    """A point in the middle of a ring sees every point of it; with others beside
+    it, so that it is shifted, and located through, with that fan."""
+    th = np.linspace(0.0, 2.0 * np.pi, n, endpoint=False) + 0.01
+    ring = np.stack([np.cos(th), np.sin(th)], axis=1) * (1.0 + 1e-5 * np.sin(5.0 * th))[:, None]
+    pts = np.concatenate([ring, [[1e-4, 2e-4]], 1e-5 * D.uniform_points(40, n)])
+    engine.set_cluster_limit(limit)
+    try:
+        dt = engine.triangulate(G.GPUDTParams(pts, fboSize=fbo))
+    finally:
+        engine.set_cluster_limit(-1)
+    assert canon_set(dt.vtx) == canon_set(O.dt(pts)[0])
